@@ -58,7 +58,7 @@ def build(force=False):
 
 def build_ref():
     """Builds _ref/libsphref.so from the reference sources when they are present."""
-    if not os.path.isdir(REF_SRC):
+    if not os.path.isfile(os.path.join(REF_SRC, "core", "container", "SoAContainer.cpp")):
         return None
     subprocess.check_call(["make", "-s", "-C", HERE, "ref", "REF=" + REF_SRC])
     return REF_SO
