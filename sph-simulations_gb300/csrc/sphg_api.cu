@@ -232,22 +232,21 @@ namespace sphg_detail {
 static sphg::MoverArgs mover_args(sphg_sim* s, unsigned long long cond) {
   sphg::MoverArgs m = {};
   m.n = s->n;
-  m.keyA = s->keyA;
-  m.mask = s->mmask;
-  m.movers = s->mlist;
-  m.count = s->flags + 7;
+  m.limit = sphg::mover_limit(s->n);
+  m.rec = s->mrec;
   m.ctl = s->flags + 3;
   m.epoch = s->flags + 2;
-  m.ranges = s->ranges;
-  m.keyS = s->keyTmp;
-  m.perm = s->perm;
-  m.cond = cond;
+  m.keyB = s->keyB;
   m.posB = s->posB;
   m.velB = s->velB;
   m.idsB = s->opt.track_ids ? s->idsB : nullptr;
+  m.keyA = s->keyA;
   m.posA = s->posA;
   m.velpA = s->velpA;
   m.idsA = s->opt.track_ids ? s->idsA : nullptr;
+  m.perm = s->perm;
+  m.ranges = s->ranges;
+  m.cond = cond;
   m.early_next = s->n <= sphg::kEarlyNextMaxN ? 1 : 0;
   return m;
 }
@@ -285,12 +284,14 @@ sphg_status enqueue_full_sort(sphg_sim* s, cudaStream_t st, const uint32_t* skip
 // size_lists: (lists mode) size the index buffer from this iteration's total
 // first -- a host synchronisation, done on the first iteration after an upload
 // (never inside a graph capture).
-sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bool size_lists = false) {
+// reorder: the gather after a full sort is launched here (else the caller has
+// placed it with the sort).
+sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bool size_lists = false,
+                               bool reorder = true) {
   const StepArgs a = s->args();
   const int prec = s->opt.precision;
   if (s->tile_bits) SPHG_CUDA(cudaMemsetAsync(s->flags + 1, 0, sizeof(uint32_t), st));
-  // (the reorder zeroes the mover count of this iteration's force pass)
-  SPHG_CUDA(sphg::launch_reorder(a, st));
+  if (reorder) SPHG_CUDA(sphg::launch_reorder(a, st));
   if (ev) SPHG_CUDA(cudaEventRecord(ev[3], st));
   if (s->opt.compute == SPHG_COMPUTE_LISTS) {
     // AssembleNeighborList: count, offsets, fill -- then density and forces over the lists
@@ -427,14 +428,16 @@ sphg_status build_graph_conditional(sphg_sim* s, cudaGraphExec_t* exec, bool hea
       cudaSuccess)
     return done(fail(SPHG_CUDA_ERROR, "capture of the conditional body"));
   st = enqueue_full_sort(s, s->cap_stream2, nullptr);
-  if (st == SPHG_OK && fused) st = enqueue_fused(s, s->cap_stream2, true, 0);  // ranges, density, forces
+  if (st == SPHG_OK && fused) st = enqueue_fused(s, s->cap_stream2, true, 0);  // reorder, density, forces
+  if (st == SPHG_OK && !fused && sphg::launch_reorder(s->args(), s->cap_stream2) != cudaSuccess)
+    st = fail(SPHG_CUDA_ERROR, "reorder in the conditional body");
   cudaGraph_t body_out = nullptr;
   const cudaError_t eb = cudaStreamEndCapture(s->cap_stream2, &body_out);
   if (st != SPHG_OK) return done(st);
   if (eb != cudaSuccess) return done(fail(SPHG_CUDA_ERROR, "end of the conditional body capture"));
   if (cudaStreamUpdateCaptureDependencies(s->cap_stream, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies) != cudaSuccess)
     return done(fail(SPHG_CUDA_ERROR, "capture dependencies"));
-  if (!fused) st = enqueue_after_sort(s, s->cap_stream, nullptr);
+  if (!fused) st = enqueue_after_sort(s, s->cap_stream, nullptr, false, false);
   if (st == SPHG_OK && header) st = enqueue_header(s, s->cap_stream);
   if (st != SPHG_OK) return done(st);
   cudaGraph_t out = nullptr;
@@ -571,7 +574,7 @@ sphg_status alloc_arena(sphg_sim* s, size_t N, uint64_t keys, int ninst, int dia
     s->perm = A.take<uint32_t>(N);
     s->valTmp = A.take<uint32_t>(N);
     s->scratch = A.take<uint32_t>(sphg::sort_scratch_words(N));
-    s->flags = A.take<uint32_t>(16);
+    s->flags = A.take<uint32_t>(32);
     s->diag_partials = A.take<double>((size_t)ninst * s->diag_chunks * 6);
     s->diag_out = A.take<double>((size_t)ninst * 6);
     s->hslot = A.take<sphg::HeaderSlot>(1);
@@ -588,8 +591,13 @@ sphg_status alloc_arena(sphg_sim* s, size_t N, uint64_t keys, int ninst, int dia
       s->ncount = A.take<uint32_t>(N);
     }
     if (s->movers_on) {
-      s->mmask = A.take<uint32_t>((N + 31) / 32);
-      s->mlist = A.take<unsigned long long>(sphg::kMoverCap);
+      sphg::MoverRecord& r = s->mrec;
+      r.mask = A.take<uint32_t>((N + 31) / 32);
+      r.head = A.take<uint32_t>(N + 1);
+      r.next = A.take<uint32_t>(N);
+      r.counts = A.take<uint32_t>(2 * sphg::mover_counts_words((int64_t)N));
+      r.next_epoch = s->flags + 13;
+      r.cap = (int64_t)N;
     }
     if (s->opt.compute == SPHG_COMPUTE_LISTS) {
       s->csr_counts = A.take<int32_t>(N);
@@ -619,6 +627,9 @@ sphg_status alloc_arena(sphg_sim* s, size_t N, uint64_t keys, int ninst, int dia
   // first sort, so no range entry is valid before its cell is written; the
   // table is never cleared again
   e = cudaMemset(s->arena.base, 0, s->arena.size);
+  const uint32_t first_epoch = 1;
+  if (e == cudaSuccess && s->movers_on)
+    e = cudaMemcpy(s->mrec.next_epoch, &first_epoch, sizeof(first_epoch), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail(SPHG_CUDA_ERROR, std::string("state init: ") + cudaGetErrorString(e));
   return SPHG_OK;
 }
@@ -1119,8 +1130,8 @@ sphg_status sphg_get_debug(sphg_sim* s, int32_t which, void* host, void* stream)
         SPHG_CUDA(cudaMemcpyAsync(c, s->flags + 3, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         SPHG_CUDA(cudaStreamSynchronize(st));
       }
-      // histogram + radix passes of a full sort (+ the post part of the single-launch iteration)
-      c[2] = (uint32_t)((s->key_bits + 7) / 8 + 1 + (fused_on(s) ? 1 : 0));
+      // histogram + radix passes of a full sort + the reorder (single-launch iteration: its post part)
+      c[2] = (uint32_t)((s->key_bits + 7) / 8 + 2);
       std::memcpy(host, c, sizeof(c));
       return SPHG_OK;
     }
@@ -1295,7 +1306,7 @@ int32_t sphg_launches_per_step(const sphg_sim* s) {
   // an iteration that runs the full sort: its histogram kernel + radix passes +
   // reorder + density + force (+ the incremental re-sort's merge kernel; + list
   // count, three scan kernels and list fill in the lists mode).  An iteration
-  // that merges launches (key_bits + 7) / 8 + 1 kernels fewer in a graph.
+  // that merges launches (key_bits + 7) / 8 + 2 kernels fewer in a graph.
   // With the single-launch iteration: the launch (which only decides), the
   // histogram + radix passes and the launch's post part; an iteration that
   // merges is the one launch.

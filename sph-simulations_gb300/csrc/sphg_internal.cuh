@@ -71,11 +71,10 @@ struct sphg_sim {
   int64_t *csr_offs = nullptr, *csr_sums = nullptr;
   uint32_t* csr_idx = nullptr;
   int64_t csr_cap = 0, csr_total = 0;
-  // incremental re-sort: mover bits and group counts written by the force pass
+  // incremental re-sort: the record written by the force pass
   bool movers_on = false;
   bool force_full_sort = false;  // the next iteration sorts fully (the slot record is stale)
-  uint32_t* mmask = nullptr;
-  unsigned long long* mlist = nullptr;
+  sphg::MoverRecord mrec{};
   size_t cap_n = 0;             // arena capacity (particles)
   uint64_t cap_keys = 0;        // arena capacity (cell keys)
   int cap_inst = 0;             // arena capacity (instances)
@@ -145,9 +144,7 @@ struct sphg_sim {
     a.csr_overflow = flags + 8;
     a.keyS = keyTmp;
     a.merged = movers_on ? flags + 3 : nullptr;
-    a.mover_mask = movers_on ? mmask : nullptr;
-    a.mover_list = movers_on ? mlist : nullptr;
-    a.mover_count = movers_on ? flags + 7 : nullptr;
+    if (movers_on) a.movers = mrec;
     return a;
   }
 };

@@ -4,27 +4,27 @@
 // cell, so almost every particle keeps its cell key.  The stable sort of the
 // new keys (GenericNeighborSearch::SortParticleIds,
 // core/alg/GenericNeighborSearch.h:69-76, with ties in previous-slot order)
-// is then a merge of two sorted sequences:
+// is then a merge of two sequences:
 //   * stayers: slots whose key did not change -- already in (key, slot) order,
 //     because the current state is sorted;
 //   * movers: slots whose key changed -- few.
-// Writing v_s = (key, slot) for the order of slot s:
-//   final position of a stayer i = i - (movers with slot < i)
-//                                    + (movers with v < v_i)
-//   final position of a mover m  = (movers with v < v_m)
-//                                    + (slots s with v_s < v_m in the current order)
-//                                    - (movers among those slots)
-// The force pass records every mover (key << 32 | slot, appended with one
-// atomic per warp) and one bit per slot.  One kernel then places everything:
-// each block of 512 consecutive slots counts, over the whole (short) mover
-// list, the movers before its first slot and before its first stayer's key,
-// keeps the few movers whose key falls inside its own key span in shared
-// memory, and places its stayers; the movers go to leading blocks of their
-// own, a warp each, which start with the launch.  When more than kMoverCap
-// slots changed the kernel only records
-// that and the full radix sort runs instead (under a conditional graph node,
-// or its kernels skip themselves on the decision word).
-#include <algorithm>
+// The force pass finds each mover's insertion point p while the current cell
+// ranges are at hand -- the number of current slots ordered before its (new
+// key, slot) -- and records it there (record_movers): a count per p, the chain
+// of the movers at p, and the net change (insertions - movers) of every 512
+// slots and of every 32,768.  The sorted order is then: for p = 0, 1, ..., n
+// the movers of p by (key, slot), then slot p if it stays.
+//
+// One kernel writes it.  A block takes 512 slots with the movers inserted
+// before them, whose output is one contiguous run that starts at the block's
+// first slot plus the net change of the slots before it; the positions inside
+// are bit counts.  Having the run's keys in shared memory, the block writes the
+// cell ranges too (the keys either side of the run come from the neighbouring
+// slots), so an iteration that merges needs no pass over the sorted keys.  The
+// cost does not depend on how many slots changed.  When more did than
+// mover_limit(), or a group or a block passed its cap, the kernel only records
+// that and the full radix sort and the reorder run instead (under a conditional
+// graph node, or they return at once on the decision word).
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -38,26 +38,18 @@ namespace sphg {
 namespace {
 
 __global__ void __launch_bounds__(kMergeThreads) movers_merge(MoverArgs a) {
+  __shared__ MergeShared sh;
   cudaGridDependencySynchronize();  // the mover record of the previous force pass
   allow_next_kernel(a.early_next);
-  uint32_t m = 0;
-  if (!merge_decide(a, blockIdx.x == 0 && threadIdx.x == 0, &m)) return;
-  constexpr uint32_t W = kMergeThreads / 32;
-  if (blockIdx.x < a.mover_blocks)
-    merge_movers<false>(a, blockIdx.x * W + (threadIdx.x >> 5), a.mover_blocks * W, m);
-  else
-    merge_block<false>(a, blockIdx.x - a.mover_blocks, 0, m);
+  merge_block<false>(a, sh, blockIdx.x);
 }
 
 }  // namespace
 
 cudaError_t launch_movers(const MoverArgs& a, cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
-  const int64_t nb = (a.n + kMergeBlockSlots - 1) / kMergeBlockSlots;
-  MoverArgs b = a;
-  b.mover_blocks = (uint32_t)std::min<int64_t>(kMoverBlocks, std::max<int64_t>(8, nb / 4));
-  const unsigned g = (unsigned)nb + b.mover_blocks;
-  cudaError_t e = launch_pdl(movers_merge, dim3(g), dim3(kMergeThreads), 0, st, b);
+  // the block of p = n included
+  cudaError_t e = launch_pdl(movers_merge, dim3((unsigned)((a.n >> kMergeShift) + 1)), dim3(kMergeThreads), 0, st, a);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }

@@ -1,11 +1,7 @@
-// sphg_movers_body.cuh -- the incremental re-sort's per-block work, shared by
-// the stand-alone merge kernel (sphg_movers.cu) and the fused single-launch
-// iteration (sphg_step.cu).  The algorithm is described in sphg_movers.cu.
-//
-// COHERENT: the caller is a kernel that rewrites keyA and the cell-range table
-// later in the same launch (the fused iteration); their loads then bypass the
-// incoherent L1 / texture path (ld.global.cg), so no stale line of them is left
-// in an SM's L1 for the later phases' reads.
+// sphg_movers_body.cuh -- the incremental re-sort's device code, shared by the
+// stand-alone kernels (sphg_movers.cu: the merge; sphg_step.cu: the force
+// pass's record) and the single-launch iteration (sphg_step.cu).  The algorithm
+// is described in sphg_movers.cu.
 #pragma once
 #include <cstdint>
 
@@ -13,230 +9,363 @@
 
 #include "sphg_common.cuh"
 #include "sphg_movers.cuh"
+#include "sphg_step.cuh"
 
 namespace sphg {
 
 constexpr int kMergeThreads = 128;
-#ifndef SPHG_MERGE_SLOTS
-#define SPHG_MERGE_SLOTS 4
-#endif
-constexpr int kMergeSlots = SPHG_MERGE_SLOTS;               // slots per thread
-constexpr int kMergeBlockSlots = kMergeThreads * kMergeSlots;  // 512 slots, 16 mask words
-constexpr int kSpanCap = 256;                               // movers inside a block's key span kept in shared memory
-// The stand-alone merge kernel's first blocks place the movers (a warp each,
-// from the start of the launch: their chain of dependent loads overlaps the
-// other blocks' work), the others only the unchanged slots: at most
-// kMoverBlocks of them (1M dam break: 17.7 -> 14.9 us against every block
-// placing its share of the movers after its unchanged slots).
-constexpr int kMoverBlocks = 512;
-static_assert(kMergeBlockSlots / 32 <= kMergeThreads, "one thread per mask word of the block");
+constexpr int kMergeSlots = kMergeBlockSlots / kMergeThreads;  // slots per thread
+constexpr int kMergeWords = kMergeBlockSlots / 32;             // mask words per block
+constexpr int kMergeWarps = kMergeThreads / 32;
+static_assert(kMergeWords <= 32 && kMergeWarps >= 4, "one warp scans the words; warps 2 and 3 find the neighbours");
 
-template <bool COHERENT, class T>
-__device__ __forceinline__ T merge_load(const T* p) {
-  if constexpr (COHERENT) return __ldcg(p);
-  else return __ldg(p);
+// ---------------------------------------------------------------- the record
+// Clears slot i's part of the copy the next force pass adds to (the reorder
+// after a full sort; a merge clears its blocks' parts itself).
+__device__ __forceinline__ void clear_mover_counts(const StepArgs& a, int64_t i, uint32_t epoch) {
+  if (!a.movers.mask) return;
+  const MoverCounts r = mover_counts(a.movers, epoch + 1u);
+  const bool last = i == a.n - 1;  // also the entries of p = n
+  if ((i & 3) == 0) r.insc[i >> 2] = 0u;
+  if (last) r.insc[a.n >> 2] = 0u;
+  for (int k = 0; k < 2; ++k) {
+    const int64_t q = k == 0 ? i : a.n;
+    if (k == 0 ? (i & (kMergeBlockSlots - 1)) != 0 : !last) continue;
+    const int64_t b = q >> kMergeShift;
+    r.blk_net[b] = 0;
+    r.blk_ins[b] = 0u;
+    r.sup_net[b >> kMergeSupShift] = 0;
+  }
+  if (i == 0)
+    for (int k = 0; k < kMoverCounters; ++k) r.total[k * kMoverCounterStride] = r.total[k * kMoverCounterStride + 1] = 0u;
 }
 
-// Slot `from` of the integrated state (its values p, v, id) to sorted position
-// `to` (COHERENT: stores that bypass L1, read by a later phase of the launch).
-template <bool COHERENT, class V>
+// The movers of one warp's 32 consecutive slots (bit l of moved: lane l's slot
+// i moved to cell `key`) into the record.  The whole warp calls it.
+__device__ __forceinline__ void record_movers(const StepArgs& a, uint32_t i, uint32_t key, unsigned moved) {
+  const uint32_t epoch = *a.epoch;
+  const MoverCounts r = mover_counts(a.movers, epoch + 1u);
+  const int lane = threadIdx.x & 31;
+  const bool mine = (moved >> lane) & 1u;
+  if (lane == __ffs(moved) - 1)
+    atomicAdd(r.total + ((i >> 5) % kMoverCounters) * kMoverCounterStride, (uint32_t)__popc(moved));
+  // insertion point: the new cell's range when it holds particles now (the slot
+  // itself is not among them), else a warp-wide 32-way search of the keys
+  uint32_t p = 0;
+  bool search = false;
+  if (mine) {
+    const uint4 cr = a.ranges[key];
+    search = cr.z != epoch || cr.x >= cr.y;
+    p = i < cr.x ? cr.x : cr.y;
+  }
+  for (unsigned todo = __ballot_sync(0xffffffffu, search); todo; todo &= todo - 1) {
+    const int l = __ffs(todo) - 1;
+    const uint32_t k = __shfl_sync(0xffffffffu, key, l);
+    int64_t lo = 0, hi = a.n;
+    while (hi > lo) {
+      const int64_t step = (hi - lo + 31) / 32;
+      const int64_t q = lo + (int64_t)(lane + 1) * step - 1;
+      const int c = __popc(__ballot_sync(0xffffffffu, q < hi && a.keyA[q] < k));
+      const int64_t nhi = lo + (int64_t)(c + 1) * step - 1;
+      lo += (int64_t)c * step;
+      if (nhi < hi) hi = nhi;
+      if (lo > hi) lo = hi;
+    }
+    if (lane == l) p = (uint32_t)lo;
+  }
+  if (mine && p <= (uint64_t)a.n) {
+    const int sh = 8 * (int)(p & 3u);
+    const uint32_t before = (atomicAdd(r.insc + (p >> 2), 1u << sh) >> sh) & 255u;
+    const uint32_t in_block = atomicAdd(r.blk_ins + (p >> kMergeShift), 1u);
+    a.movers.next[i] = atomicExch(a.movers.head + p, i);
+    // net changes: most movers stay in their block of slots, nearly all in the 64 blocks
+    const uint32_t bp = p >> kMergeShift, bi = i >> kMergeShift;
+    if (bp != bi) {
+      atomicAdd(r.blk_net + bp, 1);
+      atomicSub(r.blk_net + bi, 1);
+      if (bp >> kMergeSupShift != bi >> kMergeSupShift) {
+        atomicAdd(r.sup_net + (bp >> kMergeSupShift), 1);
+        atomicSub(r.sup_net + (bi >> kMergeSupShift), 1);
+      }
+    }
+    if (before >= (uint32_t)kGroupCap - 1u || in_block >= (uint32_t)kBlockInsertCap - 1u) r.total[1] = 1u;
+  }
+}
+
+// ---------------------------------------------------------------- the merge
+// The decision, from the force pass's record: merge when at most `limit` slots
+// changed and no cap was passed.
+// (The whole warp calls it.)
+__device__ __forceinline__ bool merge_wanted(const MoverArgs& a, const uint32_t* total, uint32_t* movers) {
+  const int lane = threadIdx.x & 31;
+  const volatile uint32_t* t = total;
+  const uint32_t m = lane < kMoverCounters ? t[lane * kMoverCounterStride] : 0u, capped = t[1];
+  *movers = __reduce_add_sync(0xffffffffu, m);
+  return (int64_t)*movers <= a.limit && capped == 0u;
+}
+// The leader's part of it: the decision word, the count, the step
+// epoch, the graph's conditional.
+__device__ __forceinline__ void merge_decided(const MoverArgs& a, bool merge, uint32_t movers, uint32_t epoch) {
+  a.ctl[0] = merge ? 1u : 0u;
+  a.ctl[1] = movers;
+  if (merge) *a.epoch = epoch;
+  if (a.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, merge ? 0u : 1u);
+}
+
+__device__ __forceinline__ uint32_t merge_inserted(const uint32_t* insc, int64_t p) {
+  return reinterpret_cast<const uint8_t*>(insc)[p];
+}
+
+// Smallest or largest key among the c movers inserted before slot p.
+__device__ __forceinline__ uint32_t merge_group_key(const MoverArgs& a, int64_t p, uint32_t c, bool largest) {
+  uint32_t m = a.rec.head[p], k = largest ? 0u : kNoIndex;
+  for (uint32_t q = 0; q < c && m < a.n; ++q) {
+    const uint32_t km = a.keyB[m];
+    k = largest ? max(k, km) : min(k, km);
+    m = a.rec.next[m];
+  }
+  return k;
+}
+
+// Key of the last element of the sorted order that comes before the insertions
+// of slot `base` (a multiple of 32), kNoIndex if none.  The whole warp calls it.
+__device__ __forceinline__ uint32_t merge_prev_key(const MoverArgs& a, const uint32_t* insc, int64_t base, int lane) {
+  for (int64_t q = base - 32; q >= 0; q -= 32) {
+    const int64_t i = q + lane;
+    const bool stay = !((a.rec.mask[q >> 5] >> lane) & 1u);
+    const uint32_t c = merge_inserted(insc, i);
+    const unsigned b = __ballot_sync(0xffffffffu, stay || c);
+    if (!b) continue;
+    const int l = 31 - __clz(b);
+    uint32_t k = 0;
+    if (lane == l) k = stay ? a.keyB[i] : merge_group_key(a, i, c, true);
+    return __shfl_sync(0xffffffffu, k, l);
+  }
+  return kNoIndex;
+}
+
+// Key of the first element from slot q on (its insertions included), kNoIndex if none.
+__device__ __forceinline__ uint32_t merge_next_key(const MoverArgs& a, const uint32_t* insc, int64_t from, int lane) {
+  for (int64_t q = from; q <= a.n; q += 32) {
+    const int64_t i = q + lane;
+    const bool stay = i < a.n && !((a.rec.mask[q >> 5] >> lane) & 1u);
+    const uint32_t c = i <= a.n ? merge_inserted(insc, i) : 0u;
+    const unsigned b = __ballot_sync(0xffffffffu, stay || c);
+    if (!b) continue;
+    const int l = __ffs(b) - 1;
+    uint32_t k = 0;
+    if (lane == l) k = c ? merge_group_key(a, i, c, false) : a.keyB[i];
+    return __shfl_sync(0xffffffffu, k, l);
+  }
+  return kNoIndex;
+}
+
+// Stores of data that a later phase of the same launch reads (FUSED) bypass L1.
+template <bool FUSED, class V>
 __device__ __forceinline__ void merge_store(V* p, V v) {
-  if constexpr (COHERENT) __stcg(p, v);
+  if constexpr (FUSED) __stcg(p, v);
   else *p = v;
 }
-template <bool COHERENT>
-__device__ __forceinline__ void merge_place(const MoverArgs& a, int64_t from, int64_t to, uint32_t key, float2 p,
-                                            float2 v, int32_t id) {
-  merge_store<COHERENT>(a.keyS + to, key);
-  merge_store<COHERENT>(a.perm + to, (uint32_t)from);
-  merge_store<COHERENT>(a.posA + to, p);
-  merge_store<COHERENT>(a.velpA + to, make_float4(v.x, v.y, 0.f, 0.f));
-  if (a.idsA) merge_store<COHERENT>(a.idsA + to, id);
-}
 
-// Position of (k, sl) among the slots of the current sorted order: the number
-// of slots s with (keyA[s], s) < (k, sl).  When cell k holds particles now its
-// range [start, end) gives it directly (an entry is current when the key at
-// its start is k: a cell that is empty now has no slot with key k); otherwise
-// a warp-wide 32-way search of the keys finds it.  All lanes return the value.
-template <bool COHERENT>
-__device__ __forceinline__ int64_t merge_current_position(const MoverArgs& a, uint32_t k, uint32_t sl, int lane) {
-  const uint4 cr = merge_load<COHERENT>(a.ranges + k);
-  if (cr.x < cr.y && cr.y <= (uint64_t)a.n && merge_load<COHERENT>(a.keyA + cr.x) == k)
-    return sl < cr.x ? (int64_t)cr.x : (sl > cr.y ? (int64_t)cr.y : (int64_t)sl);
-  int64_t lo = 0, hi = a.n;
-  while (hi - lo > 32) {
-    const int64_t step = (hi - lo + 31) / 32;
-    const int64_t pos = lo + (int64_t)(lane + 1) * step - 1;
-    bool less = false;
-    if (pos < hi) {
-      const uint32_t kp = merge_load<COHERENT>(a.keyA + pos);
-      less = kp < k || (kp == k && pos < (int64_t)sl);
-    }
-    const int cnt = __popc(__ballot_sync(0xffffffffu, less));
-    const int64_t nhi = lo + (int64_t)(cnt + 1) * step - 1;
-    lo += (int64_t)cnt * step;
-    if (nhi < hi) hi = nhi;
-  }
-  bool less = false;
-  if (lo + lane < hi) {
-    const int64_t pos = lo + lane;
-    const uint32_t kp = merge_load<COHERENT>(a.keyA + pos);
-    less = kp < k || (kp == k && pos < (int64_t)sl);
-  }
-  return lo + __popc(__ballot_sync(0xffffffffu, less));
-}
+struct MergeShared {
+  uint32_t stay[kMergeWords];            // bit per slot: it keeps its cell
+  uint32_t tot[kMergeWords];             // stayers + insertions of the word | insertions << 16
+  int32_t red[kMergeWarps];
+  bool merge;
+  uint32_t prev, next;                   // keys either side of the block's output
+  uint32_t ikey[kBlockInsertCap], islot[kBlockInsertCap];
+  uint32_t igrp[kBlockInsertCap];        // first list entry of the mover's group << 16 | its size
+  uint32_t iout[kBlockInsertCap];        // block-local output position of its group
+  uint32_t key[kMergeBlockSlots + kBlockInsertCap];  // the block's output keys
+};
 
-// The decision, by every block from the force pass's count: merge when at most
-// kMoverCap slots changed.  The leader records it (decision word, count, the
-// step epoch the skipped radix sort would have bumped, the graph's conditional).
-__device__ __forceinline__ bool merge_decide(const MoverArgs& a, bool leader, uint32_t* total) {
-  const uint32_t t = *(volatile const uint32_t*)a.count;
-  const bool inc = t <= (uint32_t)kMoverCap;
-  if (leader) {
-    a.ctl[0] = inc ? 1u : 0u;
-    a.ctl[1] = t;
-    if (inc) atomicAdd(a.epoch, 1u);
-    if (a.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, inc ? 0u : 1u);
-  }
-  *total = t;
-  return inc;
-}
-
-// Mover q of the list (key << 32 | slot): its rank among the movers, its
-// current position and the movers below that, then its state to its final
-// position.  The whole warp calls it.
-template <bool COHERENT>
-__device__ __forceinline__ void merge_mover(const MoverArgs& a, uint32_t q, uint32_t m, int lane) {
-  const unsigned long long* __restrict__ ml = a.movers;
-  const unsigned long long e = __ldg(ml + q);
-  const uint32_t k = (uint32_t)(e >> 32), sl = (uint32_t)e;
-  const int64_t pcur = merge_current_position<COHERENT>(a, k, sl, lane);
-  uint32_t rank = 0, movers_below = 0;
-  for (uint32_t r = lane; r < m; r += 32) {
-    const unsigned long long f = __ldg(ml + r);
-    rank += f < e;
-    movers_below += (int64_t)(uint32_t)f < pcur;
-  }
-  rank = __reduce_add_sync(0xffffffffu, rank);
-  movers_below = __reduce_add_sync(0xffffffffu, movers_below);
-  if (lane == 0) {
-    const int64_t fin = (int64_t)rank + pcur - (int64_t)movers_below;
-    if (fin >= 0 && fin < a.n && sl < a.n)
-      merge_place<COHERENT>(a, sl, fin, k, a.posB[sl], a.velB[sl], a.idsA ? a.idsB[sl] : 0);
-    else
-      a.ctl[2] = 1u;
-  }
-}
-
-// Merge block blk of nblk (slots [blk * 512, blk * 512 + 512) and its share of
-// the m movers; nblk = 0: the unchanged slots only); every thread of the block
-// calls it.
-template <bool COHERENT>
-__device__ __forceinline__ void merge_block(const MoverArgs& a, int64_t blk, uint32_t nblk, uint32_t m) {
-  const unsigned long long* __restrict__ ml = a.movers;
+// Merge block blk: the movers inserted before slots [512 blk, 512 blk + 512)
+// and the slots themselves that keep their cell, to one contiguous run of the
+// sorted order, with the cell ranges; and the block's part of the other copy of
+// the counts cleared.  Returns false, having written nothing, when the record
+// says to sort fully (the block of slot 0 records the decision either way).
+// Every thread of the block calls it.  What bounds it is latency -- a block
+// goes from its loads through two or four barriers to its stores -- so every
+// load that needs no other is issued at the top, before the decision is known.
+template <bool FUSED>
+__device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh, int64_t blk) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t base = blk * kMergeBlockSlots;
-  const int64_t last = min(base + kMergeBlockSlots, a.n) - 1;
-
-  __shared__ unsigned long long span[kSpanCap];
-  __shared__ uint32_t nspan, red_a[kMergeThreads / 32], red_b[kMergeThreads / 32];
-  __shared__ uint32_t wpre[kMergeBlockSlots / 32], wbits[kMergeBlockSlots / 32];
-  __syncthreads();  // (a block calling again reuses the shared arrays)
-  if (tid == 0) nspan = 0;
-  // the block's stayers: state loaded first (independent of the counts)
-  uint32_t key[kMergeSlots];
-  float2 p[kMergeSlots], vel[kMergeSlots];
+  const int64_t base = blk << kMergeShift;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t epoch = *(volatile const uint32_t*)a.rec.next_epoch;
+  uint32_t key[kMergeSlots], mw[kMergeSlots];
+  float2 p[kMergeSlots], v[kMergeSlots];
   int32_t id[kMergeSlots];
+#pragma unroll
+  for (int u = 0; u < kMergeSlots; ++u) {
+    const int64_t i = base + (u * kMergeWarps + warp) * 32 + lane;
+    const bool in = i < a.n;
+    mw[u] = in ? a.rec.mask[i >> 5] : ~0u;
+    key[u] = in ? a.keyB[i] : 0u;
+    p[u] = in ? a.posB[i] : make_float2(0.f, 0.f);
+    v[u] = in ? a.velB[i] : make_float2(0.f, 0.f);
+    id[u] = in && a.idsA ? a.idsB[i] : 0;
+  }
+  // the slots either side of the block, which nearly always decide its neighbours' keys
+  const int64_t side = warp == 2 ? base - 1 : base + kMergeBlockSlots;
+  const bool has_side = warp >= 2 && side >= 0 && side < a.n;
+  const uint32_t side_mask = has_side ? a.rec.mask[side >> 5] : 0u;
+  const uint32_t side_key = has_side ? a.keyB[side] : 0u;
+  const MoverCounts r = mover_counts(a.rec, epoch);
+  if (warp == 1) {
+    uint32_t movers;
+    const bool merge = merge_wanted(a, r.total, &movers);
+    if (lane == 0) {
+      sh.merge = merge;
+      if (blk == 0) merge_decided(a, merge, movers, epoch);
+    }
+  }
+  uint32_t c[kMergeSlots], cex[kMergeSlots];
+#pragma unroll
+  for (int u = 0; u < kMergeSlots; ++u) {
+    const int64_t i = base + (u * kMergeWarps + warp) * 32 + lane;
+    c[u] = i <= a.n ? merge_inserted(r.insc, i) : 0u;
+  }
+  const uint32_t side_ins = has_side ? merge_inserted(r.insc, side) : 0u;
+  // slots before the block whose movers left, movers inserted before it
+  int32_t d = 0;
+  const int64_t sup = blk >> kMergeSupShift, b0 = sup << kMergeSupShift;
+  for (int64_t q = tid; q < sup; q += kMergeThreads) d += r.sup_net[q];
+  if (tid < blk - b0) d += r.blk_net[b0 + tid];
+  if (warp == 2) {
+    uint32_t k = kNoIndex;
+    if (has_side) {
+      k = side_key;
+      if ((side_mask >> (side & 31)) & 1u) k = merge_prev_key(a, r.insc, base, lane);
+    }
+    if (lane == 0) sh.prev = k;
+  } else if (warp == 3) {
+    uint32_t k = side_key;
+    if (!has_side || side_ins || ((side_mask >> (side & 31)) & 1u)) k = merge_next_key(a, r.insc, side, lane);
+    if (lane == 0) sh.next = k;
+  }
   bool stay[kMergeSlots];
 #pragma unroll
   for (int u = 0; u < kMergeSlots; ++u) {
-    const int64_t i = base + (int64_t)u * kMergeThreads + tid;
-    stay[u] = false;
-    key[u] = 0;
-    id[u] = 0;
-    p[u] = vel[u] = make_float2(0.f, 0.f);
-    if (i < a.n) {
-      const uint32_t mw = __ldg(a.mask + (i >> 5));
-      stay[u] = !((mw >> (i & 31)) & 1u);
-      if (stay[u]) {
-        key[u] = merge_load<COHERENT>(a.keyA + i);
-        p[u] = a.posB[i];
-        vel[u] = a.velB[i];
-        if (a.idsA) id[u] = a.idsB[i];
+    const int w = u * kMergeWarps + warp;
+    stay[u] = !((mw[u] >> lane) & 1u);
+    const unsigned sb = __ballot_sync(0xffffffffu, stay[u]);
+    uint32_t incl = c[u];
+    if (__any_sync(0xffffffffu, c[u] != 0u)) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+    }
+    cex[u] = incl - c[u];
+    if (lane == 31) {
+      sh.stay[w] = sb;
+      sh.tot[w] = ((uint32_t)__popc(sb) + incl) | (incl << 16);
+    }
+  }
+  d = __reduce_add_sync(0xffffffffu, d);
+  if (lane == 0) sh.red[warp] = d;
+  __syncthreads();
+  if (!sh.merge) return false;
+  {  // the other copy, which this iteration's force pass adds to
+    const MoverCounts o = mover_counts(a.rec, epoch + 1u);
+    if (base + 4 * tid <= a.n) o.insc[(base >> 2) + tid] = 0u;
+    if (tid == 0) {
+      o.blk_net[blk] = 0;
+      o.blk_ins[blk] = 0u;
+      if (blk == b0) o.sup_net[sup] = 0;
+    }
+    if (blk == 0 && tid < kMoverCounters)
+      o.total[tid * kMoverCounterStride] = o.total[tid * kMoverCounterStride + 1] = 0u;
+  }
+  // the same of the words before each word (every warp scans the block's words)
+  uint32_t off, all;
+  {
+    const uint32_t t = lane < kMergeWords ? sh.tot[lane] : 0u;
+    uint32_t incl = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    off = incl - t;
+    all = __shfl_sync(0xffffffffu, incl, 31);
+  }
+  int64_t out0 = base;
+#pragma unroll
+  for (int w = 0; w < kMergeWarps; ++w) out0 += sh.red[w];
+  const uint32_t total = all & 0xffffu, nins = all >> 16;
+  // a consistent record stays inside the buffers; anything else is reported, not written
+  if (out0 < 0 || out0 + (int64_t)total > a.n || nins > (uint32_t)kBlockInsertCap) {
+    if (tid == 0) a.ctl[2] = 1u;
+    __syncthreads();
+    return true;
+  }
+#pragma unroll
+  for (int u = 0; u < kMergeSlots; ++u) {
+    const int w = u * kMergeWarps + warp;
+    const int64_t i = base + w * 32 + lane;
+    const uint32_t woff = __shfl_sync(0xffffffffu, off, w);
+    const uint32_t grp = (woff & 0xffffu) + (uint32_t)__popc(sh.stay[w] & lt) + cex[u];
+    if (stay[u]) {
+      const uint32_t q = grp + c[u];
+      const int64_t to = out0 + q;
+      sh.key[q] = key[u];
+      merge_store<FUSED>(a.posA + to, p[u]);
+      merge_store<FUSED>(a.velpA + to, make_float4(v[u].x, v[u].y, 0.f, 0.f));
+      merge_store<FUSED>(a.perm + to, (uint32_t)i);
+      if (a.idsA) merge_store<FUSED>(a.idsA + to, id[u]);
+    }
+    if (c[u]) {  // the movers inserted before slot i, in any order
+      const uint32_t l0 = (woff >> 16) + cex[u];
+      uint32_t m = a.rec.head[i];
+      for (uint32_t q = 0; q < c[u]; ++q) {
+        const bool ok = m < a.n;
+        sh.islot[l0 + q] = ok ? m : kNoIndex;
+        sh.ikey[l0 + q] = ok ? a.keyB[m] : 0u;
+        sh.igrp[l0 + q] = (l0 << 16) | c[u];
+        sh.iout[l0 + q] = grp;
+        if (ok) m = a.rec.next[m];
       }
     }
   }
-  if (tid < kMergeBlockSlots / 32) {
-    const int64_t w = (base >> 5) + tid;
-    wbits[tid] = (w << 5) < a.n ? __ldg(a.mask + w) : 0u;
-  }
-  const unsigned long long v0 = ((unsigned long long)merge_load<COHERENT>(a.keyA + base) << 32) | (uint32_t)base;
-  const unsigned long long v1 = ((unsigned long long)merge_load<COHERENT>(a.keyA + last) << 32) | (uint32_t)last;
   __syncthreads();
-  // over the mover list: movers before the block's first slot, movers ordered
-  // before its first (key, slot), and the movers inside its (key, slot) span
-  uint32_t ca = 0, cb = 0;
-  for (uint32_t q = tid; q < m; q += kMergeThreads) {
-    const unsigned long long e = __ldg(ml + q);
-    ca += (uint32_t)e < (uint64_t)base;
-    cb += e < v0;
-    if (e >= v0 && e <= v1) {
-      const uint32_t at = atomicAdd(&nspan, 1u);
-      if (at < kSpanCap) span[at] = e;
+  if (nins) {
+  for (uint32_t q = tid; q < nins; q += kMergeThreads) {
+    const uint32_t k = sh.ikey[q], s = sh.islot[q], g = sh.igrp[q];
+    uint32_t rank = 0;  // among its group, by (key, slot)
+    for (uint32_t r = g >> 16, e = r + (g & 0xffffu); r < e; ++r)
+      rank += sh.ikey[r] < k || (sh.ikey[r] == k && sh.islot[r] < s);
+    const uint32_t at = sh.iout[q] + rank;
+    if (s >= a.n || at >= total) {
+      a.ctl[2] = 1u;
+      continue;
     }
-  }
-  ca = __reduce_add_sync(0xffffffffu, ca);
-  cb = __reduce_add_sync(0xffffffffu, cb);
-  if (lane == 0) {
-    red_a[warp] = ca;
-    red_b[warp] = cb;
-  }
-  if (tid == 0) {
-    uint32_t run = 0;
-    for (int w = 0; w < kMergeBlockSlots / 32; ++w) {
-      wpre[w] = run;
-      run += __popc(wbits[w]);
-    }
+    const int64_t to = out0 + at;
+    sh.key[at] = k;
+    const float2 vm = a.velB[s];
+    merge_store<FUSED>(a.posA + to, a.posB[s]);
+    merge_store<FUSED>(a.velpA + to, make_float4(vm.x, vm.y, 0.f, 0.f));
+    merge_store<FUSED>(a.perm + to, s);
+    if (a.idsA) merge_store<FUSED>(a.idsA + to, a.idsB[s]);
   }
   __syncthreads();
-  uint32_t before_block = 0, before_v0 = 0;
-#pragma unroll
-  for (int w = 0; w < kMergeThreads / 32; ++w) {
-    before_block += red_a[w];
-    before_v0 += red_b[w];
   }
-  const uint32_t ns = nspan;
-#pragma unroll
-  for (int u = 0; u < kMergeSlots; ++u) {
-    if (!stay[u]) continue;
-    const int64_t i = base + (int64_t)u * kMergeThreads + tid;
-    const int wl = (int)((i - base) >> 5);
-    const uint32_t slot_before = before_block + wpre[wl] + __popc(wbits[wl] & ((1u << (i & 31)) - 1u));
-    const unsigned long long v = ((unsigned long long)key[u] << 32) | (uint32_t)i;
-    uint32_t key_before = before_v0;
-    if (ns <= (uint32_t)kSpanCap) {
-      for (uint32_t q = 0; q < ns; ++q) key_before += span[q] < v;
-    } else {  // many movers inside this block's span: count over the whole list
-      key_before = 0;
-      for (uint32_t q = 0; q < m; ++q) key_before += __ldg(ml + q) < v;
+  uint32_t* rg = reinterpret_cast<uint32_t*>(a.ranges);
+  for (uint32_t q = tid; q < total; q += kMergeThreads) {
+    const uint32_t k = sh.key[q];
+    const uint32_t kp = q ? sh.key[q - 1] : sh.prev, kn = q + 1 < total ? sh.key[q + 1] : sh.next;
+    const uint32_t i = (uint32_t)(out0 + q);
+    merge_store<FUSED>(a.keyA + i, k);
+    if (k != kp) {
+      merge_store<FUSED>(rg + 4 * (size_t)k, i);
+      merge_store<FUSED>(rg + 4 * (size_t)k + 2, epoch);
     }
-    const int64_t fin = i - (int64_t)slot_before + key_before;
-    if (fin >= 0 && fin < a.n) merge_place<COHERENT>(a, i, fin, key[u], p[u], vel[u], id[u]);
-    else a.ctl[2] = 1u;
+    if (k != kn) merge_store<FUSED>(rg + 4 * (size_t)k + 1, i + 1u);
   }
-  // the movers, shared out over the blocks: one warp each
-  if (nblk == 0) return;  // placed by blocks of their own (merge_movers)
-  const uint32_t per = (m + nblk - 1) / nblk;
-  const uint32_t q0 = (uint32_t)blk * per, q1 = min(q0 + per, m);
-  for (uint32_t q = q0 + warp; q < q1; q += kMergeThreads / 32) merge_mover<COHERENT>(a, q, m, lane);
-}
-
-// Movers wq, wq + nw, ... of the list, one warp each (every lane calls it).
-template <bool COHERENT>
-__device__ __forceinline__ void merge_movers(const MoverArgs& a, uint32_t wq, uint32_t nw, uint32_t m) {
-  const int lane = threadIdx.x & 31;
-  for (uint32_t q = wq; q < m; q += nw) merge_mover<COHERENT>(a, q, m, lane);
+  __syncthreads();  // (a block calling again reuses the shared arrays)
+  return true;
 }
 
 }  // namespace sphg

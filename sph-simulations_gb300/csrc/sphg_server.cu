@@ -388,9 +388,23 @@ sphg_status append(sphg_server* s, const std::vector<int64_t>& ids, cudaStream_t
   SPHG_CUDA(cudaGetLastError());
   // no mover bits for the new slots (the word holding slot n_old - 1 was
   // written by the last force pass with zeros above it)
+  // and no movers inserted among them (the record of p = n_old stands: movers
+  // ordered after every old slot come before the newcomers, whose keys are larger)
   if (sim->movers_on) {
+    const sphg::MoverRecord& r = sim->mrec;
     const int64_t w0 = (n_old + 31) / 32, w1 = (L.n + 31) / 32;
-    if (w1 > w0) SPHG_CUDA(cudaMemsetAsync(sim->mmask + w0, 0, (w1 - w0) * sizeof(uint32_t), st));
+    if (w1 > w0) SPHG_CUDA(cudaMemsetAsync(r.mask + w0, 0, (w1 - w0) * sizeof(uint32_t), st));
+    const int sh = sphg::kMergeShift + sphg::kMergeSupShift;
+    const int64_t p0 = n_old > 0 ? n_old + 1 : 0;
+    const int64_t b0 = n_old > 0 ? (n_old >> sphg::kMergeShift) + 1 : 0, b1 = (L.n >> sphg::kMergeShift) + 1;
+    const int64_t s0 = n_old > 0 ? (n_old >> sh) + 1 : 0, s1 = (L.n >> sh) + 1;
+    for (uint32_t copy = 0; copy < 2; ++copy) {
+      const sphg::MoverCounts c = sphg::mover_counts(r, copy);
+      SPHG_CUDA(cudaMemsetAsync(reinterpret_cast<uint8_t*>(c.insc) + p0, 0, L.n + 1 - p0, st));
+      if (b1 > b0) SPHG_CUDA(cudaMemsetAsync(c.blk_net + b0, 0, (b1 - b0) * sizeof(int32_t), st));
+      if (b1 > b0) SPHG_CUDA(cudaMemsetAsync(c.blk_ins + b0, 0, (b1 - b0) * sizeof(uint32_t), st));
+      if (s1 > s0) SPHG_CUDA(cudaMemsetAsync(c.sup_net + s0, 0, (s1 - s0) * sizeof(int32_t), st));
+    }
   }
   SPHG_TRY(apply(s, ents, L, st));
   for (size_t k = 0; k < ids.size(); ++k) {

@@ -6,9 +6,10 @@
 //                  afterwards the force pass computes the next keys)
 //                  (GenericNeighborSearch::SetParticleCellIds, GenericNeighborSearch.h:201-231)
 //   [re-sort]      stable order of (key, slot): merge of the slots that changed
-//                  cell, or the full radix sort (SortParticleIds, :69-76)
-//   step_reorder   cell ranges (and, after a full sort, the gather of the state
-//                  into key order) (SortContainer :111-191, SetCellRanges :93-108)
+//                  cell, which also writes the sorted state and the cell ranges,
+//                  or the full radix sort (SortParticleIds, :69-76) and
+//   step_reorder   the gather of the state into key order and the cell ranges
+//                  (SortContainer :111-191, SetCellRanges :93-108)
 //   step_density   3x3-stencil density + EOS pressure, stores p/rho^2 and 1/rho
 //                  (ApproximateDensity GenericForceComputation.tpp:35-130,
 //                   CalculatePressure :23-32, cuInvertDensity)
@@ -27,7 +28,6 @@
 #include <type_traits>
 #include <cuda_runtime.h>
 
-#include "sphg_movers.cuh"
 #include "sphg_movers_body.cuh"
 #include "sphg_neighbor.cuh"
 #include "sphg_step.cuh"
@@ -87,21 +87,22 @@ __global__ void __launch_bounds__(kThreads) step_keys(StepArgs a) {
 }
 
 // ---------------------------------------------------------------- reorder + cell ranges
+// After a full sort: the gather of the state into sorted order and the cell
+// ranges (the merge of the incremental re-sort writes both itself).
 // kReorderSlots slots per thread, strided by the block size (coalesced), their
 // keys loaded before any is used.
 constexpr int kReorderSlots = 4;
 
 template <bool FUSED>
 __device__ __forceinline__ void reorder_slot(const StepArgs& a, int64_t i, uint32_t k, uint32_t kprev,
-                                             uint32_t knext, bool gather, uint32_t ep) {
+                                             uint32_t knext, uint32_t ep) {
+  clear_mover_counts(a, i, ep);
   st_out<FUSED>(a.keyA + i, k);
-  if (gather) {  // after a full sort (a merge scattered the state already)
-    const uint32_t src = a.perm[i];
-    st_out<FUSED>(a.posA + i, a.posB[src]);
-    const float2 v = a.velB[src];
-    st_out<FUSED>(a.velpA + i, make_float4(v.x, v.y, 0.f, 0.f));
-    if (a.track_ids) st_out<FUSED>(a.idsA + i, a.idsB[src]);
-  }
+  const uint32_t src = a.perm[i];
+  st_out<FUSED>(a.posA + i, a.posB[src]);
+  const float2 v = a.velB[src];
+  st_out<FUSED>(a.velpA + i, make_float4(v.x, v.y, 0.f, 0.f));
+  if (a.track_ids) st_out<FUSED>(a.idsA + i, a.idsB[src]);
   uint32_t* r = reinterpret_cast<uint32_t*>(a.ranges);
   if (k != kprev) {
     st_out<FUSED>(r + 4 * (size_t)k, (uint32_t)i);
@@ -135,21 +136,18 @@ __device__ __forceinline__ void reorder_block(const StepArgs& a, int64_t blk) {
       kn[u] = i + 1 < a.n ? a.keyS[i + 1] : kNoIndex;
     }
   }
-  const bool gather = !(a.merged && *a.merged);
   const uint32_t ep = *a.epoch;
 #pragma unroll
   for (int u = 0; u < kReorderSlots; ++u) {
     const int64_t i = base + (int64_t)u * kThreads;
-    if (i < a.n) reorder_slot<FUSED>(a, i, k[u], kp[u], kn[u], gather, ep);
+    if (i < a.n) reorder_slot<FUSED>(a, i, k[u], kp[u], kn[u], ep);
   }
 }
 
 __global__ void __launch_bounds__(kThreads) step_reorder(StepArgs a) {
   cudaGridDependencySynchronize();  // the sorted keys (and the decision word) of the re-sort
   allow_next_kernel(a.early_next);
-  // the mover count of this iteration's force pass starts at zero (this
-  // iteration's re-sort, the kernel before, has read the last one)
-  if (a.mover_count && blockIdx.x == 0 && threadIdx.x == 0) *a.mover_count = 0;
+  if (a.merged && *a.merged) return;  // the merge wrote the sorted state and the ranges
   reorder_block<false>(a, blockIdx.x);
 }
 
@@ -685,23 +683,16 @@ template <int PREC, bool BATCHED, int MODE, bool CSR>
 __device__ __forceinline__ void force_slot(const StepArgs& a, int64_t i, const float2* unit) {
   // slots of a finished served instance are skipped (no pair, no integration, no mover bit)
   const bool valid = i < a.n && (!BATCHED || inst_ref<BATCHED>(a, i).active);
-  const bool track = MODE == kForceIntegrate && a.mover_mask != nullptr;
+  const bool track = MODE == kForceIntegrate && a.movers.mask != nullptr;
   uint32_t key = 0;
   if (valid) key = force_one<PREC, BATCHED, MODE, CSR>(a, i, unit);
   if (track) {
     // slots whose cell key changed, for the incremental re-sort: one bit per
-    // slot (a warp holds 32 consecutive slots) and (key, slot) appended to the
-    // mover list, one atomic per warp
+    // slot (a warp holds 32 consecutive slots) and the record of each
     const unsigned moved = __ballot_sync(0xffffffffu, valid && key != a.keyA[i]);
-    const int lane = threadIdx.x & 31;
-    if (lane == 0 && i < a.n) a.mover_mask[i >> 5] = moved;  // every word of the slots, skipped ones included
-    if (moved) {
-      uint32_t at = 0;
-      if (lane == 0) at = atomicAdd(a.mover_count, (uint32_t)__popc(moved));
-      at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(moved & ((1u << lane) - 1u));
-      if (((moved >> lane) & 1u) && at < (uint32_t)kMoverCap)
-        a.mover_list[at] = ((unsigned long long)key << 32) | (uint32_t)i;
-    }
+    if ((threadIdx.x & 31) == 0 && i < a.n) a.movers.mask[i >> 5] = moved;  // every word, skipped slots included
+    if (i == 0) *a.movers.next_epoch = *a.epoch + 1u;
+    if (moved) record_movers(a, (uint32_t)i, key, moved);
   }
 }
 
@@ -832,17 +823,16 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
 }
 
 // ---------------------------------------------------------------- the iteration in one launch
-// step_fused runs re-sort (merge) -> cell ranges -> density -> forces +
-// integration as four phases of ONE cooperative launch, separated by grid-wide
-// barriers, instead of four kernels: for small and medium workloads the
+// step_fused runs re-sort (merge + cell ranges) -> density -> forces +
+// integration as three phases of ONE cooperative launch, separated by grid-wide
+// barriers, instead of three kernels: for small and medium workloads the
 // kernel boundaries cost as much as the work.  Every phase is the same device
 // code as its stand-alone kernel (the same bits), over the blocks in a
 // grid-stride loop.  Data a phase writes and a later phase of the same launch
-// reads is stored past L1 (st.global.cg) and the merge reads the keys and cell
-// ranges the reorder will rewrite past L1 (ld.global.cg): no SM holds a stale
-// line of them.  When more than kMoverCap slots changed, the launch only
-// records that (merge_decide) and the full radix sort runs, followed by the
-// launch in "post" mode (ranges, density, forces).
+// reads is stored past L1 (st.global.cg) and read by no earlier phase: no SM
+// holds a stale line of it.  When too many slots changed, the launch only
+// records that (merge_decided) and the full radix sort runs, followed by the
+// launch in "post" mode (reorder + ranges, density, forces).
 constexpr int kBarrierSpinLimit = 1 << 22;  // about a quarter second of 64 ns sleeps
 
 // Grid-wide barrier of a cooperative launch: bar[0] counts arrivals, bar[1] is
@@ -875,6 +865,7 @@ __device__ __forceinline__ void grid_barrier(uint32_t* bar, uint32_t* err) {
 template <int PREC, bool BATCHED>
 __global__ void __launch_bounds__(kThreads, BATCHED ? 6 : 8) step_fused(StepArgs a, MoverArgs m, uint32_t* bar, uint32_t* err,
                                                           int post) {
+  __shared__ MergeShared merge_sh;
   __shared__ float2 unit[16];
   if (threadIdx.x < 16) {
     const int k = threadIdx.x;
@@ -883,17 +874,17 @@ __global__ void __launch_bounds__(kThreads, BATCHED ? 6 : 8) step_fused(StepArgs
   __syncthreads();
   const int64_t G = gridDim.x;
   if (!post) {
-    uint32_t movers = 0;
-    if (!merge_decide(m, blockIdx.x == 0 && threadIdx.x == 0, &movers)) return;  // the full sort runs instead
-    const int64_t nb = (a.n + kMergeBlockSlots - 1) / kMergeBlockSlots;
-    for (int64_t b = blockIdx.x; b < nb; b += G) merge_block<true>(m, b, (uint32_t)nb, movers);
-    grid_barrier(bar, err);
-  } else if (a.merged && *(volatile const uint32_t*)a.merged) {
-    return;  // stream-launched iteration that merged: nothing left for the post launch
+    uint32_t movers;
+    const bool merge = merge_wanted(m, mover_counts(m.rec, *(volatile const uint32_t*)m.rec.next_epoch).total, &movers);
+    const int64_t nb = (a.n >> kMergeShift) + 1;
+    for (int64_t b = blockIdx.x; b < nb && (merge || b == 0); b += G) merge_block<true>(m, merge_sh, b);
+    if (!merge) return;  // every block: the full sort runs instead
+  } else {
+    // stream-launched iteration that merged: nothing left for the post launch
+    if (a.merged && *(volatile const uint32_t*)a.merged) return;
+    const int64_t nr = (a.n + kThreads * kReorderSlots - 1) / (kThreads * kReorderSlots);
+    for (int64_t b = blockIdx.x; b < nr; b += G) reorder_block<true>(a, b);
   }
-  if (a.mover_count && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(a.mover_count, 0u);
-  const int64_t nr = (a.n + kThreads * kReorderSlots - 1) / (kThreads * kReorderSlots);
-  for (int64_t b = blockIdx.x; b < nr; b += G) reorder_block<true>(a, b);
   grid_barrier(bar, err);
   const int64_t np = (a.n + kThreads - 1) / kThreads;
   for (int64_t b = blockIdx.x; b < np; b += G) {

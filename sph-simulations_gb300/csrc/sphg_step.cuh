@@ -6,6 +6,7 @@
 
 #include "../../include/sphg.h"
 #include "sphg_common.cuh"
+#include "sphg_movers.cuh"
 
 namespace sphg {
 
@@ -30,8 +31,8 @@ struct StepArgs {
   float2* posA;
   float4* velpA;               // (vx, vy, p/rho^2, 1/rho)
   float* rho;
-  uint32_t* keyA;              // sorted global keys (written by the reorder)
-  const uint32_t* keyS;        // sort output: sorted keys, read by the reorder
+  uint32_t* keyA;              // sorted global keys (written by the merge or the reorder)
+  const uint32_t* keyS;        // full-sort output: sorted keys, read by the reorder
   uint4* ranges;               // [total keys] {start, end, epoch, 0}
   const uint32_t* epoch;       // current step's epoch (bumped by the sort)
   int32_t* idsA;
@@ -49,10 +50,8 @@ struct StepArgs {
   const uint32_t* csr_idx;     // j << 5 | tag entries, self included, list order
   int64_t csr_cap;             // entries csr_idx holds (the passes read no further)
   uint32_t* csr_overflow;      // set by the fill when the lists exceed csr_cap
-  const uint32_t* merged;      // non-null and set: this iteration's merge scattered the state (reorder: ranges only)
-  uint32_t* mover_mask;        // [ceil(n/32)] force pass: bit per slot whose key changed (or null)
-  unsigned long long* mover_list;  // [kMoverCap] force pass: key << 32 | slot of each changed slot
-  uint32_t* mover_count;       // changed slots recorded (zeroed before the force pass)
+  const uint32_t* merged;      // non-null and set: this iteration's merge sorted the state (the reorder returns)
+  MoverRecord movers;          // the force pass's record for the next merge (mask null: off)
   uint32_t* flags;             // [0] unused, [1] number of non-empty tiles this step
   // cell tiles (Morton order only; tile_bits == 0 disables them)
   int tile_bits;               // tiles of 2^tile_bits x 2^tile_bits cells
@@ -70,7 +69,6 @@ cudaError_t launch_keys(const StepArgs& a, int precision, cudaStream_t s);
 // post: after a full sort, ranges -> density -> forces).  bar: two zeroed words,
 // err: set when a grid barrier's wait gave up.  cudaErrorNotSupported when the
 // device cannot launch it cooperatively.
-struct MoverArgs;
 cudaError_t launch_fused(const StepArgs& a, const MoverArgs& m, int precision, uint32_t* bar, uint32_t* err,
                          bool post, cudaStream_t s);
 // Blocks of the fused launch for this handle (0: not available).
