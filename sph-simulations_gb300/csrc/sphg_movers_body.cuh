@@ -9,6 +9,7 @@
 
 #include "sphg_common.cuh"
 #include "sphg_movers.cuh"
+#include "sphg_neighbor.cuh"
 #include "sphg_step.cuh"
 
 namespace sphg {
@@ -160,10 +161,10 @@ __device__ __forceinline__ uint32_t merge_next_key(const MoverArgs& a, const uin
   return kNoIndex;
 }
 
-// Stores of data that a later phase of the same launch reads (FUSED) bypass L1.
-template <bool FUSED, class V>
+// Stores of data that a later phase of the same launch reads (kFused) bypass L1.
+template <int LAUNCH, class V>
 __device__ __forceinline__ void merge_store(V* p, V v) {
-  if constexpr (FUSED) __stcg(p, v);
+  if constexpr (LAUNCH == kFused) __stcg(p, v);
   else *p = v;
 }
 
@@ -187,7 +188,7 @@ struct MergeShared {
 // Every thread of the block calls it.  What bounds it is latency -- a block
 // goes from its loads through two or four barriers to its stores -- so every
 // load that needs no other is issued at the top, before the decision is known.
-template <bool FUSED>
+template <int LAUNCH>
 __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh, int64_t blk) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t base = blk << kMergeShift;
@@ -312,10 +313,10 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
       const uint32_t q = grp + c[u];
       const int64_t to = out0 + q;
       sh.key[q] = key[u];
-      merge_store<FUSED>(a.posA + to, p[u]);
-      merge_store<FUSED>(a.velpA + to, make_float4(v[u].x, v[u].y, 0.f, 0.f));
-      merge_store<FUSED>(a.perm + to, (uint32_t)i);
-      if (a.idsA) merge_store<FUSED>(a.idsA + to, id[u]);
+      merge_store<LAUNCH>(a.posA + to, p[u]);
+      merge_store<LAUNCH>(a.velpA + to, make_float4(v[u].x, v[u].y, 0.f, 0.f));
+      merge_store<LAUNCH>(a.perm + to, (uint32_t)i);
+      if (a.idsA) merge_store<LAUNCH>(a.idsA + to, id[u]);
     }
     if (c[u]) {  // the movers inserted before slot i, in any order
       const uint32_t l0 = (woff >> 16) + cex[u];
@@ -345,10 +346,10 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
     const int64_t to = out0 + at;
     sh.key[at] = k;
     const float2 vm = a.velB[s];
-    merge_store<FUSED>(a.posA + to, a.posB[s]);
-    merge_store<FUSED>(a.velpA + to, make_float4(vm.x, vm.y, 0.f, 0.f));
-    merge_store<FUSED>(a.perm + to, s);
-    if (a.idsA) merge_store<FUSED>(a.idsA + to, a.idsB[s]);
+    merge_store<LAUNCH>(a.posA + to, a.posB[s]);
+    merge_store<LAUNCH>(a.velpA + to, make_float4(vm.x, vm.y, 0.f, 0.f));
+    merge_store<LAUNCH>(a.perm + to, s);
+    if (a.idsA) merge_store<LAUNCH>(a.idsA + to, a.idsB[s]);
   }
   __syncthreads();
   }
@@ -357,12 +358,12 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
     const uint32_t k = sh.key[q];
     const uint32_t kp = q ? sh.key[q - 1] : sh.prev, kn = q + 1 < total ? sh.key[q + 1] : sh.next;
     const uint32_t i = (uint32_t)(out0 + q);
-    merge_store<FUSED>(a.keyA + i, k);
+    merge_store<LAUNCH>(a.keyA + i, k);
     if (k != kp) {
-      merge_store<FUSED>(rg + 4 * (size_t)k, i);
-      merge_store<FUSED>(rg + 4 * (size_t)k + 2, epoch);
+      merge_store<LAUNCH>(rg + 4 * (size_t)k, i);
+      merge_store<LAUNCH>(rg + 4 * (size_t)k + 2, epoch);
     }
-    if (k != kn) merge_store<FUSED>(rg + 4 * (size_t)k + 1, i + 1u);
+    if (k != kn) merge_store<LAUNCH>(rg + 4 * (size_t)k + 1, i + 1u);
   }
   __syncthreads();  // (a block calling again reuses the shared arrays)
   return true;

@@ -14,6 +14,20 @@
 
 namespace sphg {
 
+// How the device code of an iteration is launched: a kernel per phase, one
+// cooperative launch per iteration (step_fused), or many iterations in one
+// cluster (step_resident).
+enum LaunchKind { kKernels = 0, kFused = 1, kResident = 2 };
+
+// Loads of state that the kernel itself does not write go through the
+// read-only path; the resident kernel rewrites all of it, so there they are
+// plain loads, ordered by its barriers.
+template <int LAUNCH, class V>
+__device__ __forceinline__ V ld_state(const V* p) {
+  if constexpr (LAUNCH == kResident) return *p;
+  else return __ldg(p);
+}
+
 // Constants of the instance owning slot i (by value so they live in registers).
 // Batched: the instance of the first slot of i's 256-slot block from a table
 // built with the layout, then forward over the (rare) instance starts inside
@@ -220,15 +234,15 @@ __device__ __forceinline__ void stencil_keys(const InstDesc& d, uint32_t code, i
 // the main pass and decided by a second pass over the same cells, which keeps
 // the FP64 code out of the hot loop; only the summation order of those rare
 // pairs differs.
-template <int PREC, bool ORDERED = false, class F>
+template <int PREC, bool ORDERED = false, int LAUNCH = kKernels, class F>
 __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstDesc& d,
                                                   uint32_t key, float2 pi, int& cx, int& cy,
                                                   F&& visit) {
   const uint32_t code = key - d.cell_base;
   decode_code(d, code, cx, cy);
   const uint32_t ep = *a.epoch;
-  const uint4* __restrict__ ranges = a.ranges;
-  const float2* __restrict__ pos = a.posA;
+  const uint4* ranges = a.ranges;
+  const float2* pos = a.posA;
   uint32_t c[9], valid, wrapmask;
   stencil_keys(d, code, cx, cy, c, valid, wrapmask);
   uint32_t rs[9], re[9];
@@ -236,7 +250,7 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstD
   for (int k = 0; k < 9; ++k) {
     rs[k] = re[k] = 0;
     if ((valid >> k) & 1u) {
-      const uint4 e = __ldg(ranges + c[k]);
+      const uint4 e = ld_state<LAUNCH>(ranges + c[k]);
       if (e.z == ep) {
         rs[k] = e.x;
         re[k] = e.y;
@@ -268,7 +282,7 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstD
         }
       }
     };
-    for (uint32_t j = rs[k]; j < re[k]; ++j) candidate(j, __ldg(pos + j));
+    for (uint32_t j = rs[k]; j < re[k]; ++j) candidate(j, ld_state<LAUNCH>(pos + j));
   }
   if (ORDERED || !border) return;
 #pragma unroll 1
@@ -282,7 +296,7 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstD
     for (int q = 0; q < 9; ++q)
       if (q == k) { s = rs[q]; e = re[q]; }
     for (uint32_t j = s; j < e; ++j) {
-      const float2 pj = __ldg(pos + j);
+      const float2 pj = ld_state<LAUNCH>(pos + j);
       const float dx = (pi.x - pj.x) - shx;
       const float dy = (pi.y - pj.y) - shy;
       const float r2 = fmaf(dx, dx, dy * dy);

@@ -39,9 +39,9 @@ constexpr int kThreads = 128;  // 128-thread blocks: measured a little faster th
 // Stores of the phase outputs that a later phase of the fused single-launch
 // iteration (step_fused) reads: there they bypass L1 (st.global.cg), so no
 // SM keeps a partial line of data other SMs write in the same launch.
-template <bool FUSED, class V>
+template <int LAUNCH, class V>
 __device__ __forceinline__ void st_out(V* p, V v) {
-  if constexpr (FUSED) __stcg(p, v);
+  if constexpr (LAUNCH == kFused) __stcg(p, v);
   else *p = v;
 }
 
@@ -93,22 +93,22 @@ __global__ void __launch_bounds__(kThreads) step_keys(StepArgs a) {
 // keys loaded before any is used.
 constexpr int kReorderSlots = 4;
 
-template <bool FUSED>
+template <int LAUNCH>
 __device__ __forceinline__ void reorder_slot(const StepArgs& a, int64_t i, uint32_t k, uint32_t kprev,
                                              uint32_t knext, uint32_t ep) {
   clear_mover_counts(a, i, ep);
-  st_out<FUSED>(a.keyA + i, k);
+  st_out<LAUNCH>(a.keyA + i, k);
   const uint32_t src = a.perm[i];
-  st_out<FUSED>(a.posA + i, a.posB[src]);
+  st_out<LAUNCH>(a.posA + i, a.posB[src]);
   const float2 v = a.velB[src];
-  st_out<FUSED>(a.velpA + i, make_float4(v.x, v.y, 0.f, 0.f));
-  if (a.track_ids) st_out<FUSED>(a.idsA + i, a.idsB[src]);
+  st_out<LAUNCH>(a.velpA + i, make_float4(v.x, v.y, 0.f, 0.f));
+  if (a.track_ids) st_out<LAUNCH>(a.idsA + i, a.idsB[src]);
   uint32_t* r = reinterpret_cast<uint32_t*>(a.ranges);
   if (k != kprev) {
-    st_out<FUSED>(r + 4 * (size_t)k, (uint32_t)i);
-    st_out<FUSED>(r + 4 * (size_t)k + 2, ep);
+    st_out<LAUNCH>(r + 4 * (size_t)k, (uint32_t)i);
+    st_out<LAUNCH>(r + 4 * (size_t)k + 2, ep);
   }
-  if (k != knext) st_out<FUSED>(r + 4 * (size_t)k + 1, (uint32_t)(i + 1));
+  if (k != knext) st_out<LAUNCH>(r + 4 * (size_t)k + 1, (uint32_t)(i + 1));
   if (a.tile_bits) {
     const int sh = 2 * a.tile_bits;
     const uint32_t t = k >> sh;
@@ -122,7 +122,7 @@ __device__ __forceinline__ void reorder_slot(const StepArgs& a, int64_t i, uint3
 }
 
 // Reorder block blk: slots [blk * 512, blk * 512 + 512).
-template <bool FUSED>
+template <int LAUNCH>
 __device__ __forceinline__ void reorder_block(const StepArgs& a, int64_t blk) {
   const int64_t base = blk * (kThreads * kReorderSlots) + threadIdx.x;
   uint32_t k[kReorderSlots], kp[kReorderSlots], kn[kReorderSlots];
@@ -140,7 +140,7 @@ __device__ __forceinline__ void reorder_block(const StepArgs& a, int64_t blk) {
 #pragma unroll
   for (int u = 0; u < kReorderSlots; ++u) {
     const int64_t i = base + (int64_t)u * kThreads;
-    if (i < a.n) reorder_slot<FUSED>(a, i, k[u], kp[u], kn[u], ep);
+    if (i < a.n) reorder_slot<LAUNCH>(a, i, k[u], kp[u], kn[u], ep);
   }
 }
 
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads) step_reorder(StepArgs a) {
   cudaGridDependencySynchronize();  // the sorted keys (and the decision word) of the re-sort
   allow_next_kernel(a.early_next);
   if (a.merged && *a.merged) return;  // the merge wrote the sorted state and the ranges
-  reorder_block<false>(a, blockIdx.x);
+  reorder_block<kKernels>(a, blockIdx.x);
 }
 
 // ---------------------------------------------------------------- density + pressure
@@ -179,12 +179,30 @@ __device__ __forceinline__ void entry_vec(const InstDesc& d, float2 pi, float2 p
 constexpr bool kDensityTrim = SPHG_DENSITY_TRIM != 0;
 
 
-template <int PREC, bool BATCHED, bool CSR, int T = kThreads>
-__global__ void __launch_bounds__(T) step_density(StepArgs a);
+// A queued stencil cell: {j0 << 5 | tag, j1 << 5 | tag} and, in split precision,
+// the shift of its offsets.  Plain positions need no shift: half the shared
+// memory, the rest of it L1 (512 x 512 vortex 49.0 -> 47.6 us an iteration; split
+// precision with the shift looked up by tag instead measured slower, the 1M dam
+// break 97.3 against 94.1 us, the batch 456 against 450).
+template <int PREC>
+using QueuedCell = typename std::conditional<PREC == 1, uint4, uint2>::type;
+constexpr int kQueuedCells = 10;  // the stencil's nine, the own cell split at the particle
+template <int PREC>
+__device__ __forceinline__ QueuedCell<PREC> queued_cell(uint32_t j0, uint32_t j1, uint32_t tag, float shx, float shy) {
+  if constexpr (PREC == 1)
+    return make_uint4((j0 << 5) | tag, (j1 << 5) | tag, __float_as_uint(shx), __float_as_uint(shy));
+  else return make_uint2((j0 << 5) | tag, (j1 << 5) | tag);
+}
+template <int PREC>
+__device__ __forceinline__ float2 cell_shift(const QueuedCell<PREC>& w) {
+  if constexpr (PREC == 1) return make_float2(__uint_as_float(w.z), __uint_as_float(w.w));
+  else return make_float2(0.f, 0.f);
+}
 
-// Density + pressure of particle i (i < n); FUSED: the outputs bypass L1 (st_out).
-template <int PREC, bool BATCHED, bool CSR, int T, bool FUSED>
-__device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
+// Density + pressure of particle i (i < n).  s_cells: the block's queue, one
+// column per thread.
+template <int PREC, bool BATCHED, bool CSR, int T, int LAUNCH>
+__device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, QueuedCell<PREC> (*s_cells)[T]) {
   typename std::conditional<BATCHED, const InstDesc&, const InstDesc>::type d = inst_ref<BATCHED>(a, i);
   if (BATCHED && !d.active) return;  // a finished served instance
   const uint32_t key = a.keyA[i];
@@ -204,8 +222,7 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
       S.add(t * t * t);
     }
   } else {
-    __shared__ uint4 s_cells[10][T];  // per thread: its non-empty stencil cells (own cell split at itself)
-    uint32_t* __restrict__ nbr = a.nbr;
+    uint32_t* nbr = a.nbr;
     const uint32_t slots = (uint32_t)a.nbr_slots;
     const size_t n = (size_t)a.n;
     uint32_t cnt = 0;
@@ -213,7 +230,7 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
       const float t = fmaf(-r2, inv_h2, 1.0f);
       S.add(t * t * t);
       if (nbr && (e >> 5) != (uint32_t)i) {  // record the pair for the force pass
-        if (cnt < slots) st_out<FUSED>(nbr + cnt * n + i, e);
+        if (cnt < slots) st_out<LAUNCH>(nbr + cnt * n + i, e);
         ++cnt;
       }
     };
@@ -238,7 +255,7 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
       stencil_keys(d, code, cx, cy, c, valid, wrapmask);
       uint4 r[9];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) r[k] = ((valid >> k) & 1u) ? __ldg(a.ranges + c[k]) : make_uint4(0, 0, 0, 0);
+      for (int k = 0; k < 9; ++k) r[k] = ((valid >> k) & 1u) ? ld_state<LAUNCH>(a.ranges + c[k]) : make_uint4(0, 0, 0, 0);
       int nseg = 0;
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
@@ -251,18 +268,14 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
             // own cell without the particle itself (its term W(0) = 1 is added
             // first): [start, i) and (i, end), whichever are not empty
             const uint32_t self = (uint32_t)i;
-            if (self > r[k].x)
-              s_cells[nseg++][tid] = make_uint4((r[k].x << 5) | tag, (self << 5) | tag, 0u, 0u);
-            if (self + 1 < r[k].y)
-              s_cells[nseg++][tid] = make_uint4(((self + 1) << 5) | tag, (r[k].y << 5) | tag, 0u, 0u);
+            if (self > r[k].x) s_cells[nseg++][tid] = queued_cell<PREC>(r[k].x, self, tag, 0.f, 0.f);
+            if (self + 1 < r[k].y) s_cells[nseg++][tid] = queued_cell<PREC>(self + 1, r[k].y, tag, 0.f, 0.f);
             continue;
           }
-          s_cells[nseg][tid] = make_uint4((r[k].x << 5) | tag, (r[k].y << 5) | tag, __float_as_uint(shx),
-                                          __float_as_uint(shy));
-          ++nseg;
+          s_cells[nseg++][tid] = queued_cell<PREC>(r[k].x, r[k].y, tag, shx, shy);
         }
       }
-      const float2* __restrict__ pos = a.posA;
+      const float2* pos = a.posA;
       const float h2_lo = d.h2_lo, h2_hi = d.h2_hi;
       const bool record = nbr != nullptr;
       const uint32_t self = (uint32_t)i;
@@ -270,14 +283,14 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
       bool border = false;
       if (PREC == 1) S.add(1.0f);  // own term W(0) first (plain sums keep the walk's order)
       if (nseg > 0) {  // plain: always (the particle's own cell holds it); split: any other particle near
-        uint4 w = s_cells[0][tid];
+        QueuedCell<PREC> w = s_cells[0][tid];
         int q = 1;
         uint32_t jj = w.x, je = w.y;
-        float shx = __uint_as_float(w.z), shy = __uint_as_float(w.w);
-        float2 pj = __ldg(pos + (jj >> 5));
+        float2 sh = cell_shift<PREC>(w);
+        float2 pj = ld_state<LAUNCH>(pos + (jj >> 5));
         while (true) {
           uint32_t jn = jj + 32u, jen = je;
-          float shxn = shx, shyn = shy;
+          float2 shn = sh;
           bool more = true;
           if (jn == je) {
             if (q == nseg) {
@@ -287,15 +300,14 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
               ++q;
               jn = w.x;
               jen = w.y;
-              shxn = __uint_as_float(w.z);
-              shyn = __uint_as_float(w.w);
+              shn = cell_shift<PREC>(w);
             }
           }
           // one candidate ahead (past the last one: the end of its cell, at most
           // slot n -- the positions hold one entry more)
-          const float2 pn = __ldg(pos + ((kDensityTrim || more ? jn : jj) >> 5));
+          const float2 pn = ld_state<LAUNCH>(pos + ((kDensityTrim || more ? jn : jj) >> 5));
           const uint32_t j = jj >> 5;
-          const float2 dxy = sub2(sub2(pi, pj), make_float2(shx, shy));
+          const float2 dxy = PREC == 1 ? sub2(sub2(pi, pj), sh) : sub2(pi, pj);
           float dx = dxy.x, dy = dxy.y;
           float r2;
           bool in;
@@ -313,41 +325,40 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
           S.add_fast((PREC == 1 ? in && other : in) ? t * t * t : 0.0f);
           const bool rec = in && other && (kDensityTrim || record);
           if (rec && cnt < slots) {
-            st_out<FUSED>(rp, jj);
+            st_out<LAUNCH>(rp, jj);
             rp += n;
           }
           cnt += rec ? 1u : 0u;
           if (!more) break;
           jj = jn;
           je = jen;
-          shx = shxn;
-          shy = shyn;
+          sh = shn;
           pj = pn;
         }
       }
       if (border) {  // rare: pairs in the FP64 band, the same cells in the same order
 #pragma unroll 1
         for (int s = 0; s < nseg; ++s) {
-          const uint4 w = s_cells[s][tid];
+          const QueuedCell<PREC> w = s_cells[s][tid];
           const uint32_t tag = w.x & 31u;
           if (PREC == 0 && (tag & 16u)) continue;
           const int c1 = (int)(tag / 3) - 1, c2 = (int)(tag % 3) - 1;
-          const float sx = __uint_as_float(w.z), sy = __uint_as_float(w.w);
+          const float2 sh = cell_shift<PREC>(w);
           for (uint32_t e = w.x; e != w.y; e += 32u) {
-            const float2 pj = __ldg(pos + (e >> 5));
-            const float dx = (pi.x - pj.x) - sx;
-            const float dy = (pi.y - pj.y) - sy;
+            const float2 pj = ld_state<LAUNCH>(pos + (e >> 5));
+            const float dx = (pi.x - pj.x) - sh.x;
+            const float dy = (pi.y - pj.y) - sh.y;
             const float r2 = fmaf(dx, dx, dy * dy);
             if (r2 >= h2_lo && r2 <= h2_hi && pair_inside<PREC>(d, pi, pj, c1, c2, r2)) accept(e, r2);
           }
         }
       }
     } else {
-      for_each_neighbor<PREC>(a, d, key, pi, cx, cy, [&](uint32_t j, float, float, float r2, uint32_t tag) {
+      for_each_neighbor<PREC, false, LAUNCH>(a, d, key, pi, cx, cy, [&](uint32_t j, float, float, float r2, uint32_t tag) {
         accept((j << 5) | tag, r2);
       });
     }
-    if (nbr) st_out<FUSED>(a.ncount + i, cnt);
+    if (nbr) st_out<LAUNCH>(a.ncount + i, cnt);
   }
   float rho, drho;
   if constexpr (PREC == 1) {
@@ -359,17 +370,25 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i) {
   }
   const float inv = 1.0f / rho;
   const float P = d.k * drho * inv * inv;
-  st_out<FUSED>(a.rho + i, rho);
-  st_out<FUSED>(reinterpret_cast<float2*>(a.velpA + i) + 1, make_float2(P, inv));
+  st_out<LAUNCH>(a.rho + i, rho);
+  st_out<LAUNCH>(reinterpret_cast<float2*>(a.velpA + i) + 1, make_float2(P, inv));
 }
 
-template <int PREC, bool BATCHED, bool CSR, int T>
-__global__ void __launch_bounds__(T) step_density(StepArgs a) {
+// Threads per SM the density pass is compiled for.  Split precision, one
+// instance: nine 128-thread blocks; ten (the compiler's 48 registers) leave too
+// little of the shared memory to L1 beside their queues (hit rate 45 against
+// 78 %, 1M dam break 97.3 against 94.1 us an iteration).  The others take the
+// compiler's 56 registers, nine blocks too.
+constexpr int density_blocks(int prec, bool batched, int t) { return prec == 1 && !batched ? 1152 / t : 0; }
+
+template <int PREC, bool BATCHED, bool CSR, int T = kThreads>
+__global__ void __launch_bounds__(T, density_blocks(PREC, BATCHED, T)) step_density(StepArgs a) {
+  __shared__ QueuedCell<PREC> s_cells[CSR ? 1 : kQueuedCells][T];
   cudaGridDependencySynchronize();  // the sorted state and cell ranges of the reorder
   allow_next_kernel(a.early_next);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
-  density_particle<PREC, BATCHED, CSR, T, false>(a, i);
+  density_particle<PREC, BATCHED, CSR, T, kKernels>(a, i, s_cells);
 }
 
 // ---------------------------------------------------------------- density, two particles of a cell per thread
@@ -639,7 +658,7 @@ constexpr int kForceBatch = SPHG_FORCE_BATCH;  // recorded neighbours gathered t
 constexpr bool kSkipZeroViscosity = SPHG_SKIP_ZERO_VISCOSITY != 0;
 
 
-template <int PREC, bool BATCHED, int MODE, bool CSR>
+template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit);
 
 // Threads per SM the force pass is compiled for.  Split precision: 1,152
@@ -658,7 +677,7 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
 constexpr int force_threads_per_sm(int prec, bool batched) {
   return prec == 1 ? (batched ? SPHG_FORCE_BATCHED_THREADS_PER_SM : SPHG_FORCE_THREADS_PER_SM) : (batched ? 0 : 1024);
 }
-template <int PREC, bool BATCHED, int MODE, bool CSR>
+template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ void force_slot(const StepArgs& a, int64_t i, const float2* unit);
 
 template <int PREC, bool BATCHED, int MODE, bool CSR, int T = kThreads>
@@ -674,18 +693,18 @@ __global__ void __launch_bounds__(T, force_threads_per_sm(PREC, BATCHED) / T) st
   __syncthreads();
   cudaGridDependencySynchronize();  // densities, pressures and neighbour lists of the density pass
   allow_next_kernel(a.early_next);
-  force_slot<PREC, BATCHED, MODE, CSR>(a, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, unit);
+  force_slot<PREC, BATCHED, MODE, CSR, kKernels>(a, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, unit);
 }
 
 // Force pass of slot i (every thread of a warp calls it, i may be >= n): the
 // forces and, in integrate mode, the update, the new key and the mover record.
-template <int PREC, bool BATCHED, int MODE, bool CSR>
+template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ void force_slot(const StepArgs& a, int64_t i, const float2* unit) {
   // slots of a finished served instance are skipped (no pair, no integration, no mover bit)
   const bool valid = i < a.n && (!BATCHED || inst_ref<BATCHED>(a, i).active);
   const bool track = MODE == kForceIntegrate && a.movers.mask != nullptr;
   uint32_t key = 0;
-  if (valid) key = force_one<PREC, BATCHED, MODE, CSR>(a, i, unit);
+  if (valid) key = force_one<PREC, BATCHED, MODE, CSR, LAUNCH>(a, i, unit);
   if (track) {
     // slots whose cell key changed, for the incremental re-sort: one bit per
     // slot (a warp holds 32 consecutive slots) and the record of each
@@ -698,7 +717,7 @@ __device__ __forceinline__ void force_slot(const StepArgs& a, int64_t i, const f
 
 // Forces on particle i; in integrate mode also the update and the new key
 // (returned), in force-only mode the acceleration is stored.
-template <int PREC, bool BATCHED, int MODE, bool CSR>
+template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit) {
   // one instance: a copy of the kernel-argument descriptor; batched: a reference
   typename std::conditional<BATCHED, const InstDesc&, const InstDesc>::type d = inst_ref<BATCHED>(a, i);
@@ -711,7 +730,7 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
   const float h = d.h, kp = d.kp, kv = d.kv, tol2 = d.tol2;
   const float alpha_c0 = d.alpha_c0;
   const float rho_i = 1.0f / vi.w;
-  const float4* __restrict__ velp = a.velpA;
+  const float4* velp = a.velpA;
   auto pair_v = [&](const float4 vj, float dx, float dy) {
     const float r2 = fmaf(dx, dx, dy * dy);
     const float rinv = r2 > 0.f ? rsqrtf(r2) : 0.f;
@@ -741,7 +760,7 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
     }
     f.add(t);
   };
-  auto pair = [&](uint32_t j, float dx, float dy) { pair_v(__ldg(velp + j), dx, dy); };
+  auto pair = [&](uint32_t j, float dx, float dy) { pair_v(ld_state<LAUNCH>(velp + j), dx, dy); };
   int cx, cy;
   const uint32_t cnt = CSR ? 0u : (a.nbr ? a.ncount[i] : 0xffffffffu);
   if constexpr (CSR) {
@@ -775,11 +794,11 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
       float2 pj[B];
       float4 vj[B];
 #pragma unroll
-      for (int u = 0; u < B; ++u) e[u] = q + u < cnt ? __ldg(a.nbr + (q + u) * n + i) : self_e;
+      for (int u = 0; u < B; ++u) e[u] = q + u < cnt ? ld_state<LAUNCH>(a.nbr + (q + u) * n + i) : self_e;
 #pragma unroll
       for (int u = 0; u < B; ++u) {
-        pj[u] = __ldg(a.posA + (e[u] >> 5));
-        vj[u] = __ldg(velp + (e[u] >> 5));
+        pj[u] = ld_state<LAUNCH>(a.posA + (e[u] >> 5));
+        vj[u] = ld_state<LAUNCH>(velp + (e[u] >> 5));
       }
 #pragma unroll
       for (int u = 0; u < B; ++u) {
@@ -809,7 +828,7 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
   } else {
     // more neighbours than the density pass could record (or no record): the
     // stencil walk, pairs in the walk's order
-    for_each_neighbor<PREC>(a, d, key, pi, cx, cy, [&](uint32_t j, float dx, float dy, float, uint32_t) {
+    for_each_neighbor<PREC, false, LAUNCH>(a, d, key, pi, cx, cy, [&](uint32_t j, float dx, float dy, float, uint32_t) {
       if (j != (uint32_t)i) pair(j, dx, dy);
     });
   }
@@ -866,6 +885,7 @@ template <int PREC, bool BATCHED>
 __global__ void __launch_bounds__(kThreads, BATCHED ? 6 : 8) step_fused(StepArgs a, MoverArgs m, uint32_t* bar, uint32_t* err,
                                                           int post) {
   __shared__ MergeShared merge_sh;
+  __shared__ QueuedCell<PREC> s_cells[kQueuedCells][kThreads];
   __shared__ float2 unit[16];
   if (threadIdx.x < 16) {
     const int k = threadIdx.x;
@@ -877,23 +897,23 @@ __global__ void __launch_bounds__(kThreads, BATCHED ? 6 : 8) step_fused(StepArgs
     uint32_t movers;
     const bool merge = merge_wanted(m, mover_counts(m.rec, *(volatile const uint32_t*)m.rec.next_epoch).total, &movers);
     const int64_t nb = (a.n >> kMergeShift) + 1;
-    for (int64_t b = blockIdx.x; b < nb && (merge || b == 0); b += G) merge_block<true>(m, merge_sh, b);
+    for (int64_t b = blockIdx.x; b < nb && (merge || b == 0); b += G) merge_block<kFused>(m, merge_sh, b);
     if (!merge) return;  // every block: the full sort runs instead
   } else {
     // stream-launched iteration that merged: nothing left for the post launch
     if (a.merged && *(volatile const uint32_t*)a.merged) return;
     const int64_t nr = (a.n + kThreads * kReorderSlots - 1) / (kThreads * kReorderSlots);
-    for (int64_t b = blockIdx.x; b < nr; b += G) reorder_block<true>(a, b);
+    for (int64_t b = blockIdx.x; b < nr; b += G) reorder_block<kFused>(a, b);
   }
   grid_barrier(bar, err);
   const int64_t np = (a.n + kThreads - 1) / kThreads;
   for (int64_t b = blockIdx.x; b < np; b += G) {
     const int64_t i = b * kThreads + threadIdx.x;
-    if (i < a.n) density_particle<PREC, BATCHED, false, kThreads, true>(a, i);
+    if (i < a.n) density_particle<PREC, BATCHED, false, kThreads, kFused>(a, i, s_cells);
   }
   grid_barrier(bar, err);
   for (int64_t b = blockIdx.x; b < np; b += G)
-    force_slot<PREC, BATCHED, kForceIntegrate, false>(a, b * kThreads + threadIdx.x, unit);
+    force_slot<PREC, BATCHED, kForceIntegrate, false, kFused>(a, b * kThreads + threadIdx.x, unit);
 }
 
 // ---------------------------------------------------------------- diagnostics
