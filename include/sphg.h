@@ -98,7 +98,10 @@ typedef struct sphg_options {
                           SPHG_PRECISION_SPLIT: integer cell + FP32 in-cell offset,
                           compensated density/force sums */
   int32_t track_ids;   /* 1: carry each particle's creation index through the sorts */
-  int32_t use_graph;   /* 1: replay each step from a captured CUDA graph */
+  int32_t use_graph;   /* 1: replay each step from a captured CUDA graph; a single instance
+                          of up to 16,384 particles with default launch shapes runs up to
+                          128 iterations per launch in one thread-block cluster instead
+                          (the same results) */
   int32_t tile_bits;   /* density/force cell tiles of 2^b x 2^b cells staged in shared memory:
                           0 = default (off), 3..5 = that b (every instance in Morton order),
                           -1 = off (one thread per particle, L1-cached global loads) */

@@ -479,12 +479,29 @@ sphg_status build_graph(sphg_sim* s, bool header) {
   return SPHG_OK;
 }
 
+// Iterations of a small single instance run in one cluster, many a launch,
+// instead of a graph each (the same bits; other launch shapes only on request).
+static bool resident_on(const sphg_sim* s) {
+  return s->opt.use_graph && s->ninst == 1 && !s->force_batched && s->movers_on && s->nbr && !s->tile_bits &&
+         s->opt.compute == SPHG_COMPUTE_SORTED && s->opt.fused == 0 && s->opt.block_threads == 0 &&
+         s->opt.cell_pairs == 0 && s->n > 0 && s->n <= sphg::kResidentMaxN &&
+         sphg::resident_blocks(s->opt.precision) > 0;
+}
+
+static sphg_status run_resident(sphg_sim* s, int64_t k, double* headers, cudaStream_t st) {
+  if (k <= 0) return SPHG_OK;
+  SPHG_CUDA(sphg::launch_resident(s->args(), mover_args(s, 0), s->opt.precision, k, headers, s->diag_partials,
+                                  sphg::diag_chunks(s->n, 1, s->diag_chunks), st));
+  return SPHG_OK;
+}
+
 sphg_status run_steps(sphg_sim* s, int64_t k, cudaStream_t st, bool first = false) {
   if (s->n == 0) return SPHG_OK;
   if (first) {
     SPHG_TRY(enqueue_step(s, st, true));
     --k;
   }
+  if (resident_on(s)) return run_resident(s, k, nullptr, st);
   if (s->opt.use_graph) {
     SPHG_TRY(build_graph(s));
     for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(s->gexec, st));
@@ -801,7 +818,7 @@ sphg_status sphg_create_batch(int32_t ninst, const sphg_params* p, const int64_t
       !host_stage(s, (size_t)s->n * (sizeof(float2) * 2 + sizeof(float4) + sizeof(float) + sizeof(uint32_t))))
     st = fail(SPHG_OOM, "pinned host staging");
   // (lists mode: captured after the pre-loop has sized the list buffer)
-  const bool capture_now = s->opt.use_graph && s->opt.compute != SPHG_COMPUTE_LISTS;
+  const bool capture_now = s->opt.use_graph && s->opt.compute != SPHG_COMPUTE_LISTS && !resident_on(s);
   if (st == SPHG_OK && s->n > 0 && capture_now) st = build_graph(s);
   if (st == SPHG_OK && s->n > 0 && capture_now) st = build_graph(s, true);  // with step headers
   if (st != SPHG_OK) {
@@ -1093,6 +1110,7 @@ sphg_status sphg_step_headers(sphg_sim* s, int64_t nsteps, double* out, void* st
     }
     return SPHG_OK;
   }
+  if (resident_on(s)) return run_resident(s, nsteps, dv, st);
   const sphg::HeaderSlot h = {dv, 0u, 0u};
   SPHG_CUDA(cudaMemcpyAsync(s->hslot, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   if (s->opt.use_graph) {

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kMergeThreads) movers_merge(MoverArgs a) {
   __shared__ MergeShared sh;
   cudaGridDependencySynchronize();  // the mover record of the previous force pass
   allow_next_kernel(a.early_next);
-  merge_block<kKernels>(a, sh, blockIdx.x);
+  merge_block<kKernels>(a, sh, blockIdx.x, *(volatile const uint32_t*)a.rec.next_epoch);
 }
 
 }  // namespace

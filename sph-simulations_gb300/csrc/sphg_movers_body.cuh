@@ -168,6 +168,15 @@ __device__ __forceinline__ void merge_store(V* p, V v) {
   else *p = v;
 }
 
+// The barrier of a merge block's threads: a thread block, or one of several in
+// the resident kernel's blocks.
+template <int LAUNCH>
+__device__ __forceinline__ void merge_sync() {
+  if constexpr (LAUNCH == kResident)
+    asm volatile("barrier.sync %0, %1;" ::"r"(1u + threadIdx.x / kMergeThreads), "n"(kMergeThreads) : "memory");
+  else __syncthreads();
+}
+
 struct MergeShared {
   uint32_t stay[kMergeWords];            // bit per slot: it keeps its cell
   uint32_t tot[kMergeWords];             // stayers + insertions of the word | insertions << 16
@@ -185,15 +194,14 @@ struct MergeShared {
 // sorted order, with the cell ranges; and the block's part of the other copy of
 // the counts cleared.  Returns false, having written nothing, when the record
 // says to sort fully (the block of slot 0 records the decision either way).
-// Every thread of the block calls it.  What bounds it is latency -- a block
+// Every thread of the block calls it; epoch: *rec.next_epoch.  What bounds it is latency -- a block
 // goes from its loads through two or four barriers to its stores -- so every
 // load that needs no other is issued at the top, before the decision is known.
 template <int LAUNCH>
-__device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh, int64_t blk) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+__device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh, int64_t blk, uint32_t epoch) {
+  const int tid = threadIdx.x & (kMergeThreads - 1), lane = tid & 31, warp = tid >> 5;
   const int64_t base = blk << kMergeShift;
   const unsigned lt = (1u << lane) - 1u;
-  const uint32_t epoch = *(volatile const uint32_t*)a.rec.next_epoch;
   uint32_t key[kMergeSlots], mw[kMergeSlots];
   float2 p[kMergeSlots], v[kMergeSlots];
   int32_t id[kMergeSlots];
@@ -267,7 +275,7 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
   }
   d = __reduce_add_sync(0xffffffffu, d);
   if (lane == 0) sh.red[warp] = d;
-  __syncthreads();
+  merge_sync<LAUNCH>();
   if (!sh.merge) return false;
   {  // the other copy, which this iteration's force pass adds to
     const MoverCounts o = mover_counts(a.rec, epoch + 1u);
@@ -300,7 +308,7 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
   // a consistent record stays inside the buffers; anything else is reported, not written
   if (out0 < 0 || out0 + (int64_t)total > a.n || nins > (uint32_t)kBlockInsertCap) {
     if (tid == 0) a.ctl[2] = 1u;
-    __syncthreads();
+    merge_sync<LAUNCH>();
     return true;
   }
 #pragma unroll
@@ -331,7 +339,7 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
       }
     }
   }
-  __syncthreads();
+  merge_sync<LAUNCH>();
   if (nins) {
   for (uint32_t q = tid; q < nins; q += kMergeThreads) {
     const uint32_t k = sh.ikey[q], s = sh.islot[q], g = sh.igrp[q];
@@ -351,7 +359,7 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
     merge_store<LAUNCH>(a.perm + to, s);
     if (a.idsA) merge_store<LAUNCH>(a.idsA + to, a.idsB[s]);
   }
-  __syncthreads();
+  merge_sync<LAUNCH>();
   }
   uint32_t* rg = reinterpret_cast<uint32_t*>(a.ranges);
   for (uint32_t q = tid; q < total; q += kMergeThreads) {
@@ -365,7 +373,7 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
     }
     if (k != kn) merge_store<LAUNCH>(rg + 4 * (size_t)k + 1, i + 1u);
   }
-  __syncthreads();  // (a block calling again reuses the shared arrays)
+  merge_sync<LAUNCH>();  // (a block calling again reuses the shared arrays)
   return true;
 }
 

@@ -895,9 +895,10 @@ __global__ void __launch_bounds__(kThreads, BATCHED ? 6 : 8) step_fused(StepArgs
   const int64_t G = gridDim.x;
   if (!post) {
     uint32_t movers;
-    const bool merge = merge_wanted(m, mover_counts(m.rec, *(volatile const uint32_t*)m.rec.next_epoch).total, &movers);
+    const uint32_t epoch = *(volatile const uint32_t*)m.rec.next_epoch;
+    const bool merge = merge_wanted(m, mover_counts(m.rec, epoch).total, &movers);
     const int64_t nb = (a.n >> kMergeShift) + 1;
-    for (int64_t b = blockIdx.x; b < nb && (merge || b == 0); b += G) merge_block<kFused>(m, merge_sh, b);
+    for (int64_t b = blockIdx.x; b < nb && (merge || b == 0); b += G) merge_block<kFused>(m, merge_sh, b, epoch);
     if (!merge) return;  // every block: the full sort runs instead
   } else {
     // stream-launched iteration that merged: nothing left for the post launch
@@ -1021,6 +1022,80 @@ __device__ __forceinline__ DiagPart load_part(const DiagPart* p) {
   return r;
 }
 
+// The constants of an instance that the diagnostics use per particle.
+struct DiagConst {
+  float lo_x, hi_x, lo_y, hi_y, cs_x, cs_y, Lx, Ly, band;
+  uint32_t cell_base;
+  int order, nx;
+};
+__device__ __forceinline__ DiagConst diag_const(const InstDesc& d) {
+  DiagConst c;
+  c.lo_x = d.lo_x, c.hi_x = d.hi_x, c.lo_y = d.lo_y, c.hi_y = d.hi_y;
+  c.cs_x = d.cs_x, c.cs_y = d.cs_y, c.Lx = d.Lx, c.Ly = d.Ly;
+  c.band = 1.0e-6f * fmaxf(fabsf(d.hi_x - d.lo_x), fabsf(d.hi_y - d.lo_y));
+  c.cell_base = d.cell_base;
+  c.order = d.order, c.nx = d.nx;
+  return c;
+}
+
+// One particle into the partial v.
+template <int PREC>
+__device__ __forceinline__ void diag_particle(DiagPart& v, const InstDesc& d, const DiagConst& q, float2 vel, float2 p,
+                                              float rho, uint32_t key) {
+  const float p1 = vel.x * vel.x, e1 = fmaf(vel.x, vel.x, -p1);
+  const float p2 = vel.y * vel.y, e2 = fmaf(vel.y, vel.y, -p2);
+  v.e2.add(p1, e1);
+  v.e2.add(p2, e2);
+  v.mx.add(vel.x, 0.f);
+  v.my.add(vel.y, 0.f);
+  float h, l;
+  two_sum(p1, p2, h, l);
+  l += e1 + e2;
+  fast_two_sum(h, l, h, l);
+  if (h > v.mh || (h == v.mh && l > v.ml)) {
+    v.mh = h;
+    v.ml = l;
+  }
+  int cx = 0, cy = 0;
+  const float x = p.x, y = p.y;  // position, or offset in cell (cx, cy)
+  float lox = q.lo_x, hix = q.hi_x, loy = q.lo_y, hiy = q.hi_y;
+  if (PREC == 1) {
+    const uint32_t code = key - q.cell_base;
+    if (q.order == 0) {
+      cx = (int)compact1by1(code);
+      cy = (int)compact1by1(code >> 1);
+    } else {
+      cx = (int)(code % (uint32_t)q.nx);
+      cy = (int)(code / (uint32_t)q.nx);
+    }
+    lox = -(float)cx * q.cs_x;  // the walls in the cell's frame
+    hix = q.Lx - (float)cx * q.cs_x;
+    loy = -(float)cy * q.cs_y;
+    hiy = q.Ly - (float)cy * q.cs_y;
+  }
+  const bool fin = isfinite(x) && isfinite(y) && isfinite(vel.x) && isfinite(vel.y) && isfinite(rho);
+  bool in = fin && x >= lox && x <= hix && y >= loy && y <= hiy;
+  const bool near = fin && (fabsf(x - lox) <= q.band || fabsf(x - hix) <= q.band || fabsf(y - loy) <= q.band ||
+                            fabsf(y - hiy) <= q.band);
+  if (near) {
+    const double xd = PREC == 1 ? d.lo_xd + cx * d.cs_xd + (double)x : (double)x;
+    const double yd = PREC == 1 ? d.lo_yd + cy * d.cs_yd + (double)y : (double)y;
+    in = inside_d(xd, yd, d.lo_xd, d.hi_xd, d.lo_yd, d.hi_yd);
+  }
+  v.inside += in ? 1u : 0u;
+  v.bad += fin ? 0u : 1u;
+}
+
+// The six values of an instance's summed partials.
+__device__ __forceinline__ void diag_values(const DiagPart& f, double m, double* out) {
+  out[0] = 0.5 * m * f.e2.value();
+  out[1] = (double)f.mh + (double)f.ml;
+  out[2] = (double)f.inside;
+  out[3] = m * f.mx.value();
+  out[4] = m * f.my.value();
+  out[5] = (double)f.bad;
+}
+
 // One launch: every (chunk, instance) block reduces its particles into a
 // partial; the last block of an instance to finish (a ticket counter, reset
 // by it for the next launch) reduces the instance's partials into its six
@@ -1046,12 +1121,7 @@ __global__ void __launch_bounds__(kDiagThreads) step_diag(StepArgs a, int chunks
   const int64_t per = (cnt + ck - 1) / ck;
   const int64_t b = d.begin + per * chunk;
   const int64_t e = min((int64_t)d.end, b + per);
-  // the instance constants used per particle, in registers
-  const float lo_x = d.lo_x, hi_x = d.hi_x, lo_y = d.lo_y, hi_y = d.hi_y;
-  const float cs_x = d.cs_x, cs_y = d.cs_y, Lx = d.Lx, Ly = d.Ly;
-  const uint32_t cell_base = d.cell_base;
-  const int order = d.order, nx = d.nx;
-  const float band = 1.0e-6f * fmaxf(fabsf(hi_x - lo_x), fabsf(hi_y - lo_y));
+  const DiagConst dc = diag_const(d);  // in registers
   DiagPart v = {};
   // kDiagBatch particles per thread at a time: all their loads are issued
   // before any of them is used (the rare FP64 wall test is an out-of-line call
@@ -1066,58 +1136,14 @@ __global__ void __launch_bounds__(kDiagThreads) step_diag(StepArgs a, int chunks
       const int64_t i = i0 + (int64_t)u * blockDim.x;
       const bool ok = i < e;
       vb[u] = ok ? reinterpret_cast<const float2*>(a.velpA)[2 * i] : make_float2(0.f, 0.f);
-      pb[u] = ok ? a.posA[i] : make_float2(0.5f * (lo_x + hi_x), 0.5f * (lo_y + hi_y));
+      pb[u] = ok ? a.posA[i] : make_float2(0.5f * (dc.lo_x + dc.hi_x), 0.5f * (dc.lo_y + dc.hi_y));
       rb[u] = ok ? a.rho[i] : 1.f;
-      kb[u] = (PREC == 1 && ok) ? a.keyA[i] : cell_base;
+      kb[u] = (PREC == 1 && ok) ? a.keyA[i] : dc.cell_base;
     }
 #pragma unroll
     for (int u = 0; u < kDiagBatch; ++u) {
       if (i0 + (int64_t)u * blockDim.x >= e) break;
-      const float2 vel = vb[u];
-      const float2 p = pb[u];
-      const float rho = rb[u];
-      const float p1 = vel.x * vel.x, e1 = fmaf(vel.x, vel.x, -p1);
-      const float p2 = vel.y * vel.y, e2 = fmaf(vel.y, vel.y, -p2);
-      v.e2.add(p1, e1);
-      v.e2.add(p2, e2);
-      v.mx.add(vel.x, 0.f);
-      v.my.add(vel.y, 0.f);
-      float h, l;
-      two_sum(p1, p2, h, l);
-      l += e1 + e2;
-      fast_two_sum(h, l, h, l);
-      if (h > v.mh || (h == v.mh && l > v.ml)) {
-        v.mh = h;
-        v.ml = l;
-      }
-      int cx = 0, cy = 0;
-      const float x = p.x, y = p.y;  // position, or offset in cell (cx, cy)
-      float lox = lo_x, hix = hi_x, loy = lo_y, hiy = hi_y;
-      if (PREC == 1) {
-        const uint32_t code = kb[u] - cell_base;
-        if (order == 0) {
-          cx = (int)compact1by1(code);
-          cy = (int)compact1by1(code >> 1);
-        } else {
-          cx = (int)(code % (uint32_t)nx);
-          cy = (int)(code / (uint32_t)nx);
-        }
-        lox = -(float)cx * cs_x;  // the walls in the cell's frame
-        hix = Lx - (float)cx * cs_x;
-        loy = -(float)cy * cs_y;
-        hiy = Ly - (float)cy * cs_y;
-      }
-      const bool fin = isfinite(x) && isfinite(y) && isfinite(vel.x) && isfinite(vel.y) && isfinite(rho);
-      bool in = fin && x >= lox && x <= hix && y >= loy && y <= hiy;
-      const bool near = fin && (fabsf(x - lox) <= band || fabsf(x - hix) <= band || fabsf(y - loy) <= band ||
-                                fabsf(y - hiy) <= band);
-      if (near) {
-        const double xd = PREC == 1 ? d.lo_xd + cx * d.cs_xd + (double)x : (double)x;
-        const double yd = PREC == 1 ? d.lo_yd + cy * d.cs_yd + (double)y : (double)y;
-        in = inside_d(xd, yd, d.lo_xd, d.hi_xd, d.lo_yd, d.hi_yd);
-      }
-      v.inside += in ? 1u : 0u;
-      v.bad += fin ? 0u : 1u;
+      diag_particle<PREC>(v, d, dc, vb[u], pb[u], rb[u], kb[u]);
     }
   }
   __shared__ DiagPart sh[kDiagThreads / 32];
@@ -1137,21 +1163,191 @@ __global__ void __launch_bounds__(kDiagThreads) step_diag(StepArgs a, int chunks
   f = part_block_reduce(f, sh);
   if (threadIdx.x != 0) return;
   tickets[inst] = 0;
-  const double m = d.mass_d;
-  const double r[6] = {0.5 * m * f.e2.value(), (double)f.mh + (double)f.ml, (double)f.inside, m * f.mx.value(),
-                       m * f.my.value(), (double)f.bad};
   if (!SLOT) {
-    for (int q = 0; q < 6; ++q) out[inst * 6 + q] = r[q];
+    diag_values(f, d.mass_d, out + inst * 6);
     return;
   }
   const size_t k = *(volatile uint32_t*)&slot->k;
-  for (int q = 0; q < 6; ++q) slot->out[(k * a.ninst + inst) * 6 + q] = r[q];
+  diag_values(f, d.mass_d, slot->out + (k * a.ninst + inst) * 6);
   __threadfence();
   if (atomicAdd(&slot->done, 1u) == (uint32_t)a.ninst - 1u) {
     slot->done = 0;
     slot->k += 1;
     __threadfence();
   }
+}
+
+// ---------------------------------------------------------------- many iterations in one cluster
+// step_resident: one instance of up to kResidentMaxN particles, `iters`
+// iterations in one launch of one thread-block cluster (16 or 8 blocks of 1,024
+// threads, an SM each), the phases of an iteration -- merge, density, forces --
+// between cluster barriers.  A small iteration as a graph of kernels costs its
+// launches: 23 us an iteration of 1,023 particles, of which the host's graph
+// launch is nearly all, and 25 us of 12,800, whose three kernels and the
+// conditional node's decision take 5-8 us each however little they do.  A
+// cluster's blocks are scheduled together by the hardware, so the barriers need
+// no co-residency of the whole grid and several handles may run at once.  The
+// phases are the same device code as the kernels (the same bits); what one
+// phase wrote the next reads after a barrier with release / acquire order, by
+// plain loads.  An iteration the merge does not take (merge_wanted) is sorted
+// by counting, for every particle, the (key, slot) pairs before its own.
+// Measured, us an iteration, cluster against graph (split precision, 64
+// iterations a call): 1,023 particles 12.9 / 23.4, 6,400 14.8 / 25.1, 14,375
+// 18.4 / 25.3, 16,200 18.8 / 25.9, 20,300 25.5 / 25.8 (a second round of the
+// cluster's 16,384 threads), 32,400 30.2 / 27.0; one iteration a call 17.1 / 23.4
+// at 1,023, 22.9 / 26.0 at 16,200.
+constexpr int kResidentThreads = 1024;
+constexpr int kResidentGroups = kResidentThreads / kMergeThreads;   // merge blocks at a time
+constexpr int kResidentChunks = kResidentThreads / kDiagThreads;    // diagnostics chunks at a time
+constexpr int kResidentIters = 128;  // iterations a launch: launches amortised, about a millisecond at most
+
+template <int PREC>
+struct ResidentShared {
+  union {
+    QueuedCell<PREC> cells[kQueuedCells][kResidentThreads];
+    MergeShared merge[kResidentGroups];
+    uint4 keys[kResidentThreads / 4];
+  };
+  DiagPart warps[kResidentThreads / 32];
+  float2 unit[16];
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The stable sort of an iteration that the merge does not take: every thread
+// counts, over all keys, the slots ordered before its own.
+template <int PREC>
+__device__ __forceinline__ void resident_sort(const StepArgs& a, ResidentShared<PREC>& sh, uint32_t i0, uint32_t i1,
+                                              uint32_t epoch) {
+  const uint32_t n = (uint32_t)a.n, tid = threadIdx.x;
+  uint32_t* tile = reinterpret_cast<uint32_t*>(sh.keys);
+  for (uint32_t b = i0; b < i1; b += kResidentThreads) {
+    const uint32_t i = b + tid;
+    const bool in = i < i1;
+    const uint32_t k = in ? a.keyB[i] : 0u;
+    uint32_t rank = 0;
+    for (uint32_t t0 = 0; t0 < n; t0 += kResidentThreads) {
+      __syncthreads();
+      tile[tid] = t0 + tid < n ? a.keyB[t0 + tid] : kNoIndex;  // keys are below kNoIndex
+      __syncthreads();
+      if (t0 + kResidentThreads <= i) {  // every slot of the tile comes before i: ties count
+        for (int q = 0; q < kResidentThreads / 4; ++q) {
+          const uint4 t = sh.keys[q];
+          rank += (t.x <= k) + (t.y <= k) + (t.z <= k) + (t.w <= k);
+        }
+      } else {
+        for (int q = 0; q < kResidentThreads; ++q) rank += tile[q] < k || (tile[q] == k && t0 + q < i);
+      }
+    }
+    if (in) {
+      const float2 v = a.velB[i];
+      a.keyA[rank] = k;
+      a.perm[rank] = i;
+      a.posA[rank] = a.posB[i];
+      a.velpA[rank] = make_float4(v.x, v.y, 0.f, 0.f);
+      if (a.track_ids) a.idsA[rank] = a.idsB[i];
+    }
+  }
+  cluster_barrier();
+  uint32_t* r = reinterpret_cast<uint32_t*>(a.ranges);
+  for (uint32_t i = i0 + tid; i < i1; i += kResidentThreads) {
+    const uint32_t k = a.keyA[i];
+    if (i == 0 || a.keyA[i - 1] != k) {
+      r[4 * (size_t)k] = i;
+      r[4 * (size_t)k + 2] = epoch;
+    }
+    if (i + 1 == n || a.keyA[i + 1] != k) r[4 * (size_t)k + 1] = i + 1;
+    clear_mover_counts(a, i, epoch);
+  }
+}
+
+// The header of the iteration whose partials lie in parts (one warp group of
+// kDiagThreads threads; the fixed shape of step_diag's last block).
+__device__ __forceinline__ void resident_header(const StepArgs& a, const DiagPart* parts, int ck, DiagPart* warps,
+                                                double* out) {
+  const int t = threadIdx.x & (kDiagThreads - 1), lane = t & 31, w = t >> 5;
+  DiagPart f = {};
+  for (int c = t; c < ck; c += kDiagThreads) part_add(f, load_part(parts + c));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) part_add(f, part_shfl_down(f, o));
+  if (lane == 0) warps[w] = f;
+  asm volatile("barrier.sync 15, %0;" ::"n"(kDiagThreads) : "memory");
+  if (t == 0) {
+    for (int k = 1; k < kDiagThreads / 32; ++k) part_add(f, warps[k]);
+    diag_values(f, a.d0.mass_d, out);
+  }
+}
+
+template <int PREC>
+__global__ void __launch_bounds__(kResidentThreads, 1)
+    step_resident(StepArgs a, MoverArgs m, int iters, double* headers, DiagPart* parts, int ck) {
+  extern __shared__ __align__(16) unsigned char resident_smem[];
+  ResidentShared<PREC>& sh = *reinterpret_cast<ResidentShared<PREC>*>(resident_smem);
+  const uint32_t C = gridDim.x, cta = blockIdx.x;  // the grid is one cluster
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  if (tid < 16) {
+    const int k = (int)tid;
+    sh.unit[k] = k < 9 ? make_float2((float)(k / 3 - 1), (float)(k % 3 - 1)) : make_float2(0.f, 0.f);
+  }
+  const uint32_t n = (uint32_t)a.n;
+  const uint32_t per = ((n + C - 1) / C + 31) & ~31u;  // consecutive slots of a block, whole warps
+  const uint32_t i0 = min(n, cta * per), i1 = min(n, i0 + per);
+  const uint32_t nb = (n >> kMergeShift) + 1;
+  const DiagConst dc = diag_const(a.d0);
+  __syncthreads();
+  uint32_t epoch = *(volatile const uint32_t*)m.rec.next_epoch;
+  for (int it = 0; it < iters; ++it, ++epoch) {
+    // the decision is the same for every thread; a merge block takes it beside its loads
+    const uint32_t g = tid / kMergeThreads;
+    uint32_t b = g * C + cta, movers;
+    bool merge;
+    if (b < nb) {
+      merge = merge_block<kResident>(m, sh.merge[g], b, epoch);
+      for (b += C * kResidentGroups; merge && b < nb; b += C * kResidentGroups)
+        merge_block<kResident>(m, sh.merge[g], b, epoch);
+    } else {
+      merge = merge_wanted(m, mover_counts(m.rec, epoch).total, &movers);
+    }
+    if (!merge) {
+      if (cta == 0 && tid == 0) *m.epoch = epoch;
+      resident_sort<PREC>(a, sh, i0, i1, epoch);
+    }
+    // the header of the iteration before: by the block with the least of the merge
+    if (headers && it > 0 && cta == C - 1 && tid >= kResidentThreads - kDiagThreads)
+      resident_header(a, parts, ck, sh.warps, headers + 6 * (size_t)(it - 1));
+    cluster_barrier();
+    for (uint32_t i = i0 + tid; i < i1; i += kResidentThreads)
+      density_particle<PREC, false, false, kResidentThreads, kResident>(a, i, sh.cells);
+    cluster_barrier();
+    if (headers) {  // step_diag's chunks, kDiagThreads threads each
+      const uint32_t dper = (n + ck - 1) / ck;
+      for (uint32_t c0 = cta * kResidentChunks; c0 < (uint32_t)ck; c0 += C * kResidentChunks) {
+        const uint32_t c = c0 + tid / kDiagThreads, b = dper * c, e = min(n, b + dper);
+        DiagPart v = {};
+        if (c < (uint32_t)ck)
+          for (uint32_t i = b + tid % kDiagThreads; i < e; i += kDiagThreads) {
+            const float4 vp = a.velpA[i];
+            diag_particle<PREC>(v, a.d0, dc, make_float2(vp.x, vp.y), a.posA[i], a.rho[i], PREC == 1 ? a.keyA[i] : 0u);
+          }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part_add(v, part_shfl_down(v, o));
+        if (lane == 0) sh.warps[tid >> 5] = v;
+        __syncthreads();
+        if (tid % kDiagThreads == 0 && c < (uint32_t)ck) {
+          for (int k = 1; k < kDiagThreads / 32; ++k) part_add(v, sh.warps[(tid >> 5) + k]);
+          parts[c] = v;
+        }
+        __syncthreads();
+      }
+    }
+    for (uint32_t b = i0 + (tid & ~31u); b < i1; b += kResidentThreads)
+      force_slot<PREC, false, kForceIntegrate, false, kResident>(a, (int64_t)b + lane, sh.unit);
+    cluster_barrier();
+  }
+  if (headers && cta == C - 1 && tid >= kResidentThreads - kDiagThreads)
+    resident_header(a, parts, ck, sh.warps, headers + 6 * (size_t)(iters - 1));
 }
 
 // CFL inputs per (chunk, instance): FP64 maxima of |v|^2 and |a|^2 (a from the
@@ -1371,6 +1567,66 @@ cudaError_t launch_cell_keys_plain(const InstDesc& d, const float* x, const floa
                                    int32_t* keys, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   cell_keys_plain<<<blocks_for(n, kThreads), kThreads, 0, s>>>(d, x, y, n, keys);
+  return cudaGetLastError();
+}
+
+// Blocks of the resident cluster on this device (0: it cannot be launched).
+template <int PREC>
+static int resident_cluster() {
+  static const int blocks = [] {
+    const int smem = (int)sizeof(ResidentShared<PREC>);
+    const auto k = step_resident<PREC>;
+    int found = 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+      for (int c : {16, 8}) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(kResidentThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0) {
+          found = c;
+          break;
+        }
+      }
+    cudaGetLastError();
+    return found;
+  }();
+  return blocks;
+}
+
+int resident_blocks(int precision) { return precision ? resident_cluster<1>() : resident_cluster<0>(); }
+
+cudaError_t launch_resident(const StepArgs& a, const MoverArgs& m, int precision, int64_t iters, double* headers,
+                            double* partials, int chunks, cudaStream_t s) {
+  const int c = resident_blocks(precision);
+  if (c <= 0) return cudaErrorNotSupported;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(c);
+  cfg.blockDim = dim3(kResidentThreads);
+  cfg.dynamicSmemBytes = precision ? sizeof(ResidentShared<1>) : sizeof(ResidentShared<0>);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = c;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  DiagPart* parts = reinterpret_cast<DiagPart*>(partials);
+  for (int64_t k = 0; k < iters; k += kResidentIters) {
+    const int it = (int)std::min<int64_t>(kResidentIters, iters - k);
+    double* h = headers ? headers + 6 * k : nullptr;
+    const cudaError_t e = precision ? cudaLaunchKernelEx(&cfg, step_resident<1>, a, m, it, h, parts, chunks)
+                                    : cudaLaunchKernelEx(&cfg, step_resident<0>, a, m, it, h, parts, chunks);
+    if (e != cudaSuccess) return e;
+  }
   return cudaGetLastError();
 }
 

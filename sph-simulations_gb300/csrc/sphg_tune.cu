@@ -5,7 +5,7 @@
 // cells staged in shared memory, b = 3..5; tiles need every instance in Morton
 // order); without tiles, the particles per thread of the density pass (two of
 // a cell sharing the stencil walk, or one), the threads per block of the
-// density and force passes (64, 128, 256) and the re-sort strategy
+// density and force passes (64, 128 = default, 256) and the re-sort strategy
 // (incremental merge of the particles that changed cell, or the full radix
 // sort every iteration); and the iteration as one cooperative launch.  Each candidate gets its own handle with the caller's
 // state, runs the pre-loop and a few warm-up iterations, then `steps` timed
@@ -91,7 +91,7 @@ extern "C" sphg_status sphg_autotune(int32_t ninst, const sphg_params* p, const 
     // the iteration as one cooperative launch (merge re-sort, 128 threads, one particle per thread)
     if (b.compute == SPHG_COMPUTE_SORTED) cands.push_back({tb, 1, 128, 0, 1});
     for (int resort : {1, 0})
-      for (int block : {128, 64, 256})
+      for (int block : {0, 64, 256})  // 0: the default, 128 (a small instance's resident cluster)
         for (int pairs : {0, 1}) {
           if (b.compute == SPHG_COMPUTE_LISTS && pairs) continue;  // lists mode: no stencil walk in the density
           cands.push_back({tb, resort, block, pairs, 0});
