@@ -144,11 +144,13 @@ const char* sphg_version(void);
 sphg_status sphg_device_attributes(int32_t device, int32_t* out);
 /* How upload and download reach the caller's FP64 arrays:
  *   0: through a pinned staging buffer, converted on the host;
- *   1: upload converts the caller's arrays on the device, reading them in place
- *      (the default when the device can access pageable host memory);
- *   2: download writes them from the device as well (fast when their pages are
- *      already resident: writes into untouched pages fault them in one by one).
- * The results are the same. */
+ *   1: upload converts the caller's arrays on the device, reading them in place,
+ *      and download writes them from the device once the host has touched their
+ *      pages (the default when the device can access pageable host memory);
+ *   2: the same without touching the pages (writes into pages the host never
+ *      touched fault them in one by one).
+ * The results are the same.  A download that returns an error leaves the arrays'
+ * contents undefined. */
 sphg_status sphg_set_host_access(sphg_sim* s, int32_t mode);
 
 /* One instance of n particles. */

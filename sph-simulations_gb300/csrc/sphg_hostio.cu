@@ -30,6 +30,12 @@ __device__ __forceinline__ double floor_div(double t, double cs, double inv_cs) 
   return floor(__ddiv_rn(t, cs));
 }
 
+// The error words of the device state into the handle's pinned block (one
+// thread; the host reads them after the synchronisation that ends the call).
+__device__ __forceinline__ void report_errors(const HostErrors& e) {
+  for (int k = 0; k < kErrorWords; ++k) e.out[k] = *e.word[k];
+}
+
 // One particle of the caller's FP64 state into the device representation
 // (false: not finite, nothing written).
 __device__ __forceinline__ bool upload_one(const StepArgs& a, int precision, int64_t i, double xi, double yi,
@@ -58,13 +64,14 @@ __device__ __forceinline__ bool upload_one(const StepArgs& a, int precision, int
 
 __global__ void upload_direct_kernel(StepArgs a, int precision, const double* __restrict__ x,
                                      const double* __restrict__ y, const double* __restrict__ vx,
-                                     const double* __restrict__ vy, uint32_t* first_bad) {
+                                     const double* __restrict__ vy, uint32_t* first_bad, volatile uint32_t* any_bad) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   float2 pos, vel;
   uint32_t key = 0;
   if (!upload_one(a, precision, i, x[i], y[i], vx[i], vy[i], pos, vel, key)) {
     atomicMin(first_bad, (uint32_t)i);
+    *any_bad = 1u;
     return;
   }
   a.velB[i] = vel;
@@ -77,7 +84,7 @@ __global__ void upload_direct_kernel(StepArgs a, int precision, const double* __
 // (all four 16-byte aligned; n odd: the last particle alone).
 __global__ void upload_direct_kernel2(StepArgs a, int precision, const double2* __restrict__ x,
                                       const double2* __restrict__ y, const double2* __restrict__ vx,
-                                      const double2* __restrict__ vy, uint32_t* first_bad) {
+                                      const double2* __restrict__ vy, uint32_t* first_bad, volatile uint32_t* any_bad) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i0 = 2 * t;
   if (i0 >= a.n) return;
@@ -90,6 +97,7 @@ __global__ void upload_direct_kernel2(StepArgs a, int precision, const double2* 
     uint32_t key = 0;
     if (!upload_one(a, precision, i0, xs[i0], ys[i0], vxs[i0], vys[i0], pos, vel, key)) {
       atomicMin(first_bad, (uint32_t)i0);
+      *any_bad = 1u;
       return;
     }
     a.velB[i0] = vel;
@@ -105,6 +113,7 @@ __global__ void upload_direct_kernel2(StepArgs a, int precision, const double2* 
   const bool ok1 = upload_one(a, precision, i0 + 1, xv.y, yv.y, vxv.y, vyv.y, p1, v1, k1);
   if (!ok0 || !ok1) {
     atomicMin(first_bad, (uint32_t)(ok0 ? i0 + 1 : i0));
+    *any_bad = 1u;
     if (!ok0 && !ok1) return;
   }
   if (ok0 && ok1) {
@@ -121,101 +130,48 @@ __global__ void upload_direct_kernel2(StepArgs a, int precision, const double2* 
   if (a.track_ids) a.idsB[i] = (int32_t)i;
 }
 
-// Particle i of the device state in the caller's FP64 representation.
-__device__ __forceinline__ void download_one(const StepArgs& a, int precision, int64_t i, double& px, double& py) {
+// One position coordinate (axis 0 or 1) of slot i in the caller's FP64 representation.
+__device__ __forceinline__ double download_position(const StepArgs& a, int precision, int64_t i, int axis) {
   const float2 p = a.posA[i];
-  px = p.x;
-  py = p.y;
-  if (precision == SPHG_PRECISION_SPLIT) {
-    const InstDesc& d = inst_ref<true>(a, i);
-    int cx, cy;
-    decode_code(d, a.keyA[i] - d.cell_base, cx, cy);
-    px = __dadd_rn(__dadd_rn(d.lo_xd, __dmul_rn((double)cx, d.cs_xd)), px);
-    py = __dadd_rn(__dadd_rn(d.lo_yd, __dmul_rn((double)cy, d.cs_yd)), py);
-  }
+  const double o = axis ? p.y : p.x;
+  if (precision != SPHG_PRECISION_SPLIT) return o;
+  const InstDesc& d = inst_ref<true>(a, i);
+  int cx, cy;
+  decode_code(d, a.keyA[i] - d.cell_base, cx, cy);
+  return axis ? __dadd_rn(__dadd_rn(d.lo_yd, __dmul_rn((double)cy, d.cs_yd)), o)
+              : __dadd_rn(__dadd_rn(d.lo_xd, __dmul_rn((double)cx, d.cs_xd)), o);
 }
+
+// Entry of `out` that thread t writes: t less the entries between the 128-byte
+// line the array starts in and its first one, so that a warp's stores cover
+// whole lines wherever the caller's array lies (malloc's large blocks start 16
+// bytes into a page: 170 GB/s of the host link with lines split between warps,
+// 192 with whole ones -- what the link takes of writes).
+template <class T>
+__device__ __forceinline__ int64_t line_entry(const T* out, int64_t t) {
+  return t - (int64_t)((reinterpret_cast<uintptr_t>(out) & 127u) / sizeof(T));
+}
+constexpr int kLineEntries = 32;  // at most this many threads more than entries
 
 __global__ void download_direct_kernel(StepArgs a, int precision, double* __restrict__ x, double* __restrict__ y,
                                        double* __restrict__ vx, double* __restrict__ vy,
                                        double* __restrict__ rho, double* __restrict__ fx,
-                                       double* __restrict__ fy, int32_t* __restrict__ ids) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  if (x || y) {
-    double px, py;
-    download_one(a, precision, i, px, py);
-    if (x) x[i] = px;
-    if (y) y[i] = py;
-  }
-  if (vx || vy) {
-    const float4 v = a.velpA[i];
-    if (vx) vx[i] = v.x;
-    if (vy) vy[i] = v.y;
-  }
-  if (rho) rho[i] = a.rho[i];
-  if (fx || fy) {
-    const float2 f = a.acc[i];
-    if (fx) fx[i] = f.x;
-    if (fy) fy[i] = f.y;
-  }
-  if (ids) ids[i] = a.track_ids ? a.idsA[i] : -1;
-}
-
-// Two consecutive particles a thread, 16-byte writes of the caller's arrays
-// (every given array 16-byte aligned, the ids 8-byte; n odd: the last one alone).
-__global__ void download_direct_kernel2(StepArgs a, int precision, double* __restrict__ x, double* __restrict__ y,
-                                        double* __restrict__ vx, double* __restrict__ vy,
-                                        double* __restrict__ rho, double* __restrict__ fx,
-                                        double* __restrict__ fy, int32_t* __restrict__ ids) {
+                                       double* __restrict__ fy, int32_t* __restrict__ ids, HostErrors errors) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t i0 = 2 * t;
-  if (i0 >= a.n) return;
-  if (i0 + 1 == a.n) {  // the odd last particle
-    if (x || y) {
-      double px, py;
-      download_one(a, precision, i0, px, py);
-      if (x) x[i0] = px;
-      if (y) y[i0] = py;
-    }
-    if (vx || vy) {
-      const float4 v = a.velpA[i0];
-      if (vx) vx[i0] = v.x;
-      if (vy) vy[i0] = v.y;
-    }
-    if (rho) rho[i0] = a.rho[i0];
-    if (fx || fy) {
-      const float2 f = a.acc[i0];
-      if (fx) fx[i0] = f.x;
-      if (fy) fy[i0] = f.y;
-    }
-    if (ids) ids[i0] = a.track_ids ? a.idsA[i0] : -1;
-    return;
-  }
-  if (x || y) {
-    double px0, py0, px1, py1;
-    download_one(a, precision, i0, px0, py0);
-    download_one(a, precision, i0 + 1, px1, py1);
-    if (x) reinterpret_cast<double2*>(x)[t] = make_double2(px0, px1);
-    if (y) reinterpret_cast<double2*>(y)[t] = make_double2(py0, py1);
-  }
-  if (vx || vy) {
-    const float4 v0 = a.velpA[i0], v1 = a.velpA[i0 + 1];
-    if (vx) reinterpret_cast<double2*>(vx)[t] = make_double2(v0.x, v1.x);
-    if (vy) reinterpret_cast<double2*>(vy)[t] = make_double2(v0.y, v1.y);
-  }
-  if (rho) {
-    const float2 r = reinterpret_cast<const float2*>(a.rho)[t];
-    reinterpret_cast<double2*>(rho)[t] = make_double2(r.x, r.y);
-  }
-  if (fx || fy) {
-    const float4 f = reinterpret_cast<const float4*>(a.acc)[t];
-    if (fx) reinterpret_cast<double2*>(fx)[t] = make_double2(f.x, f.z);
-    if (fy) reinterpret_cast<double2*>(fy)[t] = make_double2(f.y, f.w);
-  }
-  if (ids) {
-    const int2 d = a.track_ids ? reinterpret_cast<const int2*>(a.idsA)[t] : make_int2(-1, -1);
-    reinterpret_cast<int2*>(ids)[t] = d;
-  }
+  if (t == 0) report_errors(errors);
+  auto write = [&](auto* out, auto&& value) {
+    if (!out) return;
+    const int64_t i = line_entry(out, t);
+    if (i >= 0 && i < a.n) out[i] = value(i);
+  };
+  write(x, [&](int64_t i) { return download_position(a, precision, i, 0); });
+  write(y, [&](int64_t i) { return download_position(a, precision, i, 1); });
+  write(vx, [&](int64_t i) { return (double)a.velpA[i].x; });
+  write(vy, [&](int64_t i) { return (double)a.velpA[i].y; });
+  write(rho, [&](int64_t i) { return (double)a.rho[i]; });
+  write(fx, [&](int64_t i) { return (double)a.acc[i].x; });
+  write(fy, [&](int64_t i) { return (double)a.acc[i].y; });
+  write(ids, [&](int64_t i) { return a.track_ids ? a.idsA[i] : -1; });
 }
 
 bool aligned(const void* p, uintptr_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; }
@@ -223,31 +179,27 @@ bool aligned(const void* p, uintptr_t to) { return (reinterpret_cast<uintptr_t>(
 }  // namespace
 
 cudaError_t launch_upload_direct(const StepArgs& a, int precision, const double* x, const double* y,
-                                 const double* vx, const double* vy, uint32_t* first_bad, cudaStream_t st) {
+                                 const double* vx, const double* vy, uint32_t* first_bad, uint32_t* any_bad,
+                                 cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
   if (aligned(x, 16) && aligned(y, 16) && aligned(vx, 16) && aligned(vy, 16)) {
     const int64_t pairs = (a.n + 1) / 2;
     upload_direct_kernel2<<<(unsigned)((pairs + 255) / 256), 256, 0, st>>>(
         a, precision, reinterpret_cast<const double2*>(x), reinterpret_cast<const double2*>(y),
-        reinterpret_cast<const double2*>(vx), reinterpret_cast<const double2*>(vy), first_bad);
+        reinterpret_cast<const double2*>(vx), reinterpret_cast<const double2*>(vy), first_bad, any_bad);
   } else {
-    upload_direct_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a, precision, x, y, vx, vy, first_bad);
+    upload_direct_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a, precision, x, y, vx, vy, first_bad,
+                                                                          any_bad);
   }
   return cudaGetLastError();
 }
 
 cudaError_t launch_download_direct(const StepArgs& a, int precision, double* x, double* y, double* vx, double* vy,
-                                   double* rho, double* fx, double* fy, int32_t* ids, cudaStream_t st) {
+                                   double* rho, double* fx, double* fy, int32_t* ids, const HostErrors& errors,
+                                   cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
-  if (aligned(x, 16) && aligned(y, 16) && aligned(vx, 16) && aligned(vy, 16) && aligned(rho, 16) &&
-      aligned(fx, 16) && aligned(fy, 16) && aligned(ids, 8)) {
-    const int64_t pairs = (a.n + 1) / 2;
-    download_direct_kernel2<<<(unsigned)((pairs + 255) / 256), 256, 0, st>>>(a, precision, x, y, vx, vy, rho, fx,
-                                                                               fy, ids);
-  } else {
-    download_direct_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a, precision, x, y, vx, vy, rho, fx, fy,
-                                                                           ids);
-  }
+  const unsigned g = (unsigned)((a.n + kLineEntries + 255) / 256);
+  download_direct_kernel<<<g, 256, 0, st>>>(a, precision, x, y, vx, vy, rho, fx, fy, ids, errors);
   return cudaGetLastError();
 }
 

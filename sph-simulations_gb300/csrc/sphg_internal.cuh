@@ -81,10 +81,13 @@ struct sphg_sim {
   int force_batched = 0;        // always use the per-instance-descriptor kernels
   int tile_bits = 0, tile_cap = 0, tile_grid = 0;
   bool uploaded = false, preloop_done = false;
-  // 1: upload reads the caller's arrays from the device (pageable host memory
-  // access); 2: download writes them from the device too; 0: both through the
-  // pinned staging below
+  // 1, 2: upload reads and download writes the caller's arrays from the device
+  // (pageable host memory access; 1: their pages are touched first); 0: both
+  // through the pinned staging below
   int host_direct = 0;
+  // pinned words the device reports in: [0, kErrorWords) error words, then the
+  // upload's "a value is not finite"
+  uint32_t* hwords = nullptr;
   // pinned host staging of upload/download (grows on demand)
   char* hstage = nullptr;
   size_t hstage_bytes = 0;
@@ -170,8 +173,9 @@ sphg_status fail(sphg_status st, const std::string& msg);
 sphg_status make_desc(const sphg_params& p, int64_t begin, int64_t count, uint64_t cell_base,
                       InstDesc& d, uint64_t& span);
 int host_cell(double x, double lo, double cs, int cmax);
-// f(begin, end) over [0, n) split across host threads (one thread for small n).
-void parallel_for(int64_t n, const std::function<void(int64_t, int64_t)>& f);
+// f(begin, end) over [0, n) split across host threads, at least `grain` each
+// (one thread for small n).
+void parallel_for(int64_t n, const std::function<void(int64_t, int64_t)>& f, int64_t grain = 1 << 16);
 // Pinned host staging of at least `bytes` owned by the handle (nullptr: out of memory).
 char* host_stage(sphg_sim* s, size_t bytes);
 // In-cell offset o (FP64, in [0, cs)) as FP32, kept below cs after rounding.
