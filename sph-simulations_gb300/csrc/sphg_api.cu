@@ -288,7 +288,7 @@ sphg_status enqueue_full_sort(sphg_sim* s, cudaStream_t st, const uint32_t* skip
 // reorder: the gather after a full sort is launched here (else the caller has
 // placed it with the sort).
 sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bool size_lists = false,
-                               bool reorder = true) {
+                               bool reorder = true, bool header = false) {
   const StepArgs a = s->args();
   const int prec = s->opt.precision;
   if (s->tile_bits) SPHG_CUDA(cudaMemsetAsync(s->flags + 1, 0, sizeof(uint32_t), st));
@@ -332,7 +332,9 @@ sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bo
   } else {
     SPHG_CUDA(sphg::launch_density(a, prec, st));
     if (ev) SPHG_CUDA(cudaEventRecord(ev[4], st));
-    SPHG_CUDA(sphg::launch_force(a, prec, sphg::kForceIntegrate, st));
+    StepArgs f = a;
+    if (header) f.early_next = 1;  // the step header needs nothing of the force pass
+    SPHG_CUDA(sphg::launch_force(f, prec, sphg::kForceIntegrate, st));
   }
   if (ev) SPHG_CUDA(cudaEventRecord(ev[5], st));
   return SPHG_OK;
@@ -438,7 +440,7 @@ sphg_status build_graph_conditional(sphg_sim* s, cudaGraphExec_t* exec, bool hea
   if (eb != cudaSuccess) return done(fail(SPHG_CUDA_ERROR, "end of the conditional body capture"));
   if (cudaStreamUpdateCaptureDependencies(s->cap_stream, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies) != cudaSuccess)
     return done(fail(SPHG_CUDA_ERROR, "capture dependencies"));
-  if (!fused) st = enqueue_after_sort(s, s->cap_stream, nullptr, false, false);
+  if (!fused) st = enqueue_after_sort(s, s->cap_stream, nullptr, false, false, header);
   if (st == SPHG_OK && header) st = enqueue_header(s, s->cap_stream);
   if (st != SPHG_OK) return done(st);
   cudaGraph_t out = nullptr;

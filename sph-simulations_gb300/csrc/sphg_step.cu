@@ -920,6 +920,10 @@ __global__ void __launch_bounds__(kThreads, BATCHED ? 6 : 8) step_fused(StepArgs
 // ---------------------------------------------------------------- diagnostics
 constexpr int kDiagThreads = 256;
 constexpr int kDiagBatch = 4;
+// Blocks per SM (80 registers): two left the loads of the next particles waiting
+// for the sums of the last (batch of 256: header 53 us with two, 44 with three,
+// 48 with four and two particles' loads in flight a thread).
+constexpr int kDiagBlocks = 3;
 
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
@@ -938,16 +942,27 @@ __device__ __forceinline__ void fast_two_sum(float a, float b, float& s, float& 
   s = __fadd_rn(a, b);
   e = __fsub_rn(b, __fsub_rn(s, a));
 }
-struct FFSum {
-  float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add(float v, float err) {
-    float t, e;
-    two_sum(s, v, t, e);
+// Two sums at once (paired instructions, the components independent).
+struct FFSum2 {
+  float2 s = {0.f, 0.f}, c = {0.f, 0.f};
+  __device__ __forceinline__ void two_sum(float2 v, float2& e) {
+    const float2 t = add2(s, v);
+    const float2 bp = sub2(t, s);
+    e = add2(sub2(s, sub2(t, bp)), sub2(v, bp));
     s = t;
-    c = __fadd_rn(c, __fadd_rn(e, err));
   }
-  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+  __device__ __forceinline__ void add(float2 v) {
+    float2 e;
+    two_sum(v, e);
+    c = add2(c, e);
+  }
+  __device__ __forceinline__ void add(float2 v, float2 err) {
+    float2 e;
+    two_sum(v, e);
+    c = add2(c, add2(e, err));
+  }
 };
+__device__ __forceinline__ double ff_value(float s, float c) { return (double)s + (double)c; }
 
 // Per (chunk, instance) block.  The conservation sums (kinetic energy,
 // momentum) and max |v|^2 carry the FP32 velocities' exact squares in
@@ -964,22 +979,16 @@ static __device__ __noinline__ bool inside_d(double x, double y, double lox, dou
 // |v|^2 as a normalised float-float pair, two counts.  48 bytes, the size of
 // six doubles per chunk of the partials buffer.
 struct DiagPart {
-  FFSum e2, mx, my;
+  FFSum2 e2;  // vx^2, vy^2
+  FFSum2 m;   // vx, vy
   float mh, ml;
-  uint32_t inside, bad, pad0, pad1;
+  uint32_t inside, bad;
 };
 static_assert(sizeof(DiagPart) == 6 * sizeof(double), "a chunk's slot of the partials buffer");
 
-__device__ __forceinline__ void ff_add(FFSum& a, const FFSum& b) {  // a += b
-  float t, e;
-  two_sum(a.s, b.s, t, e);
-  a.s = t;
-  a.c = __fadd_rn(a.c, __fadd_rn(b.c, e));
-}
 __device__ __forceinline__ void part_add(DiagPart& a, const DiagPart& b) {
-  ff_add(a.e2, b.e2);
-  ff_add(a.mx, b.mx);
-  ff_add(a.my, b.my);
+  a.e2.add(b.e2.s, b.e2.c);
+  a.m.add(b.m.s, b.m.c);
   if (b.mh > a.mh || (b.mh == a.mh && b.ml > a.ml)) {
     a.mh = b.mh;
     a.ml = b.ml;
@@ -989,16 +998,10 @@ __device__ __forceinline__ void part_add(DiagPart& a, const DiagPart& b) {
 }
 __device__ __forceinline__ DiagPart part_shfl_down(const DiagPart& a, int o) {
   DiagPart b;
-  b.e2.s = __shfl_down_sync(0xffffffffu, a.e2.s, o);
-  b.e2.c = __shfl_down_sync(0xffffffffu, a.e2.c, o);
-  b.mx.s = __shfl_down_sync(0xffffffffu, a.mx.s, o);
-  b.mx.c = __shfl_down_sync(0xffffffffu, a.mx.c, o);
-  b.my.s = __shfl_down_sync(0xffffffffu, a.my.s, o);
-  b.my.c = __shfl_down_sync(0xffffffffu, a.my.c, o);
-  b.mh = __shfl_down_sync(0xffffffffu, a.mh, o);
-  b.ml = __shfl_down_sync(0xffffffffu, a.ml, o);
-  b.inside = __shfl_down_sync(0xffffffffu, a.inside, o);
-  b.bad = __shfl_down_sync(0xffffffffu, a.bad, o);
+  const float* u = reinterpret_cast<const float*>(&a);
+  float* v = reinterpret_cast<float*>(&b);
+#pragma unroll
+  for (int k = 0; k < 12; ++k) v[k] = __shfl_down_sync(0xffffffffu, u[k], o);
   return b;
 }
 // The block's sum in thread 0 (fixed shape: lanes by halving, then the warps in order).
@@ -1024,41 +1027,28 @@ __device__ __forceinline__ DiagPart load_part(const DiagPart* p) {
 
 // The constants of an instance that the diagnostics use per particle.
 struct DiagConst {
-  float lo_x, hi_x, lo_y, hi_y, cs_x, cs_y, Lx, Ly, band;
-  uint32_t cell_base;
+  float cs_x, cs_y, band;
+  uint32_t cell_base, inner_x, inner_y;  // inner: cells between the outermost two of an axis
   int order, nx;
 };
 __device__ __forceinline__ DiagConst diag_const(const InstDesc& d) {
   DiagConst c;
-  c.lo_x = d.lo_x, c.hi_x = d.hi_x, c.lo_y = d.lo_y, c.hi_y = d.hi_y;
-  c.cs_x = d.cs_x, c.cs_y = d.cs_y, c.Lx = d.Lx, c.Ly = d.Ly;
+  c.cs_x = d.cs_x, c.cs_y = d.cs_y;
   c.band = 1.0e-6f * fmaxf(fabsf(d.hi_x - d.lo_x), fabsf(d.hi_y - d.lo_y));
   c.cell_base = d.cell_base;
+  c.inner_x = d.nxr > 2 ? (uint32_t)d.nxr - 2u : 0u;
+  c.inner_y = d.nyr > 2 ? (uint32_t)d.nyr - 2u : 0u;
   c.order = d.order, c.nx = d.nx;
   return c;
 }
 
-// One particle into the partial v.
+// Whether a finite particle lies in the domain: FP32 decides, FP64 within a
+// thin band of a wall.  A split position in a cell away from the outermost ones
+// is inside by its cell alone.
 template <int PREC>
-__device__ __forceinline__ void diag_particle(DiagPart& v, const InstDesc& d, const DiagConst& q, float2 vel, float2 p,
-                                              float rho, uint32_t key) {
-  const float p1 = vel.x * vel.x, e1 = fmaf(vel.x, vel.x, -p1);
-  const float p2 = vel.y * vel.y, e2 = fmaf(vel.y, vel.y, -p2);
-  v.e2.add(p1, e1);
-  v.e2.add(p2, e2);
-  v.mx.add(vel.x, 0.f);
-  v.my.add(vel.y, 0.f);
-  float h, l;
-  two_sum(p1, p2, h, l);
-  l += e1 + e2;
-  fast_two_sum(h, l, h, l);
-  if (h > v.mh || (h == v.mh && l > v.ml)) {
-    v.mh = h;
-    v.ml = l;
-  }
+__device__ __forceinline__ bool diag_inside(const InstDesc& d, const DiagConst& q, float2 p, uint32_t key) {
   int cx = 0, cy = 0;
-  const float x = p.x, y = p.y;  // position, or offset in cell (cx, cy)
-  float lox = q.lo_x, hix = q.hi_x, loy = q.lo_y, hiy = q.hi_y;
+  float lox = d.lo_x, hix = d.hi_x, loy = d.lo_y, hiy = d.hi_y;
   if (PREC == 1) {
     const uint32_t code = key - q.cell_base;
     if (q.order == 0) {
@@ -1068,31 +1058,55 @@ __device__ __forceinline__ void diag_particle(DiagPart& v, const InstDesc& d, co
       cx = (int)(code % (uint32_t)q.nx);
       cy = (int)(code / (uint32_t)q.nx);
     }
+    if ((uint32_t)cx - 1u < q.inner_x && (uint32_t)cy - 1u < q.inner_y && p.x >= 0.f && p.x <= q.cs_x && p.y >= 0.f &&
+        p.y <= q.cs_y)
+      return true;
     lox = -(float)cx * q.cs_x;  // the walls in the cell's frame
-    hix = q.Lx - (float)cx * q.cs_x;
+    hix = d.Lx - (float)cx * q.cs_x;
     loy = -(float)cy * q.cs_y;
-    hiy = q.Ly - (float)cy * q.cs_y;
+    hiy = d.Ly - (float)cy * q.cs_y;
   }
-  const bool fin = isfinite(x) && isfinite(y) && isfinite(vel.x) && isfinite(vel.y) && isfinite(rho);
-  bool in = fin && x >= lox && x <= hix && y >= loy && y <= hiy;
-  const bool near = fin && (fabsf(x - lox) <= q.band || fabsf(x - hix) <= q.band || fabsf(y - loy) <= q.band ||
-                            fabsf(y - hiy) <= q.band);
-  if (near) {
-    const double xd = PREC == 1 ? d.lo_xd + cx * d.cs_xd + (double)x : (double)x;
-    const double yd = PREC == 1 ? d.lo_yd + cy * d.cs_yd + (double)y : (double)y;
-    in = inside_d(xd, yd, d.lo_xd, d.hi_xd, d.lo_yd, d.hi_yd);
+  // in, clear of every wall / out, clear of it
+  if (p.x - lox > q.band && hix - p.x > q.band && p.y - loy > q.band && hiy - p.y > q.band) return true;
+  const bool near = fabsf(p.x - lox) <= q.band || fabsf(p.x - hix) <= q.band || fabsf(p.y - loy) <= q.band ||
+                    fabsf(p.y - hiy) <= q.band;
+  if (!near) return false;
+  const double xd = PREC == 1 ? d.lo_xd + cx * d.cs_xd + (double)p.x : (double)p.x;
+  const double yd = PREC == 1 ? d.lo_yd + cy * d.cs_yd + (double)p.y : (double)p.y;
+  return inside_d(xd, yd, d.lo_xd, d.hi_xd, d.lo_yd, d.hi_yd);
+}
+
+// One particle into the partial v.
+template <int PREC>
+__device__ __forceinline__ void diag_particle(DiagPart& v, const InstDesc& d, const DiagConst& q, float2 vel, float2 p,
+                                              float rho, uint32_t key) {
+  const float2 sq = mul2(vel, vel);
+  const float2 er = fma2(vel, vel, make_float2(-sq.x, -sq.y));
+  v.e2.add(sq, er);
+  v.m.add(vel);
+  // the exact pair only for a particle that may pass the maximum
+  if ((sq.x + sq.y) * (1.0f + 1.0e-6f) > v.mh) {
+    float h, l;
+    two_sum(sq.x, sq.y, h, l);
+    l += er.x + er.y;
+    fast_two_sum(h, l, h, l);
+    if (h > v.mh || (h == v.mh && l > v.ml)) {
+      v.mh = h;
+      v.ml = l;
+    }
   }
-  v.inside += in ? 1u : 0u;
+  const bool fin = isfinite(p.x) && isfinite(p.y) && isfinite(vel.x) && isfinite(vel.y) && isfinite(rho);
+  v.inside += fin && diag_inside<PREC>(d, q, p, key) ? 1u : 0u;
   v.bad += fin ? 0u : 1u;
 }
 
 // The six values of an instance's summed partials.
 __device__ __forceinline__ void diag_values(const DiagPart& f, double m, double* out) {
-  out[0] = 0.5 * m * f.e2.value();
+  out[0] = 0.5 * m * (ff_value(f.e2.s.x, f.e2.c.x) + ff_value(f.e2.s.y, f.e2.c.y));
   out[1] = (double)f.mh + (double)f.ml;
   out[2] = (double)f.inside;
-  out[3] = m * f.mx.value();
-  out[4] = m * f.my.value();
+  out[3] = m * ff_value(f.m.s.x, f.m.c.x);
+  out[4] = m * ff_value(f.m.s.y, f.m.c.y);
   out[5] = (double)f.bad;
 }
 
@@ -1103,7 +1117,7 @@ __device__ __forceinline__ void diag_values(const DiagPart& f, double m, double*
 // count}, written to out[inst * 6 ..] or, with a header slot, to the slot's
 // array at step k -- whose index the last instance to finish then advances.
 template <int PREC, bool SLOT>
-__global__ void __launch_bounds__(kDiagThreads) step_diag(StepArgs a, int chunks, double* partials,
+__global__ void __launch_bounds__(kDiagThreads, kDiagBlocks) step_diag(StepArgs a, int chunks, double* partials,
                                                           uint32_t* tickets, double* out, HeaderSlot* slot) {
   // block -> (instance, chunk): one instance: the grid's x; several: the
   // layout's table (about 4,096 particles a block for every instance, so a
@@ -1136,7 +1150,7 @@ __global__ void __launch_bounds__(kDiagThreads) step_diag(StepArgs a, int chunks
       const int64_t i = i0 + (int64_t)u * blockDim.x;
       const bool ok = i < e;
       vb[u] = ok ? reinterpret_cast<const float2*>(a.velpA)[2 * i] : make_float2(0.f, 0.f);
-      pb[u] = ok ? a.posA[i] : make_float2(0.5f * (dc.lo_x + dc.hi_x), 0.5f * (dc.lo_y + dc.hi_y));
+      pb[u] = ok ? a.posA[i] : make_float2(0.f, 0.f);
       rb[u] = ok ? a.rho[i] : 1.f;
       kb[u] = (PREC == 1 && ok) ? a.keyA[i] : dc.cell_base;
     }
@@ -1156,6 +1170,9 @@ __global__ void __launch_bounds__(kDiagThreads) step_diag(StepArgs a, int chunks
     last = atomicAdd(tickets + inst, 1u) == (uint32_t)ck - 1u;
   }
   __syncthreads();
+  // a step header is launched while the force pass finishes (it reads what the
+  // passes before that wrote): the iteration ends when both have
+  if (SLOT) cudaGridDependencySynchronize();
   if (!last) return;
   __threadfence();
   DiagPart f = {};
@@ -1168,13 +1185,12 @@ __global__ void __launch_bounds__(kDiagThreads) step_diag(StepArgs a, int chunks
     return;
   }
   const size_t k = *(volatile uint32_t*)&slot->k;
-  diag_values(f, d.mass_d, slot->out + (k * a.ninst + inst) * 6);
-  __threadfence();
+  __threadfence();  // k is read before it may advance (and before the values leave for the host)
   if (atomicAdd(&slot->done, 1u) == (uint32_t)a.ninst - 1u) {
     slot->done = 0;
-    slot->k += 1;
-    __threadfence();
+    slot->k = (uint32_t)k + 1u;
   }
+  diag_values(f, d.mass_d, slot->out + (k * a.ninst + inst) * 6);
 }
 
 // ---------------------------------------------------------------- many iterations in one cluster
@@ -1551,9 +1567,10 @@ cudaError_t launch_diagnostics(const StepArgs& a, int precision, double* partial
 cudaError_t launch_diagnostics_slot(const StepArgs& a, int precision, double* partials, uint32_t* tickets,
                                     int chunks, HeaderSlot* slot, cudaStream_t s) {
   const dim3 g = a.diag_tab ? dim3(a.diag_blocks) : dim3(chunks, a.ninst);
-  if (precision) step_diag<1, true><<<g, kDiagThreads, 0, s>>>(a, chunks, partials, tickets, nullptr, slot);
-  else step_diag<0, true><<<g, kDiagThreads, 0, s>>>(a, chunks, partials, tickets, nullptr, slot);
-  return cudaGetLastError();
+  cudaError_t e;
+  if (precision) e = launch_pdl(step_diag<1, true>, g, dim3(kDiagThreads), 0, s, a, chunks, partials, tickets, (double*)nullptr, slot);
+  else e = launch_pdl(step_diag<0, true>, g, dim3(kDiagThreads), 0, s, a, chunks, partials, tickets, (double*)nullptr, slot);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_cfl(const StepArgs& a, double* partials, int chunks, double* out, cudaStream_t s) {
