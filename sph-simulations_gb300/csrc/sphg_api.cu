@@ -277,7 +277,7 @@ sphg_status enqueue_fused(sphg_sim* s, cudaStream_t st, bool post, unsigned long
 // its kernels return at once, or null).
 sphg_status enqueue_full_sort(sphg_sim* s, cudaStream_t st, const uint32_t* skip) {
   SPHG_CUDA(sphg::radix_sort_pairs(s->keyB, nullptr, s->keyTmp, s->perm, s->keyA, s->valTmp,
-                                   s->scratch, s->n, s->key_bits, st, s->flags + 2, nullptr, skip));
+                                   s->scratch, s->n, s->key_bits, st, s->flags + 2, skip));
   return SPHG_OK;
 }
 
@@ -1362,7 +1362,6 @@ sphg_status sphg_restore(sphg_sim* s, const void* buf, uint64_t bytes, void* str
     SPHG_CUDA(cudaMemcpyAsync(s->velB, vel, n * sizeof(float2), cudaMemcpyHostToDevice, st));
     SPHG_CUDA(cudaMemcpyAsync(s->keyA, key, n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     if (s->opt.track_ids) SPHG_CUDA(cudaMemcpyAsync(s->idsB, ids, n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    SPHG_CUDA(cudaMemsetAsync(s->scratch, 0, sizeof(uint32_t) * 4 * 256, st));
     SPHG_CUDA(cudaStreamSynchronize(st));
   }
   s->uploaded = true;
@@ -1413,7 +1412,7 @@ sphg_status sphg_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, ui
   uint32_t* vtmp = ktmp + n;
   cudaError_t e = sphg::radix_sort_pairs(keys_in, vals_in, keys_out, vals_out,
                                          bits > 8 ? ktmp : nullptr, bits > 8 ? vtmp : nullptr,
-                                         scratch, n, bits, st, nullptr, nullptr, nullptr, true);
+                                         scratch, n, bits, st, nullptr, nullptr, true);
   cudaError_t e2 = cudaFreeAsync(scratch, st);
   SPHG_CUDA(e);
   SPHG_CUDA(e2);

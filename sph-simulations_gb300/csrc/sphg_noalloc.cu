@@ -34,7 +34,7 @@ constexpr size_t kHistWords = sphg::sort_scratch_words_c(kNoAllocMaxPairs);
 constexpr size_t kScratchWords = kHistWords + 2 * (size_t)kNoAllocMaxPairs;
 static_assert(kScratchWords * 4 == SPHG_SORT_NOALLOC_SCRATCH_BYTES, "documented scratch size");
 
-// [histograms, tile counters, error word, look-back words | ping-pong keys | ping-pong values]
+// [error word, histograms, tile counters, look-back words | ping-pong keys | ping-pong values]
 static __device__ __align__(256) uint32_t g_noalloc_sort_scratch[kScratchWords];
 
 constexpr int kMaxDevices = 64;
@@ -126,8 +126,7 @@ sphg_status sphg_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* val
   uint32_t* keys_tmp = scratch + kHistWords;
   uint32_t* vals_tmp = keys_tmp + kNoAllocMaxPairs;
   cudaError_t e = sphg::radix_sort_pairs(keys_in, vals_in, keys_out, vals_out, keys_tmp, vals_tmp,
-                                         scratch, n, bits, (cudaStream_t)stream, nullptr, nullptr, nullptr,
-                                         true);
+                                         scratch, n, bits, (cudaStream_t)stream, nullptr, nullptr, true);
   if (e != cudaSuccess) return noalloc_fail(SPHG_CUDA_ERROR, std::string("radix sort launch: ") + cudaGetErrorString(e));
   return SPHG_OK;
 }

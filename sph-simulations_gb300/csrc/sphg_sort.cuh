@@ -19,9 +19,7 @@ uint32_t* sort_error_word(uint32_t* scratch);
 // means the identity 0..n-1.  keys_tmp/vals_tmp are ping-pong buffers of n
 // entries (unused for bits <= 8).  The result lands in keys_out/vals_out.
 // No buffer may alias another.  When epoch is not null the first pass
-// increments *epoch once (the step epoch of the cell-range table).  hist, when
-// not null, holds the digit histograms of all passes already ([4][256], digit
-// d of pass p at p*256 + d, summed over all keys); otherwise they are computed.
+// increments *epoch once (the step epoch of the cell-range table).
 // When *skip (device word, read by the kernels) is non-zero the kernels return
 // at once: the step's incremental re-sort produced the result instead.
 // clear_err: zero the error word first (stand-alone sorts, whose callers have
@@ -30,8 +28,7 @@ cudaError_t radix_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in,
                              uint32_t* keys_out, uint32_t* vals_out, uint32_t* keys_tmp,
                              uint32_t* vals_tmp, uint32_t* scratch, int64_t n, int bits,
                              cudaStream_t stream, uint32_t* epoch = nullptr,
-                             const uint32_t* hist = nullptr, const uint32_t* skip = nullptr,
-                             bool clear_err = false);
+                             const uint32_t* skip = nullptr, bool clear_err = false);
 // Largest n the sort accepts: a look-back word keeps a running count in 30 bits
 // under its two flag bits.
 constexpr int64_t kSortMaxKeys = ((int64_t)1 << 30) - 1;
