@@ -576,8 +576,14 @@ sphg_status alloc_arena(sphg_sim* s, size_t N, uint64_t keys, int ninst, int dia
   s->cap_inst = ninst;
   s->diag_chunks = diag_chunks;
   // per-particle neighbour slots filled by the density pass and read by the
-  // force pass (indices are packed as j << 5, so only below 2^27 particles)
-  s->nbr_slots = (N < ((size_t)1 << 27) && s->opt.compute == SPHG_COMPUTE_SORTED) ? 12 : 0;
+  // force pass (indices are packed as j << 5, so only below 2^27 particles).  A
+  // particle with more neighbours walks the stencil again in the force pass, with
+  // its warp.  32 slots up to 2^18 particles (slots not needed are never touched:
+  // the 6,084-particle example, whose particles gather 15 to 30 neighbours, 41.8 ->
+  // 29.5 us an iteration, others the same); 12 beyond, where 32 measured 0.6 %
+  // slower on the 1M dam break, and in a server's arena, sized for 12.
+  s->nbr_slots = (N < ((size_t)1 << 27) && s->opt.compute == SPHG_COMPUTE_SORTED)
+                     ? (N <= ((size_t)1 << 18) && !s->force_batched ? 32 : 12) : 0;
   auto layout = [&](Arena& A) {
     s->ddesc = A.take<InstDesc>(ninst);
     s->dbegins = A.take<int32_t>(ninst);
