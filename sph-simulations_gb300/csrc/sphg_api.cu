@@ -381,6 +381,17 @@ sphg_status enqueue_header(sphg_sim* s, cudaStream_t st) {
   return SPHG_OK;
 }
 
+// The node that what is captured next depends on: the kernel captured last (null
+// where the force pass is another kernel than step_force).
+static sphg_status last_node(cudaStream_t st, cudaGraphNode_t* node) {
+  cudaStreamCaptureStatus cst;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t ndeps = 0;
+  SPHG_CUDA(cudaStreamGetCaptureInfo(st, &cst, nullptr, nullptr, &deps, nullptr, &ndeps));
+  *node = ndeps == 1 ? deps[0] : nullptr;
+  return SPHG_OK;
+}
+
 // Graph of one iteration with the full sort under a conditional node: the
 // incremental re-sort's decision kernel switches it off, so iterations that
 // merge launch none of the full sort's kernels.
@@ -441,17 +452,18 @@ sphg_status build_graph_conditional(sphg_sim* s, cudaGraphExec_t* exec, bool hea
   if (cudaStreamUpdateCaptureDependencies(s->cap_stream, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies) != cudaSuccess)
     return done(fail(SPHG_CUDA_ERROR, "capture dependencies"));
   if (!fused) st = enqueue_after_sort(s, s->cap_stream, nullptr, false, false, header);
+  cudaGraphNode_t force = nullptr;
+  if (st == SPHG_OK && !fused) st = last_node(s->cap_stream, &force);
   if (st == SPHG_OK && header) st = enqueue_header(s, s->cap_stream);
   if (st != SPHG_OK) return done(st);
   cudaGraph_t out = nullptr;
   if (cudaStreamEndCapture(s->cap_stream, &out) != cudaSuccess) return done(fail(SPHG_CUDA_ERROR, "end capture"));
   const cudaError_t e = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  g = nullptr;
   if (e != cudaSuccess) {
     *exec = nullptr;
-    return fail(SPHG_CUDA_ERROR, std::string("instantiate: ") + cudaGetErrorString(e));
+    return done(fail(SPHG_CUDA_ERROR, std::string("instantiate: ") + cudaGetErrorString(e)));
   }
+  s->keep_graph(header, g, force);
   return SPHG_OK;
 }
 
@@ -469,6 +481,8 @@ sphg_status build_graph(sphg_sim* s, bool header) {
   cudaGraph_t g = nullptr;
   SPHG_CUDA(cudaStreamBeginCapture(s->cap_stream, cudaStreamCaptureModeThreadLocal));
   sphg_status st = enqueue_step(s, s->cap_stream);
+  cudaGraphNode_t force = nullptr;
+  if (st == SPHG_OK && !fused_on(s)) st = last_node(s->cap_stream, &force);
   if (st == SPHG_OK && header) st = enqueue_header(s, s->cap_stream);
   cudaError_t e = cudaStreamEndCapture(s->cap_stream, &g);
   if (st != SPHG_OK) {
@@ -477,8 +491,27 @@ sphg_status build_graph(sphg_sim* s, bool header) {
   }
   SPHG_CUDA(e);
   e = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
+  if (e != cudaSuccess) cudaGraphDestroy(g);
   SPHG_CUDA(e);
+  s->keep_graph(header, g, force);
+  return SPHG_OK;
+}
+
+// The instantiated graph, its force pass's argument brought up to date after a
+// change of the time step.
+static sphg_status current_graph(sphg_sim* s, bool header, cudaGraphExec_t* out) {
+  SPHG_TRY(build_graph(s, header));
+  *out = header ? s->gexec_hdr : s->gexec;
+  if (!s->dt_stale[header]) return SPHG_OK;
+  cudaKernelNodeParams p = {};
+  SPHG_CUDA(cudaGraphKernelNodeGetParams(s->force_node[header], &p));
+  StepArgs a = *static_cast<const StepArgs*>(p.kernelParams[0]);  // as it was captured
+  a.d0 = s->hdesc[0];
+  void* args[1] = {&a};
+  p.kernelParams = args;
+  p.extra = nullptr;
+  SPHG_CUDA(cudaGraphExecKernelNodeSetParams(*out, s->force_node[header], &p));
+  s->dt_stale[header] = false;
   return SPHG_OK;
 }
 
@@ -506,8 +539,9 @@ sphg_status run_steps(sphg_sim* s, int64_t k, cudaStream_t st, bool first = fals
   }
   if (resident_on(s)) return run_resident(s, k, nullptr, st);
   if (s->opt.use_graph) {
-    SPHG_TRY(build_graph(s));
-    for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(s->gexec, st));
+    cudaGraphExec_t g = nullptr;
+    SPHG_TRY(current_graph(s, false, &g));
+    for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(g, st));
   } else {
     for (int64_t i = 0; i < k; ++i) SPHG_TRY(enqueue_step(s, st));
   }
@@ -720,6 +754,7 @@ sphg_status destroy_impl(sphg_sim* s) {
   if (s->csr_idx) cudaFree(s->csr_idx);
   if (s->hstage) cudaFreeHost(s->hstage);
   if (s->hwords) cudaFreeHost(s->hwords);
+  if (s->hcfl) cudaFreeHost(s->hcfl);
   delete s;
   return SPHG_OK;
 }
@@ -830,6 +865,8 @@ sphg_status sphg_create_batch(int32_t ninst, const sphg_params* p, const int64_t
     if (cudaMallocHost((void**)&s->hwords, sizeof(uint32_t) * 2 * sphg::kErrorWords) == cudaSuccess)
       std::memset(s->hwords, 0, sizeof(uint32_t) * 2 * sphg::kErrorWords);
     else st = fail(SPHG_OOM, "pinned host words");
+    if (st == SPHG_OK && cudaMallocHost((void**)&s->hcfl, sizeof(double) * 2 * ninst) != cudaSuccess)
+      st = fail(SPHG_OOM, "pinned host words");
   }
   if (st == SPHG_OK && s->n > 0 && !s->host_direct &&
       !host_stage(s, (size_t)s->n * (sizeof(float2) * 2 + sizeof(float4) + sizeof(float) + sizeof(uint32_t))))
@@ -1088,25 +1125,29 @@ sphg_status sphg_diagnostics(sphg_sim* s, double* out, void* stream) {
   return device_errors(s, st);
 }
 
+static int diag_chunk_count(const sphg_sim* s) {
+  int64_t max_n = 0;
+  for (const InstDesc& d : s->hdesc) max_n = std::max<int64_t>(max_n, d.end - d.begin);
+  return sphg::diag_chunks(max_n, s->ninst, s->diag_chunks);
+}
+
 sphg_status sphg_cfl_dt(sphg_sim* s, double cfl, double force_coef, double* out, void* stream) {
   if (!s || !out || !(cfl > 0) || !(force_coef > 0)) return fail(SPHG_INVALID_ARG, "null argument or coefficient <= 0");
   if (!s->preloop_done) return fail(SPHG_INVALID_ARG, "no computed state");
   cudaStream_t st = (cudaStream_t)stream;
+  std::vector<double> none;
+  volatile double* m = s->hcfl;
   if (s->n > 0) {
     SPHG_CUDA(sphg::launch_force(s->args(), s->opt.precision, sphg::kForceOnly, st));
-    int64_t max_n = 0;
-    for (const InstDesc& d : s->hdesc) max_n = std::max<int64_t>(max_n, d.end - d.begin);
-    const int chunks = sphg::diag_chunks(max_n, s->ninst, s->diag_chunks);
-    SPHG_CUDA(sphg::launch_cfl(s->args(), s->diag_partials, chunks, s->diag_out, st));
-  }
-  std::vector<double> m((size_t)6 * s->ninst, 0.0);
-  if (s->n > 0) {
-    SPHG_CUDA(cudaMemcpyAsync(m.data(), s->diag_out, sizeof(double) * 6 * s->ninst, cudaMemcpyDeviceToHost, st));
+    SPHG_CUDA(sphg::launch_cfl(s->args(), s->diag_partials, s->diag_tickets, diag_chunk_count(s), s->hcfl, st));
     SPHG_CUDA(cudaStreamSynchronize(st));
+  } else {
+    none.assign((size_t)2 * s->ninst, 0.0);
+    m = none.data();
   }
   for (int i = 0; i < s->ninst; ++i) {
     const sphg_params& p = s->params[i];
-    const double vmax = std::sqrt(m[6 * i]), amax = std::sqrt(m[6 * i + 1]);
+    const double vmax = std::sqrt(m[2 * i]), amax = std::sqrt(m[2 * i + 1]);
     double dt = std::numeric_limits<double>::infinity();
     if (p.c0 + vmax > 0) dt = std::min(dt, cfl * p.h / (p.c0 + vmax));
     if (amax > 0) dt = std::min(dt, force_coef * std::sqrt(p.h / amax));
@@ -1122,9 +1163,15 @@ sphg_status sphg_set_dt(sphg_sim* s, int32_t inst, double dt) {
     s->params[i].dt = dt;
     s->hdesc[i].dt = (float)dt;
   }
-  if (s->ninst > 0)
+  if (s->ninst > 1 || s->force_batched) {  // the kernels read the descriptors on the device
     SPHG_CUDA(cudaMemcpy(s->ddesc, s->hdesc.data(), sizeof(InstDesc) * s->ninst, cudaMemcpyHostToDevice));
-  s->drop_graphs();  // the single-instance descriptor is a kernel argument of the captured graphs
+  } else if (s->force_node[0] || s->force_node[1]) {
+    // one instance: its descriptor is an argument of the captured kernels, of which the force pass alone uses the
+    // time step; the instantiated graphs get the new argument before their next launch
+    s->dt_stale[0] = s->dt_stale[1] = true;
+  } else {
+    s->drop_graphs();
+  }
   return SPHG_OK;
 }
 
@@ -1141,12 +1188,6 @@ static double* device_view(sphg_sim* s, double* out) {
   if (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged) return out;
   if (at.type == cudaMemoryTypeHost) return static_cast<double*>(at.devicePointer);
   return s->host_direct ? out : nullptr;  // host_direct is set only where pageable access works
-}
-
-static int diag_chunk_count(const sphg_sim* s) {
-  int64_t max_n = 0;
-  for (const InstDesc& d : s->hdesc) max_n = std::max<int64_t>(max_n, d.end - d.begin);
-  return sphg::diag_chunks(max_n, s->ninst, s->diag_chunks);
 }
 
 sphg_status sphg_diagnostics_async(sphg_sim* s, double* out, void* stream) {
@@ -1187,8 +1228,9 @@ sphg_status sphg_step_headers(sphg_sim* s, int64_t nsteps, double* out, void* st
   const sphg::HeaderSlot h = {dv, 0u, 0u};
   SPHG_CUDA(cudaMemcpyAsync(s->hslot, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   if (s->opt.use_graph) {
-    SPHG_TRY(build_graph(s, true));
-    for (int64_t k = 0; k < nsteps; ++k) SPHG_CUDA(cudaGraphLaunch(s->gexec_hdr, st));
+    cudaGraphExec_t g = nullptr;
+    SPHG_TRY(current_graph(s, true, &g));
+    for (int64_t k = 0; k < nsteps; ++k) SPHG_CUDA(cudaGraphLaunch(g, st));
   } else {
     for (int64_t k = 0; k < nsteps; ++k) {
       SPHG_TRY(enqueue_step(s, st));

@@ -88,6 +88,7 @@ struct sphg_sim {
   // pinned words the device reports in: [0, kErrorWords) error words, then the
   // upload's "a value is not finite"
   uint32_t* hwords = nullptr;
+  double* hcfl = nullptr;  // pinned: max |v|^2, max |a|^2 of each instance
   // pinned host staging of upload/download (grows on demand)
   char* hstage = nullptr;
   size_t hstage_bytes = 0;
@@ -96,10 +97,27 @@ struct sphg_sim {
   bool cond_graph = true;       // full sort under a conditional graph node (when the merge is on)
   cudaGraphExec_t gexec = nullptr;
   cudaGraphExec_t gexec_hdr = nullptr;  // the same followed by the step header into hslot
+  // the graphs they were made from, [1] with the header, and their force pass's
+  // node (null: not step_force), whose argument holds the time step; stale: the
+  // time step changed since
+  cudaGraph_t graph[2] = {nullptr, nullptr};
+  cudaGraphNode_t force_node[2] = {nullptr, nullptr};
+  bool dt_stale[2] = {false, false};
+  void keep_graph(bool header, cudaGraph_t g, cudaGraphNode_t force) {
+    graph[header] = g;
+    force_node[header] = tile_bits ? nullptr : force;
+    dt_stale[header] = false;
+  }
   void drop_graphs() {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (gexec_hdr) cudaGraphExecDestroy(gexec_hdr);
     gexec = gexec_hdr = nullptr;
+    for (int k = 0; k < 2; ++k) {
+      if (graph[k]) cudaGraphDestroy(graph[k]);
+      graph[k] = nullptr;
+      force_node[k] = nullptr;
+      dt_stale[k] = false;
+    }
   }
 
   StepArgs args() const {

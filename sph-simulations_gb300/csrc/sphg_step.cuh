@@ -121,8 +121,9 @@ __host__ __device__ inline int diag_instance_chunks(int64_t count, int chunks) {
   const int64_t c = (count + 4095) / 4096;
   return (int)(c < 1 ? 1 : (c > chunks ? chunks : c));
 }
-// out[6*inst + {0, 1}] = max |v|^2, max |a|^2 of each instance (a.acc must hold the forces).
-cudaError_t launch_cfl(const StepArgs& a, double* partials, int chunks, double* out, cudaStream_t s);
+// out[2*inst + {0, 1}] = max |v|^2, max |a|^2 of each instance (a.acc must hold the
+// forces; out device-accessible; partials and tickets as for launch_diagnostics).
+cudaError_t launch_cfl(const StepArgs& a, double* partials, uint32_t* tickets, int chunks, double* out, cudaStream_t s);
 // CSR neighbour lists of the current state (sphg_lists.cu); returns an sphg_status.
 int lists_impl(const StepArgs& a, int precision, int64_t* offs, int32_t* idx, int64_t* total,
                cudaStream_t st, std::string* err, bool encoded = false);
