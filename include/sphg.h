@@ -329,8 +329,9 @@ sphg_status sphg_autotune(int32_t ninst, const sphg_params* p, const int64_t* co
  * phases; ms[0..4] = keys, sort, reorder (+cell ranges), density, force+integrate
  * (milliseconds, summed over the instances of the handle). */
 sphg_status sphg_profile_step(sphg_sim* s, float* ms, void* stream);
-/* Kernel launches of a main-loop iteration that runs the full sort; in a graph,
- * an iteration that merges launches SPHG_DBG_RESORT[2] fewer. */
+/* Kernel launches of a main-loop iteration that runs the full sort (an upper
+ * bound in the lists mode and for small single instances, which launch fewer);
+ * in a graph, an iteration that merges launches SPHG_DBG_RESORT[2] fewer. */
 int32_t sphg_launches_per_step(const sphg_sim* s);
 
 /* Stand-alone kernels on caller-owned DEVICE buffers. */

@@ -281,6 +281,14 @@ sphg_status enqueue_full_sort(sphg_sim* s, cudaStream_t st, const uint32_t* skip
   return SPHG_OK;
 }
 
+static sphg::ListArgs list_args(sphg_sim* s) {
+  sphg::ListArgs l = {};
+  l.words = s->list_words;
+  l.ctl = s->list_ctl;
+  l.err = sphg::sort_error_word(s->scratch);  // the same report: a look-back wait gave up
+  return l;
+}
+
 // Reorder + cell ranges, density, forces + integration (ev: events 3..5).
 // size_lists: (lists mode) size the index buffer from this iteration's total
 // first -- a host synchronisation, done on the first iteration after an upload
@@ -295,15 +303,17 @@ sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bo
   if (reorder) SPHG_CUDA(sphg::launch_reorder(a, st));
   if (ev) SPHG_CUDA(cudaEventRecord(ev[3], st));
   if (s->opt.compute == SPHG_COMPUTE_LISTS) {
-    // AssembleNeighborList: count, offsets, fill -- then density and forces over the lists
-    SPHG_CUDA(sphg::launch_lists_count_scan(a, prec, s->csr_counts, s->csr_offs, s->csr_sums, st));
+    // AssembleNeighborList, then density and forces over the lists
+    sphg::ListArgs l = list_args(s);
+    l.offs = s->csr_offs;
     if (size_lists || !s->csr_idx) {
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
       SPHG_CUDA(cudaStreamIsCapturing(st, &cs));
       if (cs != cudaStreamCaptureStatusNone)
         return fail(SPHG_INVALID_ARG, "lists mode: the neighbour-list buffer is sized before any graph capture");
-      SPHG_CUDA(cudaMemcpyAsync(&s->csr_total, s->csr_sums + sphg::lists_scan_tiles(s->n), sizeof(int64_t),
-                                cudaMemcpyDeviceToHost, st));
+      l.total = s->csr_sum;
+      SPHG_CUDA(sphg::launch_lists(a, prec, sphg::kListPacked, l, st));
+      SPHG_CUDA(cudaMemcpyAsync(&s->csr_total, s->csr_sum, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
       SPHG_CUDA(cudaStreamSynchronize(st));
       // twice this iteration's total (the lists of a compressing flow grow):
       // later iterations run without a host synchronisation and report an
@@ -321,7 +331,11 @@ sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bo
       }
     }
     const StepArgs b = s->args();
-    SPHG_CUDA(sphg::launch_lists_fill_packed(b, prec, s->csr_offs, s->csr_idx, s->csr_cap, s->flags + 8, st));
+    l.total = nullptr;
+    l.idx = s->csr_idx;
+    l.cap = s->csr_cap;
+    l.overflow = s->flags + 8;
+    SPHG_CUDA(sphg::launch_lists(b, prec, sphg::kListPacked, l, st));
     SPHG_CUDA(sphg::launch_density(b, prec, st, true));
     if (ev) SPHG_CUDA(cudaEventRecord(ev[4], st));
     SPHG_CUDA(sphg::launch_force(b, prec, sphg::kForceIntegrate, st, true));
@@ -660,10 +674,11 @@ sphg_status alloc_arena(sphg_sim* s, size_t N, uint64_t keys, int ninst, int dia
       r.cap = (int64_t)N;
     }
     if (s->opt.compute == SPHG_COMPUTE_LISTS) {
-      s->csr_counts = A.take<int32_t>(N);
       s->csr_offs = A.take<int64_t>(N + 1);
-      s->csr_sums = A.take<int64_t>((size_t)sphg::lists_scan_tiles((int64_t)N) + 1);
+      s->csr_sum = A.take<int64_t>(1);
     }
+    s->list_words = A.take<unsigned long long>((size_t)sphg::lists_blocks((int64_t)N));
+    s->list_ctl = A.take<uint32_t>(4);
     if (s->tile_bits) {
       s->tile_ranges = A.take<uint2>((keys >> (2 * s->tile_bits)) + 1);
       s->tile_list = A.take<uint32_t>(std::min<uint64_t>(N, (keys >> (2 * s->tile_bits)) + 1));
@@ -752,6 +767,9 @@ sphg_status destroy_impl(sphg_sim* s) {
   if (s->cap_stream2) cudaStreamDestroy(s->cap_stream2);
   if (s->arena.base) cudaFree(s->arena.base);
   if (s->csr_idx) cudaFree(s->csr_idx);
+  if (s->exp_offs) cudaFree(s->exp_offs);
+  if (s->exp_idx) cudaFree(s->exp_idx);
+  if (s->htotal) cudaFreeHost(s->htotal);
   if (s->hstage) cudaFreeHost(s->hstage);
   if (s->hwords) cudaFreeHost(s->hwords);
   if (s->hcfl) cudaFreeHost(s->hcfl);
@@ -1310,22 +1328,83 @@ sphg_status sphg_get_debug(sphg_sim* s, int32_t which, void* host, void* stream)
   }
 }
 
+// Device memory into a host array of the caller's, in stream order: written by
+// the device where it reaches the array (its pages touched first), else copied.
+static sphg_status copy_out(sphg_sim* s, void* host, const void* dev, size_t bytes, cudaStream_t st) {
+  if (s->host_direct) {
+    void* const arrays[8] = {host};
+    const size_t sizes[8] = {bytes};
+    touch_pages(arrays, sizes);
+    SPHG_CUDA(sphg::launch_host_copy(static_cast<uint32_t*>(host), static_cast<const uint32_t*>(dev),
+                                     (int64_t)(bytes / sizeof(uint32_t)), st));
+  } else {
+    SPHG_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st));
+  }
+  return SPHG_OK;
+}
+
+// The lists of the current state into host arrays (offs, idx: null to leave out).
+// The device buffers stay with the handle; a call whose lists outgrow them
+// assembles again.
+static sphg_status export_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_t* total, int form, cudaStream_t st) {
+  const int64_t n = s->n;
+  if (total) *total = 0;
+  if (n == 0) {
+    if (offs) offs[0] = 0;
+    return SPHG_OK;
+  }
+  if (!s->exp_offs) {
+    if (cudaMalloc((void**)&s->exp_offs, (size_t)(n + 1) * sizeof(int64_t)) != cudaSuccess ||
+        (!s->htotal && cudaMallocHost((void**)&s->htotal, sizeof(int64_t)) != cudaSuccess)) {
+      cudaGetLastError();
+      return fail(SPHG_OOM, "neighbour-list buffers");
+    }
+  }
+  auto grow = [&](int64_t entries) -> sphg_status {
+    if (entries <= s->exp_cap) return SPHG_OK;
+    if (s->exp_idx) SPHG_CUDA(cudaFree(s->exp_idx));
+    s->exp_idx = nullptr;
+    s->exp_cap = 0;
+    if (cudaMalloc((void**)&s->exp_idx, (size_t)entries * sizeof(uint32_t)) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(SPHG_OOM, "neighbour-list buffers");
+    }
+    s->exp_cap = entries;
+    return SPHG_OK;
+  };
+  sphg::ListArgs l = list_args(s);
+  l.offs = s->exp_offs;
+  l.total = s->htotal;
+  int64_t tot = 0;
+  for (int round = 0; round < 2; ++round) {
+    l.idx = idx ? s->exp_idx : nullptr;
+    l.cap = s->exp_cap;
+    SPHG_CUDA(sphg::launch_lists(s->args(), s->opt.precision, form, l, st));
+    if (round == 0 && offs) SPHG_TRY(copy_out(s, offs, s->exp_offs, (size_t)(n + 1) * sizeof(int64_t), st));
+    SPHG_CUDA(cudaStreamSynchronize(st));
+    tot = *(volatile int64_t*)s->htotal;
+    if (!idx || tot <= l.cap) break;
+    SPHG_TRY(grow(tot));
+  }
+  if (total) *total = tot;
+  if (!idx) return grow(tot);  // for the call that asks for the entries
+  if (tot > 0) {
+    SPHG_TRY(copy_out(s, idx, s->exp_idx, (size_t)tot * sizeof(int32_t), st));
+    SPHG_CUDA(cudaStreamSynchronize(st));
+  }
+  return SPHG_OK;
+}
+
 sphg_status sphg_neighbor_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_t* total,
                                 void* stream) {
   if (!s || !s->preloop_done) return fail(SPHG_INVALID_ARG, "no computed state");
-  std::string err;
-  int st = sphg::lists_impl(s->args(), s->opt.precision, offs, idx, total, (cudaStream_t)stream, &err);
-  if (st != SPHG_OK) return fail((sphg_status)st, err);
-  return SPHG_OK;
+  return export_lists(s, offs, idx, total, sphg::kListIndices, (cudaStream_t)stream);
 }
 
 sphg_status sphg_neighbor_lists_encoded(sphg_sim* s, int64_t* offs, int32_t* enc, int64_t* total,
                                         void* stream) {
   if (!s || !s->preloop_done) return fail(SPHG_INVALID_ARG, "no computed state");
-  std::string err;
-  int st = sphg::lists_impl(s->args(), s->opt.precision, offs, enc, total, (cudaStream_t)stream, &err, true);
-  if (st != SPHG_OK) return fail((sphg_status)st, err);
-  return SPHG_OK;
+  return export_lists(s, offs, enc, total, sphg::kListCoded, (cudaStream_t)stream);
 }
 
 sphg_status sphg_delta_encode(const int64_t* offs, const int32_t* idx, int64_t n, int32_t* enc,
@@ -1436,9 +1515,11 @@ int32_t sphg_launches_per_step(const sphg_sim* s) {
   if (!s || s->n == 0) return 0;
   const int passes = (s->key_bits + 7) / 8;
   // an iteration that runs the full sort: its histogram kernel + radix passes +
-  // reorder + density + force (+ the incremental re-sort's merge kernel; + list
-  // count, three scan kernels and list fill in the lists mode).  An iteration
-  // that merges launches (key_bits + 7) / 8 + 2 kernels fewer in a graph.
+  // reorder + density + force (+ the incremental re-sort's merge kernel).  An
+  // iteration that merges launches (key_bits + 7) / 8 + 2 kernels fewer in a
+  // graph.  An upper bound: the lists mode assembles its lists in one kernel of
+  // the five counted for count, scan and fill, and a small single instance runs
+  // many iterations in one launch.
   // With the single-launch iteration: the launch (which only decides), the
   // histogram + radix passes and the launch's post part; an iteration that
   // merges is the one launch.

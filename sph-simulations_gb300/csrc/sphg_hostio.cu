@@ -174,6 +174,11 @@ __global__ void download_direct_kernel(StepArgs a, int precision, double* __rest
   write(ids, [&](int64_t i) { return a.track_ids ? a.idsA[i] : -1; });
 }
 
+__global__ void host_copy_kernel(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int64_t words) {
+  const int64_t i = line_entry(dst, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= 0 && i < words) dst[i] = src[i];
+}
+
 bool aligned(const void* p, uintptr_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; }
 
 }  // namespace
@@ -191,6 +196,12 @@ cudaError_t launch_upload_direct(const StepArgs& a, int precision, const double*
     upload_direct_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a, precision, x, y, vx, vy, first_bad,
                                                                           any_bad);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_host_copy(uint32_t* dst, const uint32_t* src, int64_t words, cudaStream_t st) {
+  if (words <= 0) return cudaSuccess;
+  host_copy_kernel<<<(unsigned)((words + kLineEntries + 255) / 256), 256, 0, st>>>(dst, src, words);
   return cudaGetLastError();
 }
 

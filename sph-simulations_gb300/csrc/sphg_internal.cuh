@@ -67,10 +67,16 @@ struct sphg_sim {
   int nbr_slots = 0;
   // lists mode: CSR of each iteration; the index buffer is sized at the pre-loop
   // (twice the list total then) and an overflow past it is reported
-  int32_t* csr_counts = nullptr;
-  int64_t *csr_offs = nullptr, *csr_sums = nullptr;
+  int64_t *csr_offs = nullptr, *csr_sum = nullptr;
   uint32_t* csr_idx = nullptr;
   int64_t csr_cap = 0, csr_total = 0;
+  // look-back words and counters of the list assembly (every compute mode)
+  unsigned long long* list_words = nullptr;
+  uint32_t* list_ctl = nullptr;
+  // exported lists: device buffers, made at the first export and kept
+  int64_t* exp_offs = nullptr;
+  uint32_t* exp_idx = nullptr;
+  int64_t exp_cap = 0;
   // incremental re-sort: the record written by the force pass
   bool movers_on = false;
   bool force_full_sort = false;  // the next iteration sorts fully (the slot record is stale)
@@ -88,6 +94,7 @@ struct sphg_sim {
   // pinned words the device reports in: [0, kErrorWords) error words, then the
   // upload's "a value is not finite"
   uint32_t* hwords = nullptr;
+  int64_t* htotal = nullptr;  // pinned: entries of the exported lists
   double* hcfl = nullptr;  // pinned: max |v|^2, max |a|^2 of each instance
   // pinned host staging of upload/download (grows on demand)
   char* hstage = nullptr;

@@ -85,13 +85,25 @@ cudaError_t launch_resident(const StepArgs& a, const MoverArgs& m, int precision
 cudaError_t launch_reorder(const StepArgs& a, cudaStream_t s);
 cudaError_t launch_density(const StepArgs& a, int precision, cudaStream_t s, bool csr = false);
 cudaError_t launch_force(const StepArgs& a, int precision, int mode, cudaStream_t s, bool csr = false);
-// Lists mode: per-particle counts, exclusive scan to int64 offsets (the total
-// lands in sums[scan_tiles(n)]), fill of packed entries (at most cap).
-int lists_scan_tiles(int64_t n);
-cudaError_t launch_lists_count_scan(const StepArgs& a, int precision, int32_t* counts, int64_t* offs,
-                                    int64_t* sums, cudaStream_t st);
-cudaError_t launch_lists_fill_packed(const StepArgs& a, int precision, const int64_t* offs,
-                                     uint32_t* idx, int64_t cap, uint32_t* overflow, cudaStream_t st);
+// CSR neighbour lists of the current state in one launch (sphg_lists.cu).
+// offs: n + 1 entries; idx: entries of the lists in `form`, at most cap (null:
+// offsets and total only); *overflow set when they would be more; total
+// (device-accessible) or null.  words: lists_blocks(n), ctl: 4 words, both zero
+// before the first launch and not shared between launches that overlap; *err set
+// when a look-back wait gave up.
+enum ListForm { kListIndices = 0, kListPacked = 1, kListCoded = 2 };  // j; j << 5 | tag; ascending, delta-coded
+struct ListArgs {
+  int64_t* offs;
+  uint32_t* idx;
+  int64_t cap;
+  uint32_t* overflow;
+  int64_t* total;
+  unsigned long long* words;
+  uint32_t* ctl;
+  uint32_t* err;
+};
+int64_t lists_blocks(int64_t n);
+cudaError_t launch_lists(const StepArgs& a, int precision, int form, const ListArgs& o, cudaStream_t st);
 // Per-instance diagnostics in one launch: float-float partials per (chunk,
 // instance) block, then the last block of an instance (ticket counter) sums them
 // in a fixed order; out[6*inst + {0..5}] = E_k, max|v|^2, inside, sum m vx,
@@ -124,9 +136,6 @@ __host__ __device__ inline int diag_instance_chunks(int64_t count, int chunks) {
 // out[2*inst + {0, 1}] = max |v|^2, max |a|^2 of each instance (a.acc must hold the
 // forces; out device-accessible; partials and tickets as for launch_diagnostics).
 cudaError_t launch_cfl(const StepArgs& a, double* partials, uint32_t* tickets, int chunks, double* out, cudaStream_t s);
-// CSR neighbour lists of the current state (sphg_lists.cu); returns an sphg_status.
-int lists_impl(const StepArgs& a, int precision, int64_t* offs, int32_t* idx, int64_t* total,
-               cudaStream_t st, std::string* err, bool encoded = false);
 // Delta codec of CSR lists on device buffers (encode: in = ascending lists).
 cudaError_t launch_delta(bool encode, const int64_t* offs, const int32_t* in, int64_t n, int32_t* out,
                          cudaStream_t st);
@@ -150,6 +159,9 @@ cudaError_t launch_upload_direct(const StepArgs& a, int precision, const double*
 cudaError_t launch_download_direct(const StepArgs& a, int precision, double* x, double* y, double* vx, double* vy,
                                    double* rho, double* fx, double* fy, int32_t* ids, const HostErrors& errors,
                                    cudaStream_t st);
+// `words` 32-bit words of device memory into the caller's host array (4-byte
+// aligned, its pages resident), from the device.
+cudaError_t launch_host_copy(uint32_t* dst, const uint32_t* src, int64_t words, cudaStream_t st);
 // A served request's lattice initial state into the admission staging (sphg_init.cu).
 cudaError_t launch_lattice_stage(const InstDesc& d, const sphg_lattice& L, int precision, int64_t n, float2* pos,
                                  float2* vel, uint32_t* key, int32_t* ids, cudaStream_t st);
