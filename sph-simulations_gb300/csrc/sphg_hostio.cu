@@ -36,6 +36,20 @@ __device__ __forceinline__ void report_errors(const HostErrors& e) {
   for (int k = 0; k < kErrorWords; ++k) e.out[k] = *e.word[k];
 }
 
+// An FP64 position as its cell (clamped to [0, cmax]) and FP32 offset in it.
+__device__ __forceinline__ float2 split_position(const InstDesc& d, double x, double y, int cmx, int cmy, int& cx,
+                                                 int& cy) {
+  const double qx = floor_div(__dsub_rn(x, d.lo_xd), d.cs_xd, d.inv_cs_xd);
+  const double qy = floor_div(__dsub_rn(y, d.lo_yd), d.cs_yd, d.inv_cs_yd);
+  cx = !(qx < (double)cmx) ? cmx : (qx < 0.0 ? 0 : (int)qx);
+  cy = !(qy < (double)cmy) ? cmy : (qy < 0.0 ? 0 : (int)qy);
+  float fx = __double2float_rn(__dsub_rn(__dsub_rn(x, d.lo_xd), __dmul_rn((double)cx, d.cs_xd)));
+  float fy = __double2float_rn(__dsub_rn(__dsub_rn(y, d.lo_yd), __dmul_rn((double)cy, d.cs_yd)));
+  if ((double)fx >= d.cs_xd) fx = nextafterf(fx, 0.0f);
+  if ((double)fy >= d.cs_yd) fy = nextafterf(fy, 0.0f);
+  return make_float2(fx, fy);
+}
+
 // One particle of the caller's FP64 state into the device representation
 // (false: not finite, nothing written).
 __device__ __forceinline__ bool upload_one(const StepArgs& a, int precision, int64_t i, double xi, double yi,
@@ -46,15 +60,8 @@ __device__ __forceinline__ bool upload_one(const StepArgs& a, int precision, int
     const InstDesc& d = inst_ref<true>(a, i);
     const int cmx = d.periodic ? d.nxr - 1 : d.nx - 1;
     const int cmy = d.periodic ? d.nyr - 1 : d.ny - 1;
-    const double qx = floor_div(__dsub_rn(xi, d.lo_xd), d.cs_xd, d.inv_cs_xd);
-    const double qy = floor_div(__dsub_rn(yi, d.lo_yd), d.cs_yd, d.inv_cs_yd);
-    const int cx = !(qx < (double)cmx) ? cmx : (qx < 0.0 ? 0 : (int)qx);
-    const int cy = !(qy < (double)cmy) ? cmy : (qy < 0.0 ? 0 : (int)qy);
-    float fx = __double2float_rn(__dsub_rn(__dsub_rn(xi, d.lo_xd), __dmul_rn((double)cx, d.cs_xd)));
-    float fy = __double2float_rn(__dsub_rn(__dsub_rn(yi, d.lo_yd), __dmul_rn((double)cy, d.cs_yd)));
-    if ((double)fx >= d.cs_xd) fx = nextafterf(fx, 0.0f);
-    if ((double)fy >= d.cs_yd) fy = nextafterf(fy, 0.0f);
-    pos = make_float2(fx, fy);
+    int cx, cy;
+    pos = split_position(d, xi, yi, cmx, cmy, cx, cy);
     key = d.cell_base + local_code(d, cx, cy);
   } else {
     pos = make_float2((float)xi, (float)yi);
@@ -174,6 +181,46 @@ __global__ void download_direct_kernel(StepArgs a, int precision, double* __rest
   write(ids, [&](int64_t i) { return a.track_ids ? a.idsA[i] : -1; });
 }
 
+// A served request's host arrays into the admission staging: device
+// representation, instance-local cell code of the held position, creation index.
+__global__ void stage_direct_kernel(InstDesc d, int precision, int64_t n, const double* __restrict__ x,
+                                    const double* __restrict__ y, const double* __restrict__ vx,
+                                    const double* __restrict__ vy, float2* __restrict__ pos, float2* __restrict__ vel,
+                                    uint32_t* __restrict__ key, int32_t* __restrict__ ids) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int cmx = d.periodic ? d.nxr - 1 : d.nx - 1;
+  const int cmy = d.periodic ? d.nyr - 1 : d.ny - 1;
+  int cx, cy;
+  float2 p;
+  if (precision == SPHG_PRECISION_SPLIT) {
+    p = split_position(d, x[i], y[i], cmx, cmy, cx, cy);
+  } else {
+    p = make_float2((float)x[i], (float)y[i]);
+    cx = cell_coord(p.x, d.lo_x, d.inv_cs_x, d.lo_xd, d.cs_xd, cmx);
+    cy = cell_coord(p.y, d.lo_y, d.inv_cs_y, d.lo_yd, d.cs_yd, cmy);
+  }
+  pos[i] = p;
+  vel[i] = make_float2((float)vx[i], (float)vy[i]);
+  key[i] = local_code(d, cx, cy);
+  if (ids) ids[i] = (int32_t)i;
+}
+
+// Slots [first, first + n) as a result: x, y, vx, vy, rho (FP64) and the creation
+// indices, n entries each, one after the other.
+__global__ void result_kernel(StepArgs a, int precision, int64_t first, int64_t n, double* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t q = first + i;
+  const float4 v = a.velpA[q];
+  out[i] = download_position(a, precision, q, 0);
+  out[n + i] = download_position(a, precision, q, 1);
+  out[2 * n + i] = v.x;
+  out[3 * n + i] = v.y;
+  out[4 * n + i] = a.rho[q];
+  reinterpret_cast<int32_t*>(out + 5 * n)[i] = a.track_ids ? a.idsA[q] : -1;
+}
+
 __global__ void host_copy_kernel(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int64_t words) {
   const int64_t i = line_entry(dst, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= 0 && i < words) dst[i] = src[i];
@@ -196,6 +243,20 @@ cudaError_t launch_upload_direct(const StepArgs& a, int precision, const double*
     upload_direct_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a, precision, x, y, vx, vy, first_bad,
                                                                           any_bad);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_stage_direct(const InstDesc& d, int precision, int64_t n, const double* x, const double* y,
+                                const double* vx, const double* vy, float2* pos, float2* vel, uint32_t* key,
+                                int32_t* ids, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  stage_direct_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, precision, n, x, y, vx, vy, pos, vel, key, ids);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_result(const StepArgs& a, int precision, int64_t first, int64_t n, double* out, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  result_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, precision, first, n, out);
   return cudaGetLastError();
 }
 

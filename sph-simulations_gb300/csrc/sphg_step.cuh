@@ -162,6 +162,14 @@ cudaError_t launch_download_direct(const StepArgs& a, int precision, double* x, 
 // `words` 32-bit words of device memory into the caller's host array (4-byte
 // aligned, its pages resident), from the device.
 cudaError_t launch_host_copy(uint32_t* dst, const uint32_t* src, int64_t words, cudaStream_t st);
+// A served request's host arrays (device-readable) into the admission staging:
+// positions, velocities, instance-local cell codes, creation indices (or null).
+cudaError_t launch_stage_direct(const InstDesc& d, int precision, int64_t n, const double* x, const double* y,
+                                const double* vx, const double* vy, float2* pos, float2* vel, uint32_t* key,
+                                int32_t* ids, cudaStream_t st);
+// Slots [first, first + n) as x, y, vx, vy, rho (FP64, n entries each) and the
+// creation indices into out (device-accessible).
+cudaError_t launch_result(const StepArgs& a, int precision, int64_t first, int64_t n, double* out, cudaStream_t st);
 // A served request's lattice initial state into the admission staging (sphg_init.cu).
 cudaError_t launch_lattice_stage(const InstDesc& d, const sphg_lattice& L, int precision, int64_t n, float2* pos,
                                  float2* vel, uint32_t* key, int32_t* ids, cudaStream_t st);
