@@ -109,12 +109,14 @@ typedef struct sphg_options {
                           (twice that iteration's total) and runs without cell tiles;
                           lists that later outgrow it make sphg_download /
                           sphg_diagnostics return SPHG_CAPACITY */
-  int32_t resort;      /* 1 (default): when at most a quarter of the particles (or 8,192)
-                          changed cell since the last iteration, re-sort by merging them
-                          into the unchanged (already sorted) rest -- the same stable order
-                          as the full radix sort, which runs otherwise (also when more than
-                          64 of them enter one gap of the order, or more than 512 one run
-                          of 512 slots); 0: full radix sort every iteration */
+  int32_t resort;      /* 1 (default): re-sort by merging the particles that changed cell
+                          since the last iteration into the unchanged (already sorted)
+                          rest -- the same stable order as the full radix sort, which runs
+                          instead when very many changed (a quarter and more than 8,192
+                          of up to 65,536 particles; a third of more in the iteration
+                          before), when more than 64 of them enter one gap of the order or
+                          more than 512 one run of 512 slots; 0: full radix sort every
+                          iteration */
   int32_t block_threads;/* threads per block of the density and force passes: 0 = default
                           (128), 64, 128 or 256 */
   int32_t cell_pairs;  /* density pass: 0 (default) one particle per thread; 1 one thread

@@ -294,10 +294,12 @@ static sphg::ListArgs list_args(sphg_sim* s) {
 // first -- a host synchronisation, done on the first iteration after an upload
 // (never inside a graph capture).
 // reorder: the gather after a full sort is launched here (else the caller has
-// placed it with the sort).
+// placed it with the sort).  guarded: the passes return at once when the merge
+// left the iteration to the full sort.
 sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bool size_lists = false,
-                               bool reorder = true, bool header = false) {
-  const StepArgs a = s->args();
+                               bool reorder = true, bool header = false, bool guarded = false) {
+  StepArgs a = s->args();
+  if (guarded) a.go = s->flags + 3;
   const int prec = s->opt.precision;
   if (s->tile_bits) SPHG_CUDA(cudaMemsetAsync(s->flags + 1, 0, sizeof(uint32_t), st));
   if (reorder) SPHG_CUDA(sphg::launch_reorder(a, st));
@@ -330,7 +332,8 @@ sphg_status enqueue_after_sort(sphg_sim* s, cudaStream_t st, cudaEvent_t* ev, bo
         s->csr_cap = cap;
       }
     }
-    const StepArgs b = s->args();
+    StepArgs b = s->args();
+    b.go = a.go;
     l.total = nullptr;
     l.idx = s->csr_idx;
     l.cap = s->csr_cap;
@@ -367,7 +370,7 @@ sphg_status enqueue_step(sphg_sim* s, cudaStream_t st, bool first, cudaEvent_t* 
     const bool inc = !first && !s->force_full_sort;
     s->force_full_sort = false;
     if (inc) SPHG_TRY(enqueue_fused(s, st, false, 0));
-    else SPHG_CUDA(cudaMemsetAsync(s->flags + 3, 0, sizeof(uint32_t), st));
+    else SPHG_CUDA(cudaMemsetAsync(s->flags + 3, 0, 2 * sizeof(uint32_t), st));
     SPHG_TRY(enqueue_full_sort(s, st, inc ? s->flags + 3 : nullptr));
     return enqueue_fused(s, st, true, 0);
   }
@@ -379,36 +382,32 @@ sphg_status enqueue_step(sphg_sim* s, cudaStream_t st, bool first, cudaEvent_t* 
   const bool inc = s->movers_on && !first && !s->force_full_sort;
   s->force_full_sort = false;
   if (inc) SPHG_TRY(enqueue_movers(s, st, 0));
-  // without the merge this iteration, its decision word must read "full sort"
-  else if (s->movers_on) SPHG_CUDA(cudaMemsetAsync(s->flags + 3, 0, sizeof(uint32_t), st));
+  // without the merge this iteration, its decision word must read "full sort" (and
+  // no movers before it)
+  else if (s->movers_on) SPHG_CUDA(cudaMemsetAsync(s->flags + 3, 0, 2 * sizeof(uint32_t), st));
   SPHG_TRY(enqueue_full_sort(s, st, inc ? s->flags + 3 : nullptr));
   if (ev) SPHG_CUDA(cudaEventRecord(ev[2], st));
   return enqueue_after_sort(s, st, ev, first);
 }
 
 // The step header of the current state into the header slot (graph-capturable).
-sphg_status enqueue_header(sphg_sim* s, cudaStream_t st) {
+sphg_status enqueue_header(sphg_sim* s, cudaStream_t st, bool guarded = false) {
+  StepArgs a = s->args();
+  if (guarded) a.go = s->flags + 3;
   int64_t max_n = 0;
   for (const InstDesc& d : s->hdesc) max_n = std::max<int64_t>(max_n, d.end - d.begin);
-  SPHG_CUDA(sphg::launch_diagnostics_slot(s->args(), s->opt.precision, s->diag_partials, s->diag_tickets,
+  SPHG_CUDA(sphg::launch_diagnostics_slot(a, s->opt.precision, s->diag_partials, s->diag_tickets,
                                           sphg::diag_chunks(max_n, s->ninst, s->diag_chunks), s->hslot, st));
   return SPHG_OK;
 }
 
-// The node that what is captured next depends on: the kernel captured last (null
-// where the force pass is another kernel than step_force).
-static sphg_status last_node(cudaStream_t st, cudaGraphNode_t* node) {
-  cudaStreamCaptureStatus cst;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t ndeps = 0;
-  SPHG_CUDA(cudaStreamGetCaptureInfo(st, &cst, nullptr, nullptr, &deps, nullptr, &ndeps));
-  *node = ndeps == 1 ? deps[0] : nullptr;
-  return SPHG_OK;
-}
-
-// Graph of one iteration with the full sort under a conditional node: the
-// incremental re-sort's decision kernel switches it off, so iterations that
-// merge launch none of the full sort's kernels.
+// Graph of one iteration with the full sort under a conditional node that the
+// merge's decision switches: merge -> density -> forces (-> header), and beside
+// them, after the merge, the conditional node with the full sort, the reorder and
+// the same passes.  The passes of the chain return at once when the merge did
+// not take the iteration, so that only one of the two does anything; an iteration
+// that merges does not wait for the conditional node (between the merge and the
+// density pass its evaluation cost 2 to 3 us an iteration).
 
 sphg_status build_graph_conditional(sphg_sim* s, cudaGraphExec_t* exec, bool header) {
   if (!s->cap_stream2) SPHG_CUDA(cudaStreamCreateWithFlags(&s->cap_stream2, cudaStreamNonBlocking));
@@ -457,27 +456,27 @@ sphg_status build_graph_conditional(sphg_sim* s, cudaGraphExec_t* exec, bool hea
     return done(fail(SPHG_CUDA_ERROR, "capture of the conditional body"));
   st = enqueue_full_sort(s, s->cap_stream2, nullptr);
   if (st == SPHG_OK && fused) st = enqueue_fused(s, s->cap_stream2, true, 0);  // reorder, density, forces
-  if (st == SPHG_OK && !fused && sphg::launch_reorder(s->args(), s->cap_stream2) != cudaSuccess)
-    st = fail(SPHG_CUDA_ERROR, "reorder in the conditional body");
+  if (st == SPHG_OK && !fused) st = enqueue_after_sort(s, s->cap_stream2, nullptr, false, true, header);
+  if (st == SPHG_OK && !fused && header) st = enqueue_header(s, s->cap_stream2);
   cudaGraph_t body_out = nullptr;
   const cudaError_t eb = cudaStreamEndCapture(s->cap_stream2, &body_out);
   if (st != SPHG_OK) return done(st);
   if (eb != cudaSuccess) return done(fail(SPHG_CUDA_ERROR, "end of the conditional body capture"));
-  if (cudaStreamUpdateCaptureDependencies(s->cap_stream, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies) != cudaSuccess)
+  // (single-launch iterations: the header waits for both)
+  if (fused && cudaStreamUpdateCaptureDependencies(s->cap_stream, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies) != cudaSuccess)
     return done(fail(SPHG_CUDA_ERROR, "capture dependencies"));
-  if (!fused) st = enqueue_after_sort(s, s->cap_stream, nullptr, false, false, header);
-  cudaGraphNode_t force = nullptr;
-  if (st == SPHG_OK && !fused) st = last_node(s->cap_stream, &force);
-  if (st == SPHG_OK && header) st = enqueue_header(s, s->cap_stream);
+  if (!fused) st = enqueue_after_sort(s, s->cap_stream, nullptr, false, false, header, true);
+  if (st == SPHG_OK && header) st = enqueue_header(s, s->cap_stream, !fused);
   if (st != SPHG_OK) return done(st);
   cudaGraph_t out = nullptr;
   if (cudaStreamEndCapture(s->cap_stream, &out) != cudaSuccess) return done(fail(SPHG_CUDA_ERROR, "end capture"));
   const cudaError_t e = cudaGraphInstantiate(exec, g, 0);
+  cudaGraphDestroy(g);
+  g = nullptr;
   if (e != cudaSuccess) {
     *exec = nullptr;
-    return done(fail(SPHG_CUDA_ERROR, std::string("instantiate: ") + cudaGetErrorString(e)));
+    return fail(SPHG_CUDA_ERROR, std::string("instantiate: ") + cudaGetErrorString(e));
   }
-  s->keep_graph(header, g, force);
   return SPHG_OK;
 }
 
@@ -495,8 +494,6 @@ sphg_status build_graph(sphg_sim* s, bool header) {
   cudaGraph_t g = nullptr;
   SPHG_CUDA(cudaStreamBeginCapture(s->cap_stream, cudaStreamCaptureModeThreadLocal));
   sphg_status st = enqueue_step(s, s->cap_stream);
-  cudaGraphNode_t force = nullptr;
-  if (st == SPHG_OK && !fused_on(s)) st = last_node(s->cap_stream, &force);
   if (st == SPHG_OK && header) st = enqueue_header(s, s->cap_stream);
   cudaError_t e = cudaStreamEndCapture(s->cap_stream, &g);
   if (st != SPHG_OK) {
@@ -505,27 +502,21 @@ sphg_status build_graph(sphg_sim* s, bool header) {
   }
   SPHG_CUDA(e);
   e = cudaGraphInstantiate(exec, g, 0);
-  if (e != cudaSuccess) cudaGraphDestroy(g);
+  cudaGraphDestroy(g);
   SPHG_CUDA(e);
-  s->keep_graph(header, g, force);
   return SPHG_OK;
 }
 
-// The instantiated graph, its force pass's argument brought up to date after a
-// change of the time step.
-static sphg_status current_graph(sphg_sim* s, bool header, cudaGraphExec_t* out) {
-  SPHG_TRY(build_graph(s, header));
-  *out = header ? s->gexec_hdr : s->gexec;
-  if (!s->dt_stale[header]) return SPHG_OK;
-  cudaKernelNodeParams p = {};
-  SPHG_CUDA(cudaGraphKernelNodeGetParams(s->force_node[header], &p));
-  StepArgs a = *static_cast<const StepArgs*>(p.kernelParams[0]);  // as it was captured
-  a.d0 = s->hdesc[0];
-  void* args[1] = {&a};
-  p.kernelParams = args;
-  p.extra = nullptr;
-  SPHG_CUDA(cudaGraphExecKernelNodeSetParams(*out, s->force_node[header], &p));
-  s->dt_stale[header] = false;
+// Brings the device word of the time step up to date in stream order: what is
+// enqueued already keeps the old one.
+__global__ void write_word(float* p, float v) { *p = v; }
+static sphg_status current_dt(sphg_sim* s, cudaStream_t st) {
+  if (!s->dt_stale || s->ninst != 1 || s->force_batched) return SPHG_OK;
+  write_word<<<1, 1, 0, st>>>(s->dt_word, s->hdesc[0].dt);
+  SPHG_CUDA(cudaGetLastError());
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  // in a caller's capture it is written when that is replayed
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) s->dt_stale = false;
   return SPHG_OK;
 }
 
@@ -547,15 +538,15 @@ static sphg_status run_resident(sphg_sim* s, int64_t k, double* headers, cudaStr
 
 sphg_status run_steps(sphg_sim* s, int64_t k, cudaStream_t st, bool first = false) {
   if (s->n == 0) return SPHG_OK;
+  SPHG_TRY(current_dt(s, st));
   if (first) {
     SPHG_TRY(enqueue_step(s, st, true));
     --k;
   }
   if (resident_on(s)) return run_resident(s, k, nullptr, st);
   if (s->opt.use_graph) {
-    cudaGraphExec_t g = nullptr;
-    SPHG_TRY(current_graph(s, false, &g));
-    for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(g, st));
+    SPHG_TRY(build_graph(s));
+    for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(s->gexec, st));
   } else {
     for (int64_t i = 0; i < k; ++i) SPHG_TRY(enqueue_step(s, st));
   }
@@ -649,6 +640,7 @@ sphg_status alloc_arena(sphg_sim* s, size_t N, uint64_t keys, int ninst, int dia
     s->valTmp = A.take<uint32_t>(N);
     s->scratch = A.take<uint32_t>(sphg::sort_scratch_words(N));
     s->flags = A.take<uint32_t>(32);
+    s->dt_word = reinterpret_cast<float*>(s->flags + 16);
     s->diag_partials = A.take<double>((size_t)ninst * s->diag_chunks * 6);
     s->diag_out = A.take<double>((size_t)ninst * 6);
     s->hslot = A.take<sphg::HeaderSlot>(1);
@@ -720,6 +712,7 @@ sphg_status apply_layout(sphg_sim* s, int ninst, const sphg_params* p, const int
   s->params.assign(p, p + ninst);
   s->counts.assign(counts, counts + ninst);
   s->hdesc = L.desc;
+  s->dt_stale = true;
   s->hbegins = L.begins;
   s->n = L.n;
   s->total_keys = L.keys;
@@ -756,6 +749,10 @@ sphg_status apply_layout(sphg_sim* s, int ninst, const sphg_params* p, const int
     SPHG_CUDA(cudaMemcpy(s->dbegins, s->hbegins.data(), sizeof(int32_t) * ninst, cudaMemcpyHostToDevice));
     SPHG_CUDA(cudaMemcpy(s->dinst_tab, s->hinst_tab.data(), sizeof(int32_t) * blocks, cudaMemcpyHostToDevice));
     if (ntab) SPHG_CUDA(cudaMemcpy(s->ddiag_tab, s->hdiag_tab.data(), sizeof(uint32_t) * ntab, cudaMemcpyHostToDevice));
+    if (ninst == 1) {
+      SPHG_CUDA(cudaMemcpy(s->dt_word, &s->hdesc[0].dt, sizeof(float), cudaMemcpyHostToDevice));
+      s->dt_stale = false;
+    }
   }
   return SPHG_OK;
 }
@@ -1183,12 +1180,8 @@ sphg_status sphg_set_dt(sphg_sim* s, int32_t inst, double dt) {
   }
   if (s->ninst > 1 || s->force_batched) {  // the kernels read the descriptors on the device
     SPHG_CUDA(cudaMemcpy(s->ddesc, s->hdesc.data(), sizeof(InstDesc) * s->ninst, cudaMemcpyHostToDevice));
-  } else if (s->force_node[0] || s->force_node[1]) {
-    // one instance: its descriptor is an argument of the captured kernels, of which the force pass alone uses the
-    // time step; the instantiated graphs get the new argument before their next launch
-    s->dt_stale[0] = s->dt_stale[1] = true;
   } else {
-    s->drop_graphs();
+    s->dt_stale = true;  // written to the device before the next iteration
   }
   return SPHG_OK;
 }
@@ -1242,13 +1235,13 @@ sphg_status sphg_step_headers(sphg_sim* s, int64_t nsteps, double* out, void* st
     }
     return SPHG_OK;
   }
+  SPHG_TRY(current_dt(s, st));
   if (resident_on(s)) return run_resident(s, nsteps, dv, st);
   const sphg::HeaderSlot h = {dv, 0u, 0u};
   SPHG_CUDA(cudaMemcpyAsync(s->hslot, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   if (s->opt.use_graph) {
-    cudaGraphExec_t g = nullptr;
-    SPHG_TRY(current_graph(s, true, &g));
-    for (int64_t k = 0; k < nsteps; ++k) SPHG_CUDA(cudaGraphLaunch(g, st));
+    SPHG_TRY(build_graph(s, true));
+    for (int64_t k = 0; k < nsteps; ++k) SPHG_CUDA(cudaGraphLaunch(s->gexec_hdr, st));
   } else {
     for (int64_t k = 0; k < nsteps; ++k) {
       SPHG_TRY(enqueue_step(s, st));
@@ -1500,6 +1493,7 @@ sphg_status sphg_profile_step(sphg_sim* s, float* ms, void* stream) {
   if (!s || !ms || !s->preloop_done) return fail(SPHG_INVALID_ARG, "no computed state or null output");
   cudaStream_t st = (cudaStream_t)stream;
   cudaEvent_t ev[6];
+  SPHG_TRY(current_dt(s, st));
   for (int i = 0; i < 6; ++i) SPHG_CUDA(cudaEventCreate(&ev[i]));
   sphg_status res = enqueue_step(s, st, false, ev);
   if (res == SPHG_OK) {

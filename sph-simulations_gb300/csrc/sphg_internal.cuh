@@ -104,27 +104,14 @@ struct sphg_sim {
   bool cond_graph = true;       // full sort under a conditional graph node (when the merge is on)
   cudaGraphExec_t gexec = nullptr;
   cudaGraphExec_t gexec_hdr = nullptr;  // the same followed by the step header into hslot
-  // the graphs they were made from, [1] with the header, and their force pass's
-  // node (null: not step_force), whose argument holds the time step; stale: the
-  // time step changed since
-  cudaGraph_t graph[2] = {nullptr, nullptr};
-  cudaGraphNode_t force_node[2] = {nullptr, nullptr};
-  bool dt_stale[2] = {false, false};
-  void keep_graph(bool header, cudaGraph_t g, cudaGraphNode_t force) {
-    graph[header] = g;
-    force_node[header] = tile_bits ? nullptr : force;
-    dt_stale[header] = false;
-  }
+  // one instance: the time step as the kernels of the graphs read it (a device
+  // word), and whether it has changed since it was written there
+  float* dt_word = nullptr;
+  bool dt_stale = true;
   void drop_graphs() {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (gexec_hdr) cudaGraphExecDestroy(gexec_hdr);
     gexec = gexec_hdr = nullptr;
-    for (int k = 0; k < 2; ++k) {
-      if (graph[k]) cudaGraphDestroy(graph[k]);
-      graph[k] = nullptr;
-      force_node[k] = nullptr;
-      dt_stale[k] = false;
-    }
   }
 
   StepArgs args() const {
@@ -172,7 +159,12 @@ struct sphg_sim {
     a.csr_overflow = flags + 8;
     a.keyS = keyTmp;
     a.merged = movers_on ? flags + 3 : nullptr;
-    if (movers_on) a.movers = mrec;
+    a.dt = ninst == 1 && !force_batched ? dt_word : nullptr;
+    if (movers_on) {
+      a.movers = mrec;
+      a.movers.last = flags + 4;
+      a.movers.record_limit = (uint32_t)sphg::record_limit(n);
+    }
     return a;
   }
 };

@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(kListThreads) lists_assemble(StepArgs a, ListA
   __shared__ unsigned long long s_before;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   cudaGridDependencySynchronize();
+  if (skip_pass(a)) return;
   // blocks in the order they start: a look-back only waits on blocks that started earlier
   if (tid == 0) s_blk = atomicAdd(o.ctl, 1u);
   const unsigned long long gen = (unsigned long long)(*(volatile uint32_t*)(o.ctl + 1) & 0xfffffu) << kGenShift;

@@ -34,6 +34,8 @@ struct MoverRecord {
   uint32_t* counts;   // the two copies
   uint32_t* next_epoch;  // step epoch of the next iteration's cell ranges
   int64_t cap;        // particles a copy is laid out for
+  const uint32_t* last;  // movers of the iteration before, and how many at most
+  uint32_t record_limit; // for this one's to be recorded (record_limit())
 };
 
 // The parts of one copy, sized for cap particles.
@@ -62,13 +64,19 @@ __host__ __device__ inline MoverCounts mover_counts(const MoverRecord& r, uint32
   return m;
 }
 
-// Movers up to which an iteration merges: a quarter of the particles (at least
-// 8,192).  Measured, merge against full sort, us an iteration of random free
-// particles: 2,000,000 particles 321 against 406 with 2 % moving, 356 with 14 %,
-// 404 with 28 %, 471 with 44 %; 423,000 particles 93 against 124 with 2 %, 108
-// with 28 %, 120 with 44 %, 137 with 64 %; 20,000 particles 45 against 55 with
-// 2 %, 53 with 44 %.
-inline int64_t mover_limit(int64_t n) { return n / 4 > 8192 ? n / 4 : 8192; }
+// Movers up to which an iteration merges, its record being there: small states a
+// quarter (at least 8,192), larger ones any number -- us an iteration of random
+// free particles, merge / full sort after the record: 423,000 particles 94 / 144
+// with 28 % moving, 124 / 168 with 64 %; 2,000,000 382 / 494 and 533 / 631.
+inline int64_t mover_limit(int64_t n) {
+  if (n > 65536) return n;
+  return n / 4 > 8192 ? n / 4 : 8192;
+}
+// Movers of an iteration beyond which the next one's are counted but not
+// recorded, and sorted fully: the record's atomics then cost more than the sort
+// (2,000,000 particles: merge 298 us with 2 % moving, 335 with 14 %, 382 with 28 %,
+// 447 with 44 %; full sort without a record 372).
+inline int64_t record_limit(int64_t n) { return n > 65536 ? n / 3 : mover_limit(n); }
 
 struct MoverArgs {
   int64_t n;

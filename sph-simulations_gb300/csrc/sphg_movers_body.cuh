@@ -50,6 +50,10 @@ __device__ __forceinline__ void record_movers(const StepArgs& a, uint32_t i, uin
   const bool mine = (moved >> lane) & 1u;
   if (lane == __ffs(moved) - 1)
     atomicAdd(r.total + ((i >> 5) % kMoverCounters) * kMoverCounterStride, (uint32_t)__popc(moved));
+  if (*a.movers.last > a.movers.record_limit) {  // many moved the last time: sort fully
+    if (lane == 0) r.total[1] = 1u;
+    return;
+  }
   // insertion point: the new cell's range when it holds particles now (the slot
   // itself is not among them), else a warp-wide 32-way search of the keys
   uint32_t p = 0;

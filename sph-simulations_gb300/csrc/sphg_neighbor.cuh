@@ -14,6 +14,11 @@
 
 namespace sphg {
 
+// The passes of a graph's iteration skip themselves when its merge left the
+// iteration to the full sort, whose branch runs them (every thread of a kernel
+// sees the same word).
+__device__ __forceinline__ bool skip_pass(const StepArgs& a) { return a.go && *a.go == 0u; }
+
 // How the device code of an iteration is launched: a kernel per phase, one
 // cooperative launch per iteration (step_fused), or many iterations in one
 // cluster (step_resident).
@@ -316,7 +321,7 @@ template <int PREC>
 __device__ __forceinline__ uint32_t integrate_and_key(const StepArgs& a, const InstDesc& d, int64_t i,
                                                   int cx, int cy, float2 pi, float4 vi, float ax,
                                                   float ay) {
-  const float dt = d.dt;
+  const float dt = a.dt ? *a.dt : d.dt;
   const float2 v = fma2(make_float2(dt, dt), make_float2(ax, ay), make_float2(vi.x, vi.y));
   const float2 xy = fma2(make_float2(dt, dt), v, pi);
   float vx = v.x, vy = v.y;

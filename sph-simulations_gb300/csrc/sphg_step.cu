@@ -384,8 +384,9 @@ constexpr int density_blocks(int prec, bool batched, int t) { return prec == 1 &
 template <int PREC, bool BATCHED, bool CSR, int T = kThreads>
 __global__ void __launch_bounds__(T, density_blocks(PREC, BATCHED, T)) step_density(StepArgs a) {
   __shared__ QueuedCell<PREC> s_cells[CSR ? 1 : kQueuedCells][T];
-  cudaGridDependencySynchronize();  // the sorted state and cell ranges of the reorder
+  cudaGridDependencySynchronize();  // the sorted state and cell ranges of the re-sort
   allow_next_kernel(a.early_next);
+  if (skip_pass(a)) return;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   density_particle<PREC, BATCHED, CSR, T, kKernels>(a, i, s_cells);
@@ -464,8 +465,9 @@ __device__ __forceinline__ void density_epilogue(const StepArgs& a, const InstDe
 template <int PREC, bool BATCHED, int T = kThreads>
 __global__ void __launch_bounds__(T) step_density_pairs(StepArgs a) {
   constexpr int kPairSlots = 2 * T;
-  cudaGridDependencySynchronize();  // the sorted state and cell ranges of the reorder
+  cudaGridDependencySynchronize();  // the sorted state and cell ranges of the re-sort
   allow_next_kernel(a.early_next);
+  if (skip_pass(a)) return;
   __shared__ uint32_t s_key[kPairSlots];
   __shared__ uint16_t s_chunk[kPairSlots];  // offset of each pair's (or odd particle's) first slot | partner << 15
   __shared__ uint32_t s_wmax[T / 32], s_wcnt[T / 32];
@@ -693,6 +695,7 @@ __global__ void __launch_bounds__(T, force_threads_per_sm(PREC, BATCHED) / T) st
   __syncthreads();
   cudaGridDependencySynchronize();  // densities, pressures and neighbour lists of the density pass
   allow_next_kernel(a.early_next);
+  if (skip_pass(a)) return;
   force_slot<PREC, BATCHED, MODE, CSR, kKernels>(a, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, unit);
 }
 
@@ -1130,6 +1133,10 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocks) step_diag(StepArgs 
     chunk = (int)(t & 4095u);
   }
   const InstDesc& d = (a.ninst == 1) ? a.d0 : a.desc[inst];
+  if (SLOT && skip_pass(a)) {
+    cudaGridDependencySynchronize();
+    return;
+  }
   const int64_t cnt = d.end - d.begin;
   const int ck = a.diag_tab ? diag_instance_chunks(cnt, chunks) : chunks;
   const int64_t per = (cnt + ck - 1) / ck;

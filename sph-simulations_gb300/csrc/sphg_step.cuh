@@ -51,6 +51,8 @@ struct StepArgs {
   int64_t csr_cap;             // entries csr_idx holds (the passes read no further)
   uint32_t* csr_overflow;      // set by the fill when the lists exceed csr_cap
   const uint32_t* merged;      // non-null and set: this iteration's merge sorted the state (the reorder returns)
+  const uint32_t* go;          // non-null and zero: the passes return at once (a full sort's own passes run instead)
+  const float* dt;             // non-null: the time step (one instance, kernels of a graph); else the descriptor's
   MoverRecord movers;          // the force pass's record for the next merge (mask null: off)
   uint32_t* flags;             // [0] unused, [1] number of non-empty tiles this step
   // cell tiles (Morton order only; tile_bits == 0 disables them)
