@@ -170,14 +170,6 @@ __device__ __forceinline__ void entry_vec(const InstDesc& d, float2 pi, float2 p
   }
 }
 
-#ifndef SPHG_DENSITY_TRIM
-#define SPHG_DENSITY_TRIM 1
-#endif
-// 1: the split walk skips the particle itself by splitting its own cell, the
-// prefetch past the last candidate reads the padding entry of the positions,
-// and the record is unconditional (the step's density pass always records)
-constexpr bool kDensityTrim = SPHG_DENSITY_TRIM != 0;
-
 
 // A queued stencil cell: {j0 << 5 | tag, j1 << 5 | tag} and, in split precision,
 // the shift of its offsets.  Plain positions need no shift: half the shared
@@ -257,6 +249,7 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, Q
 #pragma unroll
       for (int k = 0; k < 9; ++k) r[k] = ((valid >> k) & 1u) ? ld_state<LAUNCH>(a.ranges + c[k]) : make_uint4(0, 0, 0, 0);
       int nseg = 0;
+      uint32_t left = 0;  // candidates
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
         if (r[k].z == ep && r[k].y > r[k].x) {
@@ -264,7 +257,9 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, Q
           const uint32_t tag = (uint32_t)k | ((PREC == 0 && ((wrapmask >> k) & 1u)) ? 16u : 0u);
           const float shx = (PREC == 1) ? (c1 == 0 ? 0.f : (c1 > 0 ? d.cs_x : -d.cs_x)) : 0.f;
           const float shy = (PREC == 1) ? (c2 == 0 ? 0.f : (c2 > 0 ? d.cs_y : -d.cs_y)) : 0.f;
-          if (kDensityTrim && PREC == 1 && k == 4) {
+          left += r[k].y - r[k].x;
+          if (PREC == 1 && k == 4) {
+            --left;
             // own cell without the particle itself (its term W(0) = 1 is added
             // first): [start, i) and (i, end), whichever are not empty
             const uint32_t self = (uint32_t)i;
@@ -277,12 +272,12 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, Q
       }
       const float2* pos = a.posA;
       const float h2_lo = d.h2_lo, h2_hi = d.h2_hi;
-      const bool record = nbr != nullptr;
       const uint32_t self = (uint32_t)i;
-      uint32_t* rp = record ? nbr + i : nullptr;  // next record slot: nbr[cnt * n + i]
+      const uint32_t pitch = (uint32_t)n * (uint32_t)sizeof(uint32_t);  // (below 2^27 particles)
+      char* rec0 = reinterpret_cast<char*>(nbr + i);  // record c: nbr[c * n + i]
       bool border = false;
       if (PREC == 1) S.add(1.0f);  // own term W(0) first (plain sums keep the walk's order)
-      if (nseg > 0) {  // plain: always (the particle's own cell holds it); split: any other particle near
+      if (left > 0) {  // plain: always (the particle's own cell holds it); split: any other particle near
         QueuedCell<PREC> w = s_cells[0][tid];
         int q = 1;
         uint32_t jj = w.x, je = w.y;
@@ -291,22 +286,14 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, Q
         while (true) {
           uint32_t jn = jj + 32u, jen = je;
           float2 shn = sh;
-          bool more = true;
-          if (jn == je) {
-            if (q == nseg) {
-              more = false;
-            } else {
-              w = s_cells[q][tid];
-              ++q;
-              jn = w.x;
-              jen = w.y;
-              shn = cell_shift<PREC>(w);
-            }
+          if (jn == je) {  // the next cell (after the last candidate the last one again: not used)
+            w = s_cells[min(q, nseg - 1)][tid];
+            ++q;
+            jn = w.x;
+            jen = w.y;
+            shn = cell_shift<PREC>(w);
           }
-          // one candidate ahead (past the last one: the end of its cell, at most
-          // slot n -- the positions hold one entry more)
-          const float2 pn = ld_state<LAUNCH>(pos + ((kDensityTrim || more ? jn : jj) >> 5));
-          const uint32_t j = jj >> 5;
+          const float2 pn = ld_state<LAUNCH>(pos + (jn >> 5));  // one candidate ahead
           const float2 dxy = PREC == 1 ? sub2(sub2(pi, pj), sh) : sub2(pi, pj);
           float dx = dxy.x, dy = dxy.y;
           float r2;
@@ -319,17 +306,14 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, Q
             in = r2 < h2_lo;
             border |= !in && r2 <= h2_hi;
           }
-          // split: the walk never meets the particle itself; the step always records
-          const bool other = (kDensityTrim && PREC == 1) || j != self;
           const float t = fmaf(-r2, inv_h2, 1.0f);
-          S.add_fast((PREC == 1 ? in && other : in) ? t * t * t : 0.0f);
-          const bool rec = in && other && (kDensityTrim || record);
-          if (rec && cnt < slots) {
-            st_out<LAUNCH>(rp, jj);
-            rp += n;
-          }
+          S.add_fast(in ? t * t * t : 0.0f);
+          // split: the walk never meets the particle itself
+          const bool rec = in && (PREC == 1 || (jj >> 5) != self);
+          if (rec && cnt < slots)
+            st_out<LAUNCH>(reinterpret_cast<uint32_t*>(rec0 + (uint64_t)cnt * pitch), jj);
           cnt += rec ? 1u : 0u;
-          if (!more) break;
+          if (--left == 0) break;
           jj = jn;
           je = jen;
           sh = shn;
