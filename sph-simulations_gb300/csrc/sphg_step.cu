@@ -195,10 +195,10 @@ __device__ __forceinline__ float2 cell_shift(const QueuedCell<PREC>& w) {
 // column per thread.
 template <int PREC, bool BATCHED, bool CSR, int T, int LAUNCH>
 __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, QueuedCell<PREC> (*s_cells)[T]) {
-  typename std::conditional<BATCHED, const InstDesc&, const InstDesc>::type d = inst_ref<BATCHED>(a, i);
-  if (BATCHED && !d.active) return;  // a finished served instance
   const uint32_t key = a.keyA[i];
   const float2 pi = a.posA[i];
+  typename std::conditional<BATCHED, const InstDesc&, const InstDesc>::type d = inst_ref<BATCHED>(a, i);
+  if (BATCHED && !d.active) return;  // a finished served instance
   typename std::conditional<PREC == 1, CSum, PSum>::type S;
   int cx, cy;
   const float inv_h2 = d.inv_h2;
@@ -644,8 +644,19 @@ constexpr int kForceBatch = SPHG_FORCE_BATCH;  // recorded neighbours gathered t
 constexpr bool kSkipZeroViscosity = SPHG_SKIP_ZERO_VISCOSITY != 0;
 
 
+// A particle as the force pass reads it: key, position, (v, P, 1/rho), number of
+// recorded neighbours and the first batch of them (entries past the number are
+// whatever is there).
+struct ForceIn {
+  uint32_t key;
+  float2 pi;
+  float4 vi;
+  uint32_t cnt;
+  uint32_t first[kForceBatch];
+};
+
 template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
-__device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit);
+__device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit, const ForceIn& in);
 
 // Threads per SM the force pass is compiled for.  Split precision: 1,152
 // (nine 128-thread blocks, 56 registers) for one instance and 1,024 (eight
@@ -687,15 +698,33 @@ __global__ void __launch_bounds__(T, force_threads_per_sm(PREC, BATCHED) / T) st
 // forces and, in integrate mode, the update, the new key and the mover record.
 template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ void force_slot(const StepArgs& a, int64_t i, const float2* unit) {
+  // everything of the particle that needs no other load first: the instance
+  // lookup and the neighbours' gathers wait for loads of their own
+  ForceIn in = {};
+  if (i < a.n) {
+    in.key = a.keyA[i];
+    in.pi = a.posA[i];
+    in.vi = a.velpA[i];
+    if (!CSR) {
+      in.cnt = 0xffffffffu;
+      if (a.nbr) {
+        in.cnt = a.ncount[i];
+#pragma unroll
+        for (int u = 0; u < kForceBatch; ++u) in.first[u] = ld_state<LAUNCH>(a.nbr + u * (size_t)a.n + i);
+      }
+    }
+  }
   // slots of a finished served instance are skipped (no pair, no integration, no mover bit)
   const bool valid = i < a.n && (!BATCHED || inst_ref<BATCHED>(a, i).active);
   const bool track = MODE == kForceIntegrate && a.movers.mask != nullptr;
   uint32_t key = 0;
-  if (valid) key = force_one<PREC, BATCHED, MODE, CSR, LAUNCH>(a, i, unit);
+  if (valid) key = force_one<PREC, BATCHED, MODE, CSR, LAUNCH>(a, i, unit, in);
   if (track) {
     // slots whose cell key changed, for the incremental re-sort: one bit per
     // slot (a warp holds 32 consecutive slots) and the record of each
-    const unsigned moved = __ballot_sync(0xffffffffu, valid && key != a.keyA[i]);
+    // (one instance, split: read again, the register counts)
+    const bool reread = PREC == 1 && !BATCHED;
+    const unsigned moved = __ballot_sync(0xffffffffu, valid && key != (reread ? a.keyA[i] : in.key));
     if ((threadIdx.x & 31) == 0 && i < a.n) a.movers.mask[i >> 5] = moved;  // every word, skipped slots included
     if (i == 0) *a.movers.next_epoch = *a.epoch + 1u;
     if (moved) record_movers(a, (uint32_t)i, key, moved);
@@ -705,12 +734,12 @@ __device__ __forceinline__ void force_slot(const StepArgs& a, int64_t i, const f
 // Forces on particle i; in integrate mode also the update and the new key
 // (returned), in force-only mode the acceleration is stored.
 template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
-__device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit) {
+__device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit, const ForceIn& in) {
   // one instance: a copy of the kernel-argument descriptor; batched: a reference
   typename std::conditional<BATCHED, const InstDesc&, const InstDesc>::type d = inst_ref<BATCHED>(a, i);
-  const uint32_t key = a.keyA[i];
-  const float2 pi = a.posA[i];
-  const float4 vi = a.velpA[i];
+  const uint32_t key = in.key;
+  const float2 pi = in.pi;
+  const float4 vi = in.vi;
   // one (compensated) sum per axis of every pair's pressure + viscosity (+ alpha)
   // term, both axes in paired instructions
   typename std::conditional<PREC == 1, CSum2, PSum2>::type f;
@@ -749,7 +778,7 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
   };
   auto pair = [&](uint32_t j, float dx, float dy) { pair_v(ld_state<LAUNCH>(velp + j), dx, dy); };
   int cx, cy;
-  const uint32_t cnt = CSR ? 0u : (a.nbr ? a.ncount[i] : 0xffffffffu);
+  const uint32_t cnt = in.cnt;
   if constexpr (CSR) {
     // MPListsForceComputation::ComputeForces: the list in its order (self skipped:
     // its pressure term is excluded by r > TOL and its viscosity term is zero)
@@ -775,13 +804,15 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
     // whatever the batching.
     const uint32_t wmax = __reduce_max_sync(__activemask(), cnt);
     const uint32_t self_e = ((uint32_t)i << 5) | 4u;
-    auto batch = [&](auto width, uint32_t q) {
+    auto load = [&](auto width, uint32_t q, uint32_t* e) {
       constexpr int B = decltype(width)::value;
-      uint32_t e[B];
-      float2 pj[B];
-      float4 vj[B];
 #pragma unroll
       for (int u = 0; u < B; ++u) e[u] = q + u < cnt ? ld_state<LAUNCH>(a.nbr + (q + u) * n + i) : self_e;
+    };
+    auto batch = [&](auto width, const uint32_t* e) {
+      constexpr int B = decltype(width)::value;
+      float2 pj[B];
+      float4 vj[B];
 #pragma unroll
       for (int u = 0; u < B; ++u) {
         pj[u] = ld_state<LAUNCH>(a.posA + (e[u] >> 5));
@@ -801,17 +832,30 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
         pair_v(vj[u], dx, dy);
       }
     };
-#if SPHG_FORCE_TAIL
     uint32_t q = 0;
-    for (; q + kForceBatch <= wmax; q += kForceBatch) batch(std::integral_constant<int, kForceBatch>(), q);
+    if (wmax >= 3) {
+      uint32_t e[kForceBatch];
+#pragma unroll
+      for (int u = 0; u < kForceBatch; ++u) e[u] = (uint32_t)u < cnt ? in.first[u] : self_e;
+      batch(std::integral_constant<int, kForceBatch>(), e);
+      q = kForceBatch;
+    }
+    for (; q + kForceBatch <= wmax; q += kForceBatch) {
+      uint32_t e[kForceBatch];
+      load(std::integral_constant<int, kForceBatch>(), q, e);
+      batch(std::integral_constant<int, kForceBatch>(), e);
+    }
     if (q + 2 <= wmax) {
-      batch(std::integral_constant<int, 2>(), q);
+      uint32_t e[2];
+      load(std::integral_constant<int, 2>(), q, e);
+      batch(std::integral_constant<int, 2>(), e);
       q += 2;
     }
-    if (q < wmax) batch(std::integral_constant<int, 1>(), q);
-#else
-    for (uint32_t q = 0; q < wmax; q += kForceBatch) batch(std::integral_constant<int, kForceBatch>(), q);
-#endif
+    if (q < wmax) {
+      uint32_t e[1];
+      load(std::integral_constant<int, 1>(), q, e);
+      batch(std::integral_constant<int, 1>(), e);
+    }
   } else {
     // more neighbours than the density pass could record (or no record): the
     // stencil walk, pairs in the walk's order
