@@ -14,11 +14,14 @@
 
 namespace sphg {
 
+// Threads of a merge block: four slots each in the kernel of its own, whose many
+// blocks hide each other's latency; one each in the resident kernel, where a block
+// has an SM's schedulers to itself and is as long as its instructions (1,023
+// iteration: 1,023 particles 11.7 -> 10.95, 6,084 28.1 -> 25.5, 12,800 16.6 -> 16.2).
 constexpr int kMergeThreads = 128;
-constexpr int kMergeSlots = kMergeBlockSlots / kMergeThreads;  // slots per thread
-constexpr int kMergeWords = kMergeBlockSlots / 32;             // mask words per block
-constexpr int kMergeWarps = kMergeThreads / 32;
-static_assert(kMergeWords <= 32 && kMergeWarps >= 4, "one warp scans the words; warps 2 and 3 find the neighbours");
+constexpr int kResidentMergeThreads = 512;
+constexpr int kMergeWords = kMergeBlockSlots / 32;  // mask words per block
+static_assert(kMergeWords <= 32, "a warp scans the words");
 
 // ---------------------------------------------------------------- the record
 // Clears slot i's part of the copy the next force pass adds to (the reorder
@@ -174,17 +177,17 @@ __device__ __forceinline__ void merge_store(V* p, V v) {
 
 // The barrier of a merge block's threads: a thread block, or one of several in
 // the resident kernel's blocks.
-template <int LAUNCH>
+template <int LAUNCH, int THREADS>
 __device__ __forceinline__ void merge_sync() {
   if constexpr (LAUNCH == kResident)
-    asm volatile("barrier.sync %0, %1;" ::"r"(1u + threadIdx.x / kMergeThreads), "n"(kMergeThreads) : "memory");
+    asm volatile("barrier.sync %0, %1;" ::"r"(1u + threadIdx.x / THREADS), "n"(THREADS) : "memory");
   else __syncthreads();
 }
 
 struct MergeShared {
   uint32_t stay[kMergeWords];            // bit per slot: it keeps its cell
   uint32_t tot[kMergeWords];             // stayers + insertions of the word | insertions << 16
-  int32_t red[kMergeWarps];
+  int32_t red[kResidentMergeThreads / 32];
   bool merge;
   uint32_t prev, next;                   // keys either side of the block's output
   uint32_t ikey[kBlockInsertCap], islot[kBlockInsertCap];
@@ -201,17 +204,19 @@ struct MergeShared {
 // Every thread of the block calls it; epoch: *rec.next_epoch.  What bounds it is latency -- a block
 // goes from its loads through two or four barriers to its stores -- so every
 // load that needs no other is issued at the top, before the decision is known.
-template <int LAUNCH>
+template <int LAUNCH, int THREADS = kMergeThreads>
 __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh, int64_t blk, uint32_t epoch) {
-  const int tid = threadIdx.x & (kMergeThreads - 1), lane = tid & 31, warp = tid >> 5;
+  constexpr int kSlots = kMergeBlockSlots / THREADS, kWarps = THREADS / 32;  // slots per thread
+  static_assert(kWarps >= 4, "warp 1 decides, warps 2 and 3 find the neighbours");
+  const int tid = threadIdx.x & (THREADS - 1), lane = tid & 31, warp = tid >> 5;
   const int64_t base = blk << kMergeShift;
   const unsigned lt = (1u << lane) - 1u;
-  uint32_t key[kMergeSlots], mw[kMergeSlots];
-  float2 p[kMergeSlots], v[kMergeSlots];
-  int32_t id[kMergeSlots];
+  uint32_t key[kSlots], mw[kSlots];
+  float2 p[kSlots], v[kSlots];
+  int32_t id[kSlots];
 #pragma unroll
-  for (int u = 0; u < kMergeSlots; ++u) {
-    const int64_t i = base + (u * kMergeWarps + warp) * 32 + lane;
+  for (int u = 0; u < kSlots; ++u) {
+    const int64_t i = base + (u * kWarps + warp) * 32 + lane;
     const bool in = i < a.n;
     mw[u] = in ? a.rec.mask[i >> 5] : ~0u;
     key[u] = in ? a.keyB[i] : 0u;
@@ -221,7 +226,7 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
   }
   // the slots either side of the block, which nearly always decide its neighbours' keys
   const int64_t side = warp == 2 ? base - 1 : base + kMergeBlockSlots;
-  const bool has_side = warp >= 2 && side >= 0 && side < a.n;
+  const bool has_side = (warp == 2 || warp == 3) && side >= 0 && side < a.n;
   const uint32_t side_mask = has_side ? a.rec.mask[side >> 5] : 0u;
   const uint32_t side_key = has_side ? a.keyB[side] : 0u;
   const MoverCounts r = mover_counts(a.rec, epoch);
@@ -233,17 +238,17 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
       if (blk == 0) merge_decided(a, merge, movers, epoch);
     }
   }
-  uint32_t c[kMergeSlots], cex[kMergeSlots];
+  uint32_t c[kSlots], cex[kSlots];
 #pragma unroll
-  for (int u = 0; u < kMergeSlots; ++u) {
-    const int64_t i = base + (u * kMergeWarps + warp) * 32 + lane;
+  for (int u = 0; u < kSlots; ++u) {
+    const int64_t i = base + (u * kWarps + warp) * 32 + lane;
     c[u] = i <= a.n ? merge_inserted(r.insc, i) : 0u;
   }
   const uint32_t side_ins = has_side ? merge_inserted(r.insc, side) : 0u;
   // slots before the block whose movers left, movers inserted before it
   int32_t d = 0;
   const int64_t sup = blk >> kMergeSupShift, b0 = sup << kMergeSupShift;
-  for (int64_t q = tid; q < sup; q += kMergeThreads) d += r.sup_net[q];
+  for (int64_t q = tid; q < sup; q += THREADS) d += r.sup_net[q];
   if (tid < blk - b0) d += r.blk_net[b0 + tid];
   if (warp == 2) {
     uint32_t k = kNoIndex;
@@ -257,10 +262,10 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
     if (!has_side || side_ins || ((side_mask >> (side & 31)) & 1u)) k = merge_next_key(a, r.insc, side, lane);
     if (lane == 0) sh.next = k;
   }
-  bool stay[kMergeSlots];
+  bool stay[kSlots];
 #pragma unroll
-  for (int u = 0; u < kMergeSlots; ++u) {
-    const int w = u * kMergeWarps + warp;
+  for (int u = 0; u < kSlots; ++u) {
+    const int w = u * kWarps + warp;
     stay[u] = !((mw[u] >> lane) & 1u);
     const unsigned sb = __ballot_sync(0xffffffffu, stay[u]);
     uint32_t incl = c[u];
@@ -279,11 +284,11 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
   }
   d = __reduce_add_sync(0xffffffffu, d);
   if (lane == 0) sh.red[warp] = d;
-  merge_sync<LAUNCH>();
+  merge_sync<LAUNCH, THREADS>();
   if (!sh.merge) return false;
   {  // the other copy, which this iteration's force pass adds to
     const MoverCounts o = mover_counts(a.rec, epoch + 1u);
-    if (base + 4 * tid <= a.n) o.insc[(base >> 2) + tid] = 0u;
+    if (tid < kMergeBlockSlots / 4 && base + 4 * tid <= a.n) o.insc[(base >> 2) + tid] = 0u;
     if (tid == 0) {
       o.blk_net[blk] = 0;
       o.blk_ins[blk] = 0u;
@@ -307,17 +312,17 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
   }
   int64_t out0 = base;
 #pragma unroll
-  for (int w = 0; w < kMergeWarps; ++w) out0 += sh.red[w];
+  for (int w = 0; w < kWarps; ++w) out0 += sh.red[w];
   const uint32_t total = all & 0xffffu, nins = all >> 16;
   // a consistent record stays inside the buffers; anything else is reported, not written
   if (out0 < 0 || out0 + (int64_t)total > a.n || nins > (uint32_t)kBlockInsertCap) {
     if (tid == 0) a.ctl[2] = 1u;
-    merge_sync<LAUNCH>();
+    merge_sync<LAUNCH, THREADS>();
     return true;
   }
 #pragma unroll
-  for (int u = 0; u < kMergeSlots; ++u) {
-    const int w = u * kMergeWarps + warp;
+  for (int u = 0; u < kSlots; ++u) {
+    const int w = u * kWarps + warp;
     const int64_t i = base + w * 32 + lane;
     const uint32_t woff = __shfl_sync(0xffffffffu, off, w);
     const uint32_t grp = (woff & 0xffffu) + (uint32_t)__popc(sh.stay[w] & lt) + cex[u];
@@ -343,9 +348,9 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
       }
     }
   }
-  merge_sync<LAUNCH>();
+  merge_sync<LAUNCH, THREADS>();
   if (nins) {
-  for (uint32_t q = tid; q < nins; q += kMergeThreads) {
+  for (uint32_t q = tid; q < nins; q += THREADS) {
     const uint32_t k = sh.ikey[q], s = sh.islot[q], g = sh.igrp[q];
     uint32_t rank = 0;  // among its group, by (key, slot)
     for (uint32_t r = g >> 16, e = r + (g & 0xffffu); r < e; ++r)
@@ -363,10 +368,10 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
     merge_store<LAUNCH>(a.perm + to, s);
     if (a.idsA) merge_store<LAUNCH>(a.idsA + to, a.idsB[s]);
   }
-  merge_sync<LAUNCH>();
+  merge_sync<LAUNCH, THREADS>();
   }
   uint32_t* rg = reinterpret_cast<uint32_t*>(a.ranges);
-  for (uint32_t q = tid; q < total; q += kMergeThreads) {
+  for (uint32_t q = tid; q < total; q += THREADS) {
     const uint32_t k = sh.key[q];
     const uint32_t kp = q ? sh.key[q - 1] : sh.prev, kn = q + 1 < total ? sh.key[q + 1] : sh.next;
     const uint32_t i = (uint32_t)(out0 + q);
@@ -377,7 +382,7 @@ __device__ __forceinline__ bool merge_block(const MoverArgs& a, MergeShared& sh,
     }
     if (k != kn) merge_store<LAUNCH>(rg + 4 * (size_t)k + 1, i + 1u);
   }
-  merge_sync<LAUNCH>();  // (a block calling again reuses the shared arrays)
+  merge_sync<LAUNCH, THREADS>();  // (a block calling again reuses the shared arrays)
   return true;
 }
 

@@ -1248,7 +1248,7 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocks) step_diag(StepArgs 
 // cluster's 16,384 threads), 32,400 30.2 / 27.0; one iteration a call 17.1 / 23.4
 // at 1,023, 22.9 / 26.0 at 16,200.
 constexpr int kResidentThreads = 1024;
-constexpr int kResidentGroups = kResidentThreads / kMergeThreads;   // merge blocks at a time
+constexpr int kResidentGroups = kResidentThreads / kResidentMergeThreads;   // merge blocks at a time
 constexpr int kResidentChunks = kResidentThreads / kDiagThreads;    // diagnostics chunks at a time
 constexpr int kResidentIters = 128;  // iterations a launch: launches amortised, about a millisecond at most
 
@@ -1351,13 +1351,13 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   uint32_t epoch = *(volatile const uint32_t*)m.rec.next_epoch;
   for (int it = 0; it < iters; ++it, ++epoch) {
     // the decision is the same for every thread; a merge block takes it beside its loads
-    const uint32_t g = tid / kMergeThreads;
+    const uint32_t g = tid / kResidentMergeThreads;
     uint32_t b = g * C + cta, movers;
     bool merge;
     if (b < nb) {
-      merge = merge_block<kResident>(m, sh.merge[g], b, epoch);
+      merge = merge_block<kResident, kResidentMergeThreads>(m, sh.merge[g], b, epoch);
       for (b += C * kResidentGroups; merge && b < nb; b += C * kResidentGroups)
-        merge_block<kResident>(m, sh.merge[g], b, epoch);
+        merge_block<kResident, kResidentMergeThreads>(m, sh.merge[g], b, epoch);
     } else {
       merge = merge_wanted(m, mover_counts(m.rec, epoch).total, &movers);
     }
