@@ -119,6 +119,9 @@ sphg_status make_desc(const sphg_params& p, int64_t begin, int64_t count, uint64
     d.ny = nr[1];
     span = (uint64_t)d.nx * (uint64_t)d.ny;
   }
+  // cells [1, nr - 3]: their far edge is a cell away from the wall at least
+  d.inner_x = nr[0] > 3 ? morton_host((uint32_t)nr[0] - 3, 0) : 0u;
+  d.inner_y = nr[1] > 3 ? morton_host(0, (uint32_t)nr[1] - 3) : 0u;
   d.cell_base = (uint32_t)cell_base;
   d.key_span = (uint32_t)span;
   d.lo_x = (float)p.lo[0];

@@ -15,9 +15,11 @@
 namespace sphg {
 
 // Threads of a merge block: four slots each in the kernel of its own, whose many
-// blocks hide each other's latency; one each in the resident kernel, where a block
-// has an SM's schedulers to itself and is as long as its instructions (1,023
-// iteration: 1,023 particles 11.7 -> 10.95, 6,084 28.1 -> 25.5, 12,800 16.6 -> 16.2).
+// blocks hide each other's latency (eight warps of two slots: 1M dam break 81.8 ->
+// 83.3 us an iteration, batch of 256 411 -> 420); one each in the resident
+// kernel, where a block has an SM's schedulers to itself and takes as long as its
+// instructions (1,023 particles 11.7 -> 10.95 us, 6,084 28.1 -> 25.5, 12,800 16.6
+// -> 16.2).
 constexpr int kMergeThreads = 128;
 constexpr int kResidentMergeThreads = 512;
 constexpr int kMergeWords = kMergeBlockSlots / 32;  // mask words per block

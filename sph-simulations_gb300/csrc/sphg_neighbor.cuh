@@ -317,6 +317,27 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstD
 // then low) or the periodic wrap, then the cell key of the new position for
 // the next sort (SetParticleCellIds).  Split precision keeps the position as
 // (cell, offset) and renormalises the offset into the new cell.
+// The same for a split particle that stays in its cell clear of the cell's edges,
+// the cell away from the walls -- nearly all of them: nothing of the walls, the
+// new cell or its key is to be computed, nor the cell's coordinates.  false: left
+// to integrate_and_key (which decides in the same way, so the same bits).
+__device__ __forceinline__ bool integrate_in_cell(const StepArgs& a, const InstDesc& d, int64_t i, uint32_t key,
+                                                  float2 pi, float4 vi, float ax, float ay) {
+  const uint32_t code = key - d.cell_base;
+  if (d.order != 0 || (!d.periodic && !((code & 0x55555555u) - 1u < d.inner_x && (code & 0xAAAAAAAAu) - 1u < d.inner_y)))
+    return false;
+  const float dt = a.dt ? *a.dt : d.dt;
+  const float2 v = fma2(make_float2(dt, dt), make_float2(ax, ay), make_float2(vi.x, vi.y));
+  const float2 xy = fma2(make_float2(dt, dt), v, pi);
+  const float qx = xy.x * d.inv_cs_x, qy = xy.y * d.inv_cs_y;  // offset_cells: 0 in the open interval
+  if (!(qx > 1.0e-6f && qx < 1.0f - 1.0e-6f && qy > 1.0e-6f && qy < 1.0f - 1.0e-6f)) return false;
+  a.posB[i] = xy;
+  a.velB[i] = v;
+  a.keyB[i] = key;
+  if (a.track_ids) a.idsB[i] = a.idsA[i];
+  return true;
+}
+
 template <int PREC>
 __device__ __forceinline__ uint32_t integrate_and_key(const StepArgs& a, const InstDesc& d, int64_t i,
                                                   int cx, int cy, float2 pi, float4 vi, float ax,

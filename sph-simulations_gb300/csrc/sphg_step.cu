@@ -782,7 +782,6 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
   if constexpr (CSR) {
     // MPListsForceComputation::ComputeForces: the list in its order (self skipped:
     // its pressure term is excluded by r > TOL and its viscosity term is zero)
-    decode_code(d, key - d.cell_base, cx, cy);
     const int64_t b = min(a.csr_offs[i], a.csr_cap), e = min(a.csr_offs[i + 1], a.csr_cap);
     for (int64_t q = b; q < e; ++q) {
       const uint32_t ent = __ldg(a.csr_idx + q);
@@ -794,7 +793,6 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
     }
   } else if (cnt <= (uint32_t)a.nbr_slots) {  // (not CSR: the lists mode has no record)
     // the density pass recorded this particle's neighbours (stencil order)
-    decode_code(d, key - d.cell_base, cx, cy);
     const size_t n = (size_t)a.n;
     // kForceBatch neighbours at a time, their gathers in flight together.  The
     // lanes of a warp all run the warp's largest count: whole batches, then
@@ -869,6 +867,8 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
     a.acc[i] = make_float2(ax, ay);
     return 0;
   }
+  if (PREC == 1 && LAUNCH != kResident && integrate_in_cell(a, d, i, key, pi, vi, ax, ay)) return key;
+  decode_code(d, key - d.cell_base, cx, cy);
   return integrate_and_key<PREC>(a, d, i, cx, cy, pi, vi, ax, ay);
 }
 

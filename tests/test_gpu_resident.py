@@ -62,3 +62,20 @@ def test_resident_periodic_many_neighbours():
     p, x, y, vx, vy, _ = W.taylor_green(60, seed=2)
     p["h"] = 3.2 / 60
     _both(S, S.params(**p), len(x), (x, y, vx, vy), S.PLAIN, 30)
+
+
+@pytest.mark.parametrize("order", ["morton", "rowmajor"])
+@pytest.mark.parametrize("periodic", [0, 1])
+@pytest.mark.parametrize("cells", [3, 4, 5, 9])
+def test_split_update_in_a_few_cells(cells, periodic, order):
+    """Split positions in grids of a few cells: the kernels update a particle that
+    stays in a cell clear of the walls without the walls' and the key's arithmetic,
+    the resident iteration never does -- the same bits at every wall and edge."""
+    import sphg as S
+    rng = np.random.default_rng(cells + periodic)
+    n, h = 60 * cells, 1.0
+    lo, hi = (-0.25, 0.5), (-0.25 + cells * h - 0.3 * (1 - periodic), 0.5 + cells * h - 0.01 * (1 - periodic))
+    x, y = rng.uniform(lo[0], hi[0], n), rng.uniform(lo[1], hi[1], n)
+    vx, vy = rng.normal(0, 30, (2, n))
+    prm = S.params(order=order, h=h, dt=1e-3, k=1.0, mu=0.01, lo=lo, hi=hi, periodic=periodic)
+    _both(S, prm, n, (x, y, vx, vy), S.SPLIT, 60)
