@@ -546,7 +546,7 @@ sphg_status run_steps(sphg_sim* s, int64_t k, cudaStream_t st, bool first = fals
     SPHG_TRY(enqueue_step(s, st, true));
     --k;
   }
-  if (resident_on(s)) return run_resident(s, k, nullptr, st);
+  if (resident_on(s) && (k != 1 || s->n <= sphg::kResidentSingleMaxN)) return run_resident(s, k, nullptr, st);
   if (s->opt.use_graph) {
     SPHG_TRY(build_graph(s));
     for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(s->gexec, st));
@@ -890,9 +890,9 @@ sphg_status sphg_create_batch(int32_t ninst, const sphg_params* p, const int64_t
       !host_stage(s, (size_t)s->n * (sizeof(float2) * 2 + sizeof(float4) + sizeof(float) + sizeof(uint32_t))))
     st = fail(SPHG_OOM, "pinned host staging");
   // (lists mode: captured after the pre-loop has sized the list buffer)
-  const bool capture_now = s->opt.use_graph && s->opt.compute != SPHG_COMPUTE_LISTS && !resident_on(s);
-  if (st == SPHG_OK && s->n > 0 && capture_now) st = build_graph(s);
-  if (st == SPHG_OK && s->n > 0 && capture_now) st = build_graph(s, true);  // with step headers
+  const bool capture_now = s->opt.use_graph && s->opt.compute != SPHG_COMPUTE_LISTS;
+  if (st == SPHG_OK && s->n > 0 && capture_now && (!resident_on(s) || s->n > sphg::kResidentSingleMaxN)) st = build_graph(s);
+  if (st == SPHG_OK && s->n > 0 && capture_now && !resident_on(s)) st = build_graph(s, true);  // with step headers
   if (st != SPHG_OK) {
     destroy_impl(s);
     return st;

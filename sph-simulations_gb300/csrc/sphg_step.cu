@@ -1246,7 +1246,9 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocks) step_diag(StepArgs 
 // iterations a call): 1,023 particles 12.9 / 23.4, 6,400 14.8 / 25.1, 14,375
 // 18.4 / 25.3, 16,200 18.8 / 25.9, 20,300 25.5 / 25.8 (a second round of the
 // cluster's 16,384 threads), 32,400 30.2 / 27.0; one iteration a call 17.1 / 23.4
-// at 1,023, 22.9 / 26.0 at 16,200.
+// at 1,023, 22.9 / 26.0 at 16,200.  (Later: 1,023 11.5 / 17.6, 6,400 13.1 / 18.8,
+// 16,129 17.7 / 19.6; one a call 15.3 / 17.6, 17.2 / 18.7 and 21.6 / 19.6, so calls
+// of one iteration above kResidentSingleMaxN use the graph.)
 constexpr int kResidentThreads = 1024;
 constexpr int kResidentGroups = kResidentThreads / kResidentMergeThreads;   // merge blocks at a time
 constexpr int kResidentChunks = kResidentThreads / kDiagThreads;    // diagnostics chunks at a time
@@ -1372,25 +1374,25 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     for (uint32_t i = i0 + tid; i < i1; i += kResidentThreads)
       density_particle<PREC, false, false, kResidentThreads, kResident>(a, i, sh.cells);
     cluster_barrier();
-    if (headers) {  // step_diag's chunks, kDiagThreads threads each
-      const uint32_t dper = (n + ck - 1) / ck;
-      for (uint32_t c0 = cta * kResidentChunks; c0 < (uint32_t)ck; c0 += C * kResidentChunks) {
-        const uint32_t c = c0 + tid / kDiagThreads, b = dper * c, e = min(n, b + dper);
+    if (headers) {  // step_diag's chunks, kDiagThreads threads each: the last threads of every block first, which
+                    // have the fewest particles in the force phase beside it
+      const uint32_t dper = (n + ck - 1) / ck, g = kResidentChunks - 1u - tid / kDiagThreads;
+      for (uint32_t c = g * C + cta; c < (uint32_t)ck; c += C * kResidentChunks) {
+        const uint32_t b = dper * c, e = min(n, b + dper);
         DiagPart v = {};
-        if (c < (uint32_t)ck)
-          for (uint32_t i = b + tid % kDiagThreads; i < e; i += kDiagThreads) {
-            const float4 vp = a.velpA[i];
-            diag_particle<PREC>(v, a.d0, dc, make_float2(vp.x, vp.y), a.posA[i], a.rho[i], PREC == 1 ? a.keyA[i] : 0u);
-          }
+        for (uint32_t i = b + tid % kDiagThreads; i < e; i += kDiagThreads) {
+          const float4 vp = a.velpA[i];
+          diag_particle<PREC>(v, a.d0, dc, make_float2(vp.x, vp.y), a.posA[i], a.rho[i], PREC == 1 ? a.keyA[i] : 0u);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) part_add(v, part_shfl_down(v, o));
         if (lane == 0) sh.warps[tid >> 5] = v;
-        __syncthreads();
-        if (tid % kDiagThreads == 0 && c < (uint32_t)ck) {
+        asm volatile("barrier.sync %0, %1;" ::"r"(8u + g), "n"(kDiagThreads) : "memory");
+        if (tid % kDiagThreads == 0) {
           for (int k = 1; k < kDiagThreads / 32; ++k) part_add(v, sh.warps[(tid >> 5) + k]);
           parts[c] = v;
         }
-        __syncthreads();
+        asm volatile("barrier.sync %0, %1;" ::"r"(8u + g), "n"(kDiagThreads) : "memory");
       }
     }
     for (uint32_t b = i0 + (tid & ~31u); b < i1; b += kResidentThreads)

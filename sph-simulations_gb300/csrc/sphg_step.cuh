@@ -78,6 +78,7 @@ int fused_blocks(const StepArgs& a, int precision);
 // Particles up to which a single instance's iterations run in one cluster
 // (step_resident): measured against the graph of kernels in sphg_step.cu.
 constexpr int64_t kResidentMaxN = 16384;
+constexpr int64_t kResidentSingleMaxN = 12000;  // in calls of one iteration without a header
 // Blocks of that cluster (0: not available here), and `iters` iterations of the
 // current state; headers (device-accessible, 6 doubles per iteration) or null,
 // with the diagnostics partials and chunk count of launch_diagnostics.
