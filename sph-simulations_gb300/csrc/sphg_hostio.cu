@@ -37,14 +37,19 @@ __device__ __forceinline__ void report_errors(const HostErrors& e) {
 }
 
 // An FP64 position as its cell (clamped to [0, cmax]) and FP32 offset in it.
+// FUSED: c cs taken off x - lo with one rounding, as the host code that stages a
+// served request rounds it where its compiler contracts (Arm does); an upload has
+// always rounded the product first.
+template <bool FUSED>
 __device__ __forceinline__ float2 split_position(const InstDesc& d, double x, double y, int cmx, int cmy, int& cx,
                                                  int& cy) {
   const double qx = floor_div(__dsub_rn(x, d.lo_xd), d.cs_xd, d.inv_cs_xd);
   const double qy = floor_div(__dsub_rn(y, d.lo_yd), d.cs_yd, d.inv_cs_yd);
   cx = !(qx < (double)cmx) ? cmx : (qx < 0.0 ? 0 : (int)qx);
   cy = !(qy < (double)cmy) ? cmy : (qy < 0.0 ? 0 : (int)qy);
-  float fx = __double2float_rn(__dsub_rn(__dsub_rn(x, d.lo_xd), __dmul_rn((double)cx, d.cs_xd)));
-  float fy = __double2float_rn(__dsub_rn(__dsub_rn(y, d.lo_yd), __dmul_rn((double)cy, d.cs_yd)));
+  const double tx = __dsub_rn(x, d.lo_xd), ty = __dsub_rn(y, d.lo_yd);
+  float fx = __double2float_rn(FUSED ? __fma_rn(-(double)cx, d.cs_xd, tx) : __dsub_rn(tx, __dmul_rn((double)cx, d.cs_xd)));
+  float fy = __double2float_rn(FUSED ? __fma_rn(-(double)cy, d.cs_yd, ty) : __dsub_rn(ty, __dmul_rn((double)cy, d.cs_yd)));
   if ((double)fx >= d.cs_xd) fx = nextafterf(fx, 0.0f);
   if ((double)fy >= d.cs_yd) fy = nextafterf(fy, 0.0f);
   return make_float2(fx, fy);
@@ -61,7 +66,7 @@ __device__ __forceinline__ bool upload_one(const StepArgs& a, int precision, int
     const int cmx = d.periodic ? d.nxr - 1 : d.nx - 1;
     const int cmy = d.periodic ? d.nyr - 1 : d.ny - 1;
     int cx, cy;
-    pos = split_position(d, xi, yi, cmx, cmy, cx, cy);
+    pos = split_position<false>(d, xi, yi, cmx, cmy, cx, cy);
     key = d.cell_base + local_code(d, cx, cy);
   } else {
     pos = make_float2((float)xi, (float)yi);
@@ -137,7 +142,8 @@ __global__ void upload_direct_kernel2(StepArgs a, int precision, const double2* 
   if (a.track_ids) a.idsB[i] = (int32_t)i;
 }
 
-// One position coordinate (axis 0 or 1) of slot i in the caller's FP64 representation.
+// One position coordinate (axis 0 or 1) of slot i in the caller's FP64 representation
+// (lo + c cs in one rounding, as the contracted host code of the staged download).
 __device__ __forceinline__ double download_position(const StepArgs& a, int precision, int64_t i, int axis) {
   const float2 p = a.posA[i];
   const double o = axis ? p.y : p.x;
@@ -145,8 +151,8 @@ __device__ __forceinline__ double download_position(const StepArgs& a, int preci
   const InstDesc& d = inst_ref<true>(a, i);
   int cx, cy;
   decode_code(d, a.keyA[i] - d.cell_base, cx, cy);
-  return axis ? __dadd_rn(__dadd_rn(d.lo_yd, __dmul_rn((double)cy, d.cs_yd)), o)
-              : __dadd_rn(__dadd_rn(d.lo_xd, __dmul_rn((double)cx, d.cs_xd)), o);
+  return axis ? __dadd_rn(__fma_rn((double)cy, d.cs_yd, d.lo_yd), o)
+              : __dadd_rn(__fma_rn((double)cx, d.cs_xd, d.lo_xd), o);
 }
 
 // Entry of `out` that thread t writes: t less the entries between the 128-byte
@@ -194,7 +200,7 @@ __global__ void stage_direct_kernel(InstDesc d, int precision, int64_t n, const 
   int cx, cy;
   float2 p;
   if (precision == SPHG_PRECISION_SPLIT) {
-    p = split_position(d, x[i], y[i], cmx, cmy, cx, cy);
+    p = split_position<true>(d, x[i], y[i], cmx, cmy, cx, cy);
   } else {
     p = make_float2((float)x[i], (float)y[i]);
     cx = cell_coord(p.x, d.lo_x, d.inv_cs_x, d.lo_xd, d.cs_xd, cmx);

@@ -70,3 +70,31 @@ def test_upload_reports_the_first_bad_particle_and_recovers(bad):
     sim.preloop()
     assert sim.diagnostics()[0, 5] == 0
     sim.close()
+
+
+def test_served_positions_round_once():
+    """A served position near a tie of its FP32 offset: c cs is taken off x - lo in
+    one rounding, and added back to lo in one."""
+    from fractions import Fraction
+    import sphg as S
+    lo, cs, m = (-0.3, 0.7), 0.01, 40
+    rng = np.random.default_rng(5)
+    c = 3 * np.arange(m) + 1  # particles three cells apart: no pair, no force, nothing moves
+    xs, want = [], []
+    for axis in (0, 1):
+        o = rng.uniform(0.2 * cs, 0.8 * cs, m).astype(np.float32)
+        tie = (o.astype(np.float64) + np.nextafter(o, np.float32(1)).astype(np.float64)) / 2
+        x = np.array([float(Fraction(lo[axis]) + int(k) * Fraction(cs) + Fraction(t)) for k, t in zip(c, tie)])
+        xs.append(x)
+        off = [np.float32(float(Fraction(v - lo[axis]) - int(k) * Fraction(cs))) for v, k in zip(x, c)]
+        want.append(np.array([float(Fraction(lo[axis]) + int(k) * Fraction(cs)) + float(f) for k, f in zip(c, off)]))
+    x, y = (a.ravel() for a in np.meshgrid(xs[0], xs[1], indexing="ij"))
+    wx, wy = (a.ravel() for a in np.meshgrid(want[0], want[1], indexing="ij"))
+    prm = S.params(order="morton", h=cs, lo=lo, hi=(lo[0] + 1.27, lo[1] + 1.27), gx=0.0, gy=0.0, dt=1e-6)
+    srv = S.Server(2e8, max_instances=4, opts=S.options(precision=S.SPLIT))
+    rid = srv.submit(prm, x, y, np.zeros_like(x), np.zeros_like(x), 1)
+    while srv.tick()[0]:
+        pass
+    r = srv.result(rid)
+    assert np.array_equal(r["x"], wx[r["ids"]]) and np.array_equal(r["y"], wy[r["ids"]])
+    srv.close()
