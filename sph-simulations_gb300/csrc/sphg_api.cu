@@ -488,6 +488,11 @@ sphg_status build_graph_conditional(sphg_sim* s, cudaGraphExec_t* exec, bool hea
 sphg_status build_graph(sphg_sim* s, bool header) {
   cudaGraphExec_t* exec = header ? &s->gexec_hdr : &s->gexec;
   if (*exec) return SPHG_OK;
+  struct InGraph {
+    sphg_sim* s;
+    explicit InGraph(sphg_sim* sim) : s(sim) { s->in_graph = true; }
+    ~InGraph() { s->in_graph = false; }
+  } in_graph(s);
   if (!s->cap_stream) SPHG_CUDA(cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking));
   if (s->movers_on && s->cond_graph) {
     if (build_graph_conditional(s, exec, header) == SPHG_OK) return SPHG_OK;
@@ -513,23 +518,31 @@ sphg_status build_graph(sphg_sim* s, bool header) {
 // Brings the device word of the time step up to date in stream order: what is
 // enqueued already keeps the old one.
 __global__ void write_word(float* p, float v) { *p = v; }
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return false;
+}
 static sphg_status current_dt(sphg_sim* s, cudaStream_t st) {
-  if (!s->dt_stale || s->ninst != 1 || s->force_batched) return SPHG_OK;
+  // in a caller's capture it is written whenever that is replayed, so from then
+  // on before every launch of the handle's graphs
+  if (capturing(st)) s->dt_captured = true;
+  if (!(s->dt_stale || s->dt_captured) || s->ninst != 1 || s->force_batched) return SPHG_OK;
   write_word<<<1, 1, 0, st>>>(s->dt_word, s->hdesc[0].dt);
   SPHG_CUDA(cudaGetLastError());
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  // in a caller's capture it is written when that is replayed
-  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) s->dt_stale = false;
+  s->dt_stale = false;
   return SPHG_OK;
 }
 
 // Iterations of a small single instance run in one cluster, many a launch,
-// instead of a graph each (the same bits; other launch shapes only on request).
-static bool resident_on(const sphg_sim* s) {
+// instead of a graph each (the same bits; other launch shapes only on request;
+// a caller's capture meets the graphs).
+static bool resident_on(const sphg_sim* s, cudaStream_t st) {
   return s->opt.use_graph && s->ninst == 1 && !s->force_batched && s->movers_on && s->nbr && !s->tile_bits &&
          s->opt.compute == SPHG_COMPUTE_SORTED && s->opt.fused == 0 && s->opt.block_threads == 0 &&
          s->opt.cell_pairs == 0 && s->n > 0 && s->n <= sphg::kResidentMaxN &&
-         sphg::resident_blocks(s->opt.precision) > 0;
+         sphg::resident_blocks(s->opt.precision) > 0 && !capturing(st);
 }
 
 static sphg_status run_resident(sphg_sim* s, int64_t k, double* headers, cudaStream_t st) {
@@ -541,14 +554,14 @@ static sphg_status run_resident(sphg_sim* s, int64_t k, double* headers, cudaStr
 
 sphg_status run_steps(sphg_sim* s, int64_t k, cudaStream_t st, bool first = false) {
   if (s->n == 0) return SPHG_OK;
-  SPHG_TRY(current_dt(s, st));
   if (first) {
     SPHG_TRY(enqueue_step(s, st, true));
     --k;
   }
-  if (resident_on(s) && (k != 1 || s->n <= sphg::kResidentSingleMaxN)) return run_resident(s, k, nullptr, st);
+  if (resident_on(s, st) && (k != 1 || s->n <= sphg::kResidentSingleMaxN)) return run_resident(s, k, nullptr, st);
   if (s->opt.use_graph) {
     SPHG_TRY(build_graph(s));
+    SPHG_TRY(current_dt(s, st));
     for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(s->gexec, st));
   } else {
     for (int64_t i = 0; i < k; ++i) SPHG_TRY(enqueue_step(s, st));
@@ -891,8 +904,8 @@ sphg_status sphg_create_batch(int32_t ninst, const sphg_params* p, const int64_t
     st = fail(SPHG_OOM, "pinned host staging");
   // (lists mode: captured after the pre-loop has sized the list buffer)
   const bool capture_now = s->opt.use_graph && s->opt.compute != SPHG_COMPUTE_LISTS;
-  if (st == SPHG_OK && s->n > 0 && capture_now && (!resident_on(s) || s->n > sphg::kResidentSingleMaxN)) st = build_graph(s);
-  if (st == SPHG_OK && s->n > 0 && capture_now && !resident_on(s)) st = build_graph(s, true);  // with step headers
+  if (st == SPHG_OK && s->n > 0 && capture_now && (!resident_on(s, nullptr) || s->n > sphg::kResidentSingleMaxN)) st = build_graph(s);
+  if (st == SPHG_OK && s->n > 0 && capture_now && !resident_on(s, nullptr)) st = build_graph(s, true);  // with step headers
   if (st != SPHG_OK) {
     destroy_impl(s);
     return st;
@@ -1238,12 +1251,12 @@ sphg_status sphg_step_headers(sphg_sim* s, int64_t nsteps, double* out, void* st
     }
     return SPHG_OK;
   }
-  SPHG_TRY(current_dt(s, st));
-  if (resident_on(s)) return run_resident(s, nsteps, dv, st);
+  if (resident_on(s, st)) return run_resident(s, nsteps, dv, st);
   const sphg::HeaderSlot h = {dv, 0u, 0u};
   SPHG_CUDA(cudaMemcpyAsync(s->hslot, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   if (s->opt.use_graph) {
     SPHG_TRY(build_graph(s, true));
+    SPHG_TRY(current_dt(s, st));
     for (int64_t k = 0; k < nsteps; ++k) SPHG_CUDA(cudaGraphLaunch(s->gexec_hdr, st));
   } else {
     for (int64_t k = 0; k < nsteps; ++k) {
@@ -1496,7 +1509,6 @@ sphg_status sphg_profile_step(sphg_sim* s, float* ms, void* stream) {
   if (!s || !ms || !s->preloop_done) return fail(SPHG_INVALID_ARG, "no computed state or null output");
   cudaStream_t st = (cudaStream_t)stream;
   cudaEvent_t ev[6];
-  SPHG_TRY(current_dt(s, st));
   for (int i = 0; i < 6; ++i) SPHG_CUDA(cudaEventCreate(&ev[i]));
   sphg_status res = enqueue_step(s, st, false, ev);
   if (res == SPHG_OK) {

@@ -104,10 +104,13 @@ struct sphg_sim {
   bool cond_graph = true;       // full sort under a conditional graph node (when the merge is on)
   cudaGraphExec_t gexec = nullptr;
   cudaGraphExec_t gexec_hdr = nullptr;  // the same followed by the step header into hslot
-  // one instance: the time step as the kernels of the graphs read it (a device
-  // word), and whether it has changed since it was written there
+  // one instance: the time step as the kernels of the handle's graphs read it (a
+  // device word; launches outside them carry it by value), whether it has changed
+  // since it was written there, and whether a graph of the caller's may write it
   float* dt_word = nullptr;
   bool dt_stale = true;
+  bool dt_captured = false;
+  bool in_graph = false;  // a graph of the handle is being captured
   void drop_graphs() {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (gexec_hdr) cudaGraphExecDestroy(gexec_hdr);
@@ -159,7 +162,7 @@ struct sphg_sim {
     a.csr_overflow = flags + 8;
     a.keyS = keyTmp;
     a.merged = movers_on ? flags + 3 : nullptr;
-    a.dt = ninst == 1 && !force_batched ? dt_word : nullptr;
+    a.dt = in_graph && ninst == 1 && !force_batched ? dt_word : nullptr;
     if (movers_on) {
       a.movers = mrec;
       a.movers.last = flags + 4;

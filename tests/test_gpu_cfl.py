@@ -60,3 +60,39 @@ def test_changed_time_step(opts, headers):
         sim.close()
     for f in out[0]:
         assert np.array_equal(out[0][f], out[1][f]), f
+
+
+def test_time_step_of_a_captured_iteration():
+    """An iteration in a caller's graph keeps the time step it was captured with
+    and leaves the handle's own as it is."""
+    import sphg as S
+    import torch
+    import workloads as W
+    p, x, y, vx, vy = W.dam_break(60, 70, 0.005, seed=4, dt=1e-5)
+    out = []
+    for captured in (True, False):
+        sim = S.Sim(S.params(**p), len(x), S.options(precision=S.SPLIT, use_graph=0))
+        st = torch.cuda.Stream()
+        ptr = st.cuda_stream
+        sim.upload(x, y, vx, vy, stream=ptr)
+        sim.preloop(stream=ptr)
+        sim.set_dt(2e-5)
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=st):
+                sim.step(1, stream=ptr)
+        for dt in (1e-5, 3e-5):
+            sim.set_dt(dt)
+            sim.step(1, stream=ptr)
+            if captured:
+                with torch.cuda.stream(st):
+                    g.replay()
+            else:
+                sim.set_dt(2e-5)
+                sim.step(1, stream=ptr)
+                sim.set_dt(dt)
+            sim.step(2, stream=ptr)
+        out.append(sim.download(stream=ptr))
+        sim.close()
+    for f in out[0]:
+        assert np.array_equal(out[0][f], out[1][f]), f
