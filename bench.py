@@ -61,7 +61,7 @@ METRIC = ("particle-steps/s on 1 GB300, batched vs plain GPU path at ≤1e-5 rel
 UNIT = "particle-steps/s"
 BYTES_PER_PARTICLE_STEP = 80.0  # algorithmic: sweep A 44 B (state in/out, key, perm, rho) + sweep B 36 B
 # DRAM bytes per particle-step measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum
-# summed over one merge-path iteration's kernels -- re-sort merge, reorder, density, force --
+# summed over one merge-path iteration's kernels -- re-sort merge, density, force --
 # caches flushed before each captured launch; profiles/traffic_dam_break_1m.md,
 # profiles/launches_batch_256.md)
 TRAFFIC_PER_PARTICLE_STEP = {"dam_break_1m": 104.3, "batch_256": 186.3}
@@ -262,7 +262,7 @@ def roofline_of(name, value, n):
             "traffic": tr * n if tr is not None else None,
             "traffic_unit": "DRAM bytes per main-loop iteration (ncu)",
             "peak_source": src,
-            "kernel": "one main-loop iteration (re-sort or radix sort + reorder + density + force)",
+            "kernel": "one main-loop iteration (re-sort, or radix sort + reorder; density; force)",
             "algorithmic_bytes_per_particle_step": BYTES_PER_PARTICLE_STEP}
 
 
@@ -316,6 +316,8 @@ def device_record(name, args, opts, stream, steps, warmup, with_e2e=True, world=
     full_sort_kernels = int(sim.debug(sphg.DBG_RESORT, stream=sptr)[2])
     per_step = sim.launches_per_step()
     rs = resort_summary(log)
+    if opts.compute == sphg.LISTS:
+        per_step -= 4  # the lists are assembled in one kernel of the five the library counts for them
     launches = int(round(steps * per_step - (rs["steps"] * rs["merged_fraction"]) * full_sort_kernels))
     # per-phase profile (CUDA events between the kernels of one iteration)
     phases = np.array([sim.profile_step(stream=sptr) for _ in range(10)])

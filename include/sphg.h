@@ -124,14 +124,13 @@ typedef struct sphg_options {
                           the same results) */
   int32_t fused;       /* 1: each iteration that merges is ONE cooperative launch (re-sort,
                           cell ranges, density, forces as phases between grid-wide
-                          barriers) instead of four kernels -- for small and medium
+                          barriers) instead of three kernels -- for small and medium
                           workloads, whose kernel boundaries cost as much as their work;
                           the same results.  Sorted compute mode without cell tiles only;
                           its grid fills the GPU, so two handles must not run such
                           iterations at the same time on one GPU (different streams):
                           their barriers would wait on each other until their bounded
-                          waits give up (SPHG_TIMEOUT).  0 (default): a graph of four
-                          kernels */
+                          waits give up (SPHG_TIMEOUT).  0 (default): a graph of kernels */
 } sphg_options;
 
 typedef struct sphg_sim sphg_sim;

@@ -4,11 +4,11 @@
 // Layout in HBM (structure of arrays, one entry per particle slot, all
 // instances of a handle concatenated in instance order):
 //   pos    float2  position (plain) or in-cell offset (split precision)
-//   velp   float4  (vx, vy, P = p/rho^2, 1/rho)  -- written by reorder (xy) and density (zw)
+//   velp   float4  (vx, vy, P = p/rho^2, 1/rho)  -- written by the re-sort (xy) and density (zw)
 //   rho    float   density
 //   key    uint32  global cell key = instance cell_base + Morton/row-major code
-//   range  uint2   per global key: [start, end) of its particles in the sorted order
-//                  (valid only when key[start] == that key; never cleared)
+//   range  uint4   per global key: [start, end) of its particles in the sorted order
+//                  and the epoch it holds for (never cleared)
 // and a second copy of pos/vel ("next" state) written by the fused
 // force+integrate kernel and consumed by the next sort.
 #pragma once

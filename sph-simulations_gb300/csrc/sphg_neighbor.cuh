@@ -2,8 +2,8 @@
 // integration epilogue shared by the density, force and neighbour-list kernels.
 //
 // Cell ranges: one 16-byte entry per global cell key, {start, end, epoch, 0}.
-// The reorder kernel writes the entries of the occupied cells with the current
-// step's epoch (bumped by the sort); an entry whose epoch is not the current
+// The re-sort (the merge, or the reorder after a full sort) writes the entries of
+// the occupied cells with the step's epoch, one more than the last; an entry whose epoch is not the current
 // one belongs to a cell that is empty now.  The table is never cleared.
 #pragma once
 #include <cstdint>

@@ -386,9 +386,6 @@ __global__ void __launch_bounds__(T, density_blocks(PREC, BATCHED, T)) step_dens
 // 256 consecutive slots, splits each run of equal keys (a cell, or the part of
 // it inside the block) into pairs from its first slot, and hands the pairs
 // and the odd particles out to its threads in slot order.
-// slots per block: two per thread
-
-
 // One particle's running state of the walk.
 template <int PREC>
 struct WalkAcc {
@@ -635,9 +632,6 @@ __global__ void __launch_bounds__(T) step_density_pairs(StepArgs a) {
 #define SPHG_FORCE_BATCH 4
 #endif
 constexpr int kForceBatch = SPHG_FORCE_BATCH;  // recorded neighbours gathered together
-#ifndef SPHG_FORCE_TAIL
-#define SPHG_FORCE_TAIL 1
-#endif
 #ifndef SPHG_SKIP_ZERO_VISCOSITY
 #define SPHG_SKIP_ZERO_VISCOSITY 1
 #endif
@@ -661,10 +655,10 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
 // Threads per SM the force pass is compiled for.  Split precision: 1,152
 // (nine 128-thread blocks, 56 registers) for one instance and 1,024 (eight
 // blocks, 64 registers; the instance lookup spills a few bytes) for the batched
-// variants -- measured on the GB300 against 1,024 / the compiler's own 72
-// registers: 29.8 against 31.7 us on the 1M dam break, 0.408 against 0.420 ms
-// per batch_256 iteration.  Plain positions need more registers: 1,024 for one
-// instance, the compiler's choice batched (fewer spill).
+// variants -- an iteration against one block fewer an SM: 1M dam break 82.2 / 82.8
+// us, batch of 256 405.8 / 408.9.  Plain positions need more registers: 1,024 for
+// one instance (512 x 512 vortex 37.4 us, 37.6 at 896), the compiler's choice
+// batched (served ticks the same at 1,024).
 #ifndef SPHG_FORCE_THREADS_PER_SM
 #define SPHG_FORCE_THREADS_PER_SM 1152
 #endif
@@ -795,11 +789,10 @@ __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, cons
     // the density pass recorded this particle's neighbours (stencil order)
     const size_t n = (size_t)a.n;
     // kForceBatch neighbours at a time, their gathers in flight together.  The
-    // lanes of a warp all run the warp's largest count: whole batches, then
-    // (SPHG_FORCE_TAIL) a batch of two and a single one for the rest; a lane's
-    // missing entries are the particle itself (stencil cell 4, no shift), whose
-    // pair term is exactly zero (r = 0, v_j = v_i), so the sums are the same
-    // whatever the batching.
+    // lanes of a warp all run the warp's largest count: whole batches, then a
+    // batch of two and a single one for the rest; a lane's missing entries are
+    // the particle itself (stencil cell 4, no shift), whose pair term is exactly
+    // zero (r = 0, v_j = v_i), so the sums are the same whatever the batching.
     const uint32_t wmax = __reduce_max_sync(__activemask(), cnt);
     const uint32_t self_e = ((uint32_t)i << 5) | 4u;
     auto load = [&](auto width, uint32_t q, uint32_t* e) {

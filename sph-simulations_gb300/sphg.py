@@ -331,8 +331,8 @@ class Sim:
         return offs, enc[:total.value]
 
     def set_host_access(self, mode):
-        """0: pinned staging; 1: upload reads the caller's arrays from the device;
-        2: download writes them from the device as well."""
+        """0: pinned staging; 1: the device reads and writes the caller's arrays, the
+        download's pages touched by the host first; 2: the same without touching them."""
         check(lib().sphg_set_host_access(self._h, int(mode)))
 
     def diagnostics_async(self, out_ptr, stream=None):
