@@ -535,6 +535,16 @@ static sphg_status current_dt(sphg_sim* s, cudaStream_t st) {
   return SPHG_OK;
 }
 
+// The graph an iteration on st needs, made if it is not there (a small instance
+// has none until one is asked for; not from inside a caller's capture, where its
+// launch fails anyway).
+static sphg_status ready_graph(sphg_sim* s, bool header, cudaStream_t st) {
+  if (!(header ? s->gexec_hdr : s->gexec) && capturing(st))
+    return fail(SPHG_CUDA_ERROR, "an iteration of a graph inside a stream capture");
+  SPHG_TRY(build_graph(s, header));
+  return current_dt(s, st);
+}
+
 // Iterations of a small single instance run in one cluster, many a launch,
 // instead of a graph each (the same bits; other launch shapes only on request;
 // a caller's capture meets the graphs).
@@ -560,8 +570,7 @@ sphg_status run_steps(sphg_sim* s, int64_t k, cudaStream_t st, bool first = fals
   }
   if (resident_on(s, st) && (k != 1 || s->n <= sphg::kResidentSingleMaxN)) return run_resident(s, k, nullptr, st);
   if (s->opt.use_graph) {
-    SPHG_TRY(build_graph(s));
-    SPHG_TRY(current_dt(s, st));
+    SPHG_TRY(ready_graph(s, false, st));
     for (int64_t i = 0; i < k; ++i) SPHG_CUDA(cudaGraphLaunch(s->gexec, st));
   } else {
     for (int64_t i = 0; i < k; ++i) SPHG_TRY(enqueue_step(s, st));
@@ -1255,8 +1264,7 @@ sphg_status sphg_step_headers(sphg_sim* s, int64_t nsteps, double* out, void* st
   const sphg::HeaderSlot h = {dv, 0u, 0u};
   SPHG_CUDA(cudaMemcpyAsync(s->hslot, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   if (s->opt.use_graph) {
-    SPHG_TRY(build_graph(s, true));
-    SPHG_TRY(current_dt(s, st));
+    SPHG_TRY(ready_graph(s, true, st));
     for (int64_t k = 0; k < nsteps; ++k) SPHG_CUDA(cudaGraphLaunch(s->gexec_hdr, st));
   } else {
     for (int64_t k = 0; k < nsteps; ++k) {
