@@ -358,15 +358,17 @@ __device__ __forceinline__ void density_particle(const StepArgs& a, int64_t i, Q
   st_out<LAUNCH>(reinterpret_cast<float2*>(a.velpA + i) + 1, make_float2(P, inv));
 }
 
-// Threads per SM the density pass is compiled for.  Split precision, one
-// instance: nine 128-thread blocks; ten (the compiler's 48 registers) leave too
-// little of the shared memory to L1 beside their queues (hit rate 45 against
-// 78 %, 1M dam break 97.3 against 94.1 us an iteration).  The others take the
-// compiler's 56 registers, nine blocks too.
-constexpr int density_blocks(int prec, bool batched, int t) { return prec == 1 && !batched ? 1152 / t : 0; }
+// Threads per SM the density pass is compiled for.  Split precision: nine
+// 128-thread blocks (56 registers).  One instance: ten (the compiler's 48
+// registers) leave too little of the shared memory to L1 beside their queues (hit
+// rate 45 against 78 %, 1M dam break 97.3 against 94.1 us an iteration).
+// Batched: eight (the compiler's 60 registers) hide less of the range and
+// candidate loads (batch of 256 397.9 against 388.2 us).  Plain precision takes
+// the compiler's 56 registers, nine blocks too.
+constexpr int density_blocks(int prec, int t) { return prec == 1 ? 1152 / t : 0; }
 
 template <int PREC, bool BATCHED, bool CSR, int T = kThreads>
-__global__ void __launch_bounds__(T, density_blocks(PREC, BATCHED, T)) step_density(StepArgs a) {
+__global__ void __launch_bounds__(T, density_blocks(PREC, T)) step_density(StepArgs a) {
   __shared__ QueuedCell<PREC> s_cells[CSR ? 1 : kQueuedCells][T];
   cudaGridDependencySynchronize();  // the sorted state and cell ranges of the re-sort
   allow_next_kernel(a.early_next);
