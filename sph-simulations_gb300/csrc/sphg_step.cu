@@ -654,21 +654,17 @@ struct ForceIn {
 template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit, const ForceIn& in);
 
-// Threads per SM the force pass is compiled for.  Split precision: 1,152
-// (nine 128-thread blocks, 56 registers) for one instance and 1,024 (eight
-// blocks, 64 registers; the instance lookup spills a few bytes) for the batched
-// variants -- an iteration against one block fewer an SM: 1M dam break 82.2 / 82.8
-// us, batch of 256 405.8 / 408.9.  Plain positions need more registers: 1,024 for
-// one instance (512 x 512 vortex 37.4 us, 37.6 at 896), the compiler's choice
-// batched (served ticks the same at 1,024).
+// Threads per SM the force pass is compiled for.  Split precision: 1,152 (nine
+// 128-thread blocks, 56 registers; the batched variants' instance lookup spills a
+// 100 bytes) -- an iteration against one block fewer: 1M dam break 82.2 / 82.8 us,
+// batch of 256 377.4 / 388.2; against one more 81.0 / 82.3 and 381.6 / 382.4.  Plain
+// positions need more registers: 1,024 for one instance (512 x 512 vortex 37.4 us,
+// 37.6 at 896), the compiler's choice batched (served ticks the same at 1,024).
 #ifndef SPHG_FORCE_THREADS_PER_SM
 #define SPHG_FORCE_THREADS_PER_SM 1152
 #endif
-#ifndef SPHG_FORCE_BATCHED_THREADS_PER_SM
-#define SPHG_FORCE_BATCHED_THREADS_PER_SM 1024
-#endif
 constexpr int force_threads_per_sm(int prec, bool batched) {
-  return prec == 1 ? (batched ? SPHG_FORCE_BATCHED_THREADS_PER_SM : SPHG_FORCE_THREADS_PER_SM) : (batched ? 0 : 1024);
+  return prec == 1 ? SPHG_FORCE_THREADS_PER_SM : (batched ? 0 : 1024);
 }
 template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ void force_slot(const StepArgs& a, int64_t i, const float2* unit);
