@@ -655,7 +655,7 @@ template <int PREC, bool BATCHED, int MODE, bool CSR, int LAUNCH>
 __device__ __forceinline__ uint32_t force_one(const StepArgs& a, int64_t i, const float2* unit, const ForceIn& in);
 
 // Threads per SM the force pass is compiled for.  Split precision: 1,152 (nine
-// 128-thread blocks, 56 registers; the batched variants' instance lookup spills a
+// 128-thread blocks, 56 registers; the batched variants' instance lookup spills
 // 100 bytes) -- an iteration against one block fewer: 1M dam break 82.2 / 82.8 us,
 // batch of 256 377.4 / 388.2; against one more 81.0 / 82.3 and 381.6 / 382.4.  Plain
 // positions need more registers: 1,024 for one instance (512 x 512 vortex 37.4 us,
