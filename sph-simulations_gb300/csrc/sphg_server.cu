@@ -5,8 +5,8 @@
 // to generate, the parameters, a step count) wait in a FIFO queue.  Each tick:
 //   1. admits queued requests, in order, while they fit;
 //   2. places the newcomers: normally APPENDED after the last slot and the last
-//      cell key in use -- their initial states are staged (pinned host copies,
-//      or the device lattice generator), sorted among themselves by cell key,
+//      cell key in use -- their initial states are staged (host arrays converted
+//      by the device or through pinned copies, or the device lattice generator), sorted among themselves by cell key,
 //      and written as "integrated states awaiting the next sort" with no mover
 //      bit, so the running instances keep their slots and the incremental
 //      re-sort keeps merging; when the arena's end is reached, or finished
@@ -297,7 +297,8 @@ sphg_status apply(sphg_server* s, const std::vector<SlotEntry>& ents, const Layo
 
 // Stages the newcomers' initial states at [at, at + m) of the staging buffers
 // (posA / acc / keyTmp / idsA: free between ticks beyond the slots in use):
-// host arrays through pinned memory, lattices generated on the device.  Keys
+// host arrays converted by the device or through pinned memory, lattices
+// generated on the device.  Keys
 // are instance-local codes.
 sphg_status stage_all(sphg_server* s, const std::vector<int64_t>& ids, const std::vector<InstDesc>& descs,
                       int64_t at, cudaStream_t st) {
