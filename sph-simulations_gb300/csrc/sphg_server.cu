@@ -6,9 +6,9 @@
 //   1. admits queued requests, in order, while they fit;
 //   2. places the newcomers: normally APPENDED after the last slot and the last
 //      cell key in use -- their initial states are staged (host arrays converted
-//      by the device or through pinned copies, or the device lattice generator), sorted among themselves by cell key,
-//      and written as "integrated states awaiting the next sort" with no mover
-//      bit, so the running instances keep their slots and the incremental
+//      by the device or through pinned copies, or the device lattice generator),
+//      sorted among themselves by cell key, and written as "integrated states
+//      awaiting the next sort" with no mover bit, so the running instances keep their slots and the incremental
 //      re-sort keeps merging; when the arena's end is reached, or finished
 //      instances hold more slots than live ones, the live set is COMPACTED
 //      (dense repack, one full radix sort);
