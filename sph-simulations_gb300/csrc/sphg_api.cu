@@ -548,17 +548,18 @@ static sphg_status ready_graph(sphg_sim* s, bool header, cudaStream_t st) {
 // Iterations of a small single instance run in one cluster, many a launch,
 // instead of a graph each (the same bits; other launch shapes only on request;
 // a caller's capture meets the graphs).
-static bool resident_on(const sphg_sim* s, cudaStream_t st) {
+static int resident_blocks(const sphg_sim* s) {
   return s->opt.use_graph && s->ninst == 1 && !s->force_batched && s->movers_on && s->nbr && !s->tile_bits &&
          s->opt.compute == SPHG_COMPUTE_SORTED && s->opt.fused == 0 && s->opt.block_threads == 0 &&
-         s->opt.cell_pairs == 0 && s->n > 0 && s->n <= sphg::kResidentMaxN &&
-         sphg::resident_blocks(s->opt.precision) > 0 && !capturing(st);
+         s->opt.cell_pairs == 0 && s->n > 0 && s->n <= sphg::kResidentMaxN
+             ? sphg::resident_blocks(s->opt.precision) : 0;
 }
+static bool resident_on(const sphg_sim* s, cudaStream_t st) { return s->resident > 0 && !capturing(st); }
 
 static sphg_status run_resident(sphg_sim* s, int64_t k, double* headers, cudaStream_t st) {
   if (k <= 0) return SPHG_OK;
-  SPHG_CUDA(sphg::launch_resident(s->args(), mover_args(s, 0), s->opt.precision, k, headers, s->diag_partials,
-                                  sphg::diag_chunks(s->n, 1, s->diag_chunks), st));
+  SPHG_CUDA(sphg::launch_resident(s->args(), mover_args(s, 0), s->opt.precision, s->resident, k, headers,
+                                  s->diag_partials, sphg::diag_chunks(s->n, 1, s->diag_chunks), st));
   return SPHG_OK;
 }
 
@@ -911,6 +912,7 @@ sphg_status sphg_create_batch(int32_t ninst, const sphg_params* p, const int64_t
   if (st == SPHG_OK && s->n > 0 && !s->host_direct &&
       !host_stage(s, (size_t)s->n * (sizeof(float2) * 2 + sizeof(float4) + sizeof(float) + sizeof(uint32_t))))
     st = fail(SPHG_OOM, "pinned host staging");
+  if (st == SPHG_OK) s->resident = resident_blocks(s);
   // (lists mode: captured after the pre-loop has sized the list buffer)
   const bool capture_now = s->opt.use_graph && s->opt.compute != SPHG_COMPUTE_LISTS;
   if (st == SPHG_OK && s->n > 0 && capture_now && (!resident_on(s, nullptr) || s->n > sphg::kResidentSingleMaxN)) st = build_graph(s);

@@ -1629,43 +1629,41 @@ cudaError_t launch_cell_keys_plain(const InstDesc& d, const float* x, const floa
   return cudaGetLastError();
 }
 
-// Blocks of the resident cluster on this device (0: it cannot be launched).
+// Blocks of the resident cluster on the current device (0: it cannot be launched).
+// The kernel's attributes, which a launch needs, belong to the device's context:
+// they are set here, for each handle when it is made.
 template <int PREC>
 static int resident_cluster() {
-  static const int blocks = [] {
-    const int smem = (int)sizeof(ResidentShared<PREC>);
-    const auto k = step_resident<PREC>;
-    int found = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
-      for (int c : {16, 8}) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(c);
-        cfg.blockDim = dim3(kResidentThreads);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = c;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0) {
-          found = c;
-          break;
-        }
+  const int smem = (int)sizeof(ResidentShared<PREC>);
+  const auto k = step_resident<PREC>;
+  int found = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+    for (int c : {16, 8}) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(c);
+      cfg.blockDim = dim3(kResidentThreads);
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0) {
+        found = c;
+        break;
       }
-    cudaGetLastError();
-    return found;
-  }();
-  return blocks;
+    }
+  cudaGetLastError();
+  return found;
 }
 
 int resident_blocks(int precision) { return precision ? resident_cluster<1>() : resident_cluster<0>(); }
 
-cudaError_t launch_resident(const StepArgs& a, const MoverArgs& m, int precision, int64_t iters, double* headers,
-                            double* partials, int chunks, cudaStream_t s) {
-  const int c = resident_blocks(precision);
+cudaError_t launch_resident(const StepArgs& a, const MoverArgs& m, int precision, int c, int64_t iters,
+                            double* headers, double* partials, int chunks, cudaStream_t s) {
   if (c <= 0) return cudaErrorNotSupported;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(c);

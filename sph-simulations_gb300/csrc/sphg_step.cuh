@@ -79,12 +79,13 @@ int fused_blocks(const StepArgs& a, int precision);
 // (step_resident): measured against the graph of kernels in sphg_step.cu.
 constexpr int64_t kResidentMaxN = 16384;
 constexpr int64_t kResidentSingleMaxN = 12000;  // in calls of one iteration without a header
-// Blocks of that cluster (0: not available here), and `iters` iterations of the
-// current state; headers (device-accessible, 6 doubles per iteration) or null,
+// Blocks of that cluster (0: not available here; makes the kernel launchable in the
+// current context), and `iters` iterations of the current state in a cluster of that
+// many blocks; headers (device-accessible, 6 doubles per iteration) or null,
 // with the diagnostics partials and chunk count of launch_diagnostics.
 int resident_blocks(int precision);
-cudaError_t launch_resident(const StepArgs& a, const MoverArgs& m, int precision, int64_t iters, double* headers,
-                            double* partials, int chunks, cudaStream_t s);
+cudaError_t launch_resident(const StepArgs& a, const MoverArgs& m, int precision, int blocks, int64_t iters,
+                            double* headers, double* partials, int chunks, cudaStream_t s);
 cudaError_t launch_reorder(const StepArgs& a, cudaStream_t s);
 cudaError_t launch_density(const StepArgs& a, int precision, cudaStream_t s, bool csr = false);
 cudaError_t launch_force(const StepArgs& a, int precision, int mode, cudaStream_t s, bool csr = false);

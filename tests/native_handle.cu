@@ -1,0 +1,103 @@
+// Host program of tests/test_gpu_native_handle.py: checks of a handle that the
+// C ABI alone cannot set up.  Linked with the library's own objects, so that both
+// share one CUDA runtime.  Usage: native_handle <check>; exits 0 when it holds.
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <set>
+#include <string>
+#include <utility>
+#include <vector>
+
+#include <cuda_runtime.h>
+
+#include "../include/sphg.h"
+
+// A kernel's attributes belong to the device that was current when they were set.
+// With one device at hand the program plays two: it keeps, by the device it plays,
+// which kernels may use more than 48 KB of shared memory, and refuses the launches
+// that the device would refuse (linked with --wrap of the two calls).
+static int fake_device = 0;
+static std::set<std::pair<int, const void*>> large_memory;
+extern "C" cudaError_t __real_cudaFuncSetAttribute(const void* f, cudaFuncAttribute attr, int value);
+extern "C" cudaError_t __wrap_cudaFuncSetAttribute(const void* f, cudaFuncAttribute attr, int value) {
+  if (attr == cudaFuncAttributeMaxDynamicSharedMemorySize) large_memory.insert({fake_device, f});
+  return __real_cudaFuncSetAttribute(f, attr, value);
+}
+extern "C" cudaError_t __real_cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args);
+extern "C" cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
+  if (c->dynamicSmemBytes > (48u << 10) && !large_memory.count({fake_device, f})) return cudaErrorInvalidValue;
+  return __real_cudaLaunchKernelExC(c, f, args);
+}
+
+namespace {
+
+int failed(const char* what) {
+  std::printf("%s: %s\n", what, sphg_last_error_string());
+  return 1;
+}
+
+struct State {
+  std::vector<double> x, y, vx, vy;
+};
+State lattice(int nx, int ny) {
+  State s;
+  for (int i = 0; i < nx * ny; ++i) {
+    s.x.push_back((i % nx + 0.5) / nx);
+    s.y.push_back((i / nx + 0.5) / ny);
+    s.vx.push_back(std::sin(0.1 * i));
+    s.vy.push_back(std::cos(0.1 * i));
+  }
+  return s;
+}
+sphg_params box(double h) {
+  sphg_params p;
+  sphg_default_params(&p);
+  p.h = h;
+  p.dt = 1e-4;
+  p.lo[0] = p.lo[1] = 0.0;
+  p.hi[0] = p.hi[1] = 1.0;
+  return p;
+}
+
+// A small handle's iterations, and its state after them.
+int small_run(int precision, std::vector<double>& out) {
+  const State st = lattice(40, 30);
+  const int64_t n = (int64_t)st.x.size();
+  const sphg_params p = box(0.04);
+  sphg_options o;
+  sphg_default_options(&o);
+  o.precision = precision;
+  sphg_sim* s = nullptr;
+  if (sphg_create(&p, &o, n, &s) != SPHG_OK) return failed("create");
+  out.assign(4 * n, 0.0);
+  const int bad = sphg_upload(s, st.x.data(), st.y.data(), st.vx.data(), st.vy.data(), nullptr) != SPHG_OK ||
+                  sphg_preloop(s, nullptr) != SPHG_OK || sphg_step(s, 10, nullptr) != SPHG_OK ||
+                  sphg_download(s, &out[0], &out[n], &out[2 * n], &out[3 * n], nullptr, nullptr, nullptr, nullptr,
+                                nullptr) != SPHG_OK;
+  if (bad) failed("run");
+  sphg_destroy(s);
+  return bad;
+}
+
+// Handles on two devices: the second is played by the wrapped calls.
+int devices() {
+  for (int precision : {SPHG_PRECISION_PLAIN, SPHG_PRECISION_SPLIT}) {
+    std::vector<double> a, b;
+    fake_device = 0;
+    if (small_run(precision, a)) return 1;
+    fake_device = 1;
+    if (small_run(precision, b)) return 1;
+    if (std::memcmp(a.data(), b.data(), a.size() * sizeof(double))) return failed("another result");
+  }
+  return 0;
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const std::string check = argc > 1 ? argv[1] : "";
+  if (check == "devices") return devices();
+  std::printf("unknown check\n");
+  return 2;
+}

@@ -1,0 +1,35 @@
+"""Checks of a handle through a host program linked with the library's objects
+(native_handle.cu): what the C ABI alone cannot set up."""
+import glob
+import os
+import subprocess
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    import build as B  # the package's own build script
+    exe = str(tmp_path_factory.mktemp("native") / "native_handle")
+    objs = sorted(glob.glob(os.path.join(B.BUILD, "*.cu.o")))
+    assert objs, "the library's objects are not built"
+    wrap = ["-Xlinker", "--wrap=cudaFuncSetAttribute,--wrap=cudaLaunchKernelExC"]
+    subprocess.check_call([B.nvcc()] + B.NVCC_FLAGS + [os.path.join(HERE, "native_handle.cu")] + objs + wrap +
+                          ["-o", exe])
+    return exe
+
+
+def _check(program, name):
+    r = subprocess.run([program, name], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_small_handles_on_a_second_device(program):
+    """The resident kernel's attributes belong to the device they were set on: a
+    handle made on another one (played by the program's wrapped calls) runs too,
+    with the same bits."""
+    _check(program, "devices")
