@@ -1231,8 +1231,8 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocks) step_diag(StepArgs 
 // no co-residency of the whole grid and several handles may run at once.  The
 // phases are the same device code as the kernels (the same bits); what one
 // phase wrote the next reads after a barrier with release / acquire order, by
-// plain loads.  An iteration the merge does not take (merge_wanted) is sorted
-// by counting, for every particle, the (key, slot) pairs before its own.
+// plain loads.  An iteration the merge does not take (merge_wanted) is sorted in
+// the cluster too (resident_sort).
 // Measured, us an iteration, cluster against graph (split precision, 64
 // iterations a call): 1,023 particles 12.9 / 23.4, 6,400 14.8 / 25.1, 14,375
 // 18.4 / 25.3, 16,200 18.8 / 25.9, 20,300 25.5 / 25.8 (a second round of the
@@ -1243,6 +1243,7 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocks) step_diag(StepArgs 
 constexpr int kResidentThreads = 1024;
 constexpr int kResidentGroups = kResidentThreads / kResidentMergeThreads;   // merge blocks at a time
 constexpr int kResidentChunks = kResidentThreads / kDiagThreads;    // diagnostics chunks at a time
+constexpr int kResidentSortKeys = kResidentMaxN / 8;  // slots of a block, in a cluster of eight at least
 constexpr int kResidentIters = 128;  // iterations a launch: launches amortised, about a millisecond at most
 
 template <int PREC>
@@ -1250,7 +1251,11 @@ struct ResidentShared {
   union {
     QueuedCell<PREC> cells[kQueuedCells][kResidentThreads];
     MergeShared merge[kResidentGroups];
-    uint4 keys[kResidentThreads / 4];
+    struct {
+      uint32_t all[kResidentMaxN];            // the blocks' sorted keys, one run a block
+      uint32_t key[kResidentSortKeys];        // the block's own
+      uint16_t slot[kResidentSortKeys];       // and where in the block's slots each comes from
+    } sort;
   };
   DiagPart warps[kResidentThreads / 32];
   float2 unit[16];
@@ -1260,41 +1265,96 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// The stable sort of an iteration that the merge does not take: every thread
-// counts, over all keys, the slots ordered before its own.
-template <int PREC>
-__device__ __forceinline__ void resident_sort(const StepArgs& a, ResidentShared<PREC>& sh, uint32_t i0, uint32_t i1,
-                                              uint32_t epoch) {
-  const uint32_t n = (uint32_t)a.n, tid = threadIdx.x;
-  uint32_t* tile = reinterpret_cast<uint32_t*>(sh.keys);
-  for (uint32_t b = i0; b < i1; b += kResidentThreads) {
-    const uint32_t i = b + tid;
-    const bool in = i < i1;
-    const uint32_t k = in ? a.keyB[i] : 0u;
-    uint32_t rank = 0;
-    for (uint32_t t0 = 0; t0 < n; t0 += kResidentThreads) {
-      __syncthreads();
-      tile[tid] = t0 + tid < n ? a.keyB[t0 + tid] : kNoIndex;  // keys are below kNoIndex
-      __syncthreads();
-      if (t0 + kResidentThreads <= i) {  // every slot of the tile comes before i: ties count
-        for (int q = 0; q < kResidentThreads / 4; ++q) {
-          const uint4 t = sh.keys[q];
-          rank += (t.x <= k) + (t.y <= k) + (t.z <= k) + (t.w <= k);
-        }
-      } else {
-        for (int q = 0; q < kResidentThreads; ++q) rank += tile[q] < k || (tile[q] == k && t0 + q < i);
-      }
-    }
-    if (in) {
-      const float2 v = a.velB[i];
-      a.keyA[rank] = k;
-      a.perm[rank] = i;
-      a.posA[rank] = a.posB[i];
-      a.velpA[rank] = make_float4(v.x, v.y, 0.f, 0.f);
-      if (a.track_ids) a.idsA[rank] = a.idsB[i];
-    }
+// 16 bytes of another block's shared memory: p is where the own block holds the same.
+__device__ __forceinline__ uint4 ld_block(const void* p, uint32_t block) {
+  uint32_t at;
+  uint4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(block));
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+  return v;
+}
+
+// Entries of the `run` (a power of two) ascending keys that come before key k: the
+// smaller ones and, when `ties`, the equal ones.
+__device__ __forceinline__ uint32_t keys_before(const uint32_t* keys, uint32_t run, uint32_t k, bool ties) {
+  uint32_t c = 0;
+  for (uint32_t s = run >> 1; s; s >>= 1) {
+    const uint32_t v = keys[c + s - 1];
+    c += v < k || (ties && v == k) ? s : 0u;
   }
+  const uint32_t v = keys[c];
+  return c + (v < k || (ties && v == k) ? 1u : 0u);
+}
+
+// The stable sort of an iteration that the merge does not take.  A block sorts the
+// keys of its own slots -- runs of 32 ranked in a warp, then merged by pairs, every
+// key finding its place in the other run by bisection -- copies every other block's
+// run out of its shared memory, and places its keys by bisecting each: equal keys
+// of the blocks before come first, of those after last.  `per` slots a block.
+// Over an iteration that merges it costs nothing at 1,023 particles and 12 us at
+// 16,384.  An iteration of 9,000 / 12,000 / 16,384 particles that nearly all move:
+// 36 / 38 / 44 us (as a graph with the radix sort about 60 at any of them; comparing
+// every key with every other 433 / 572 / 758).
+template <int PREC>
+__device__ __forceinline__ void resident_sort(const StepArgs& a, ResidentShared<PREC>& sh, uint32_t per, uint32_t i0,
+                                              uint32_t i1, uint32_t epoch) {
+  const uint32_t n = (uint32_t)a.n, C = gridDim.x, cta = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  constexpr uint32_t kEach = kResidentSortKeys / kResidentThreads;  // keys a thread at most
+  auto& so = sh.sort;
+  uint32_t run = 32;  // of a block; missing keys are kNoIndex, which no key reaches
+  while (run < per) run <<= 1;
+  uint32_t key[kEach], at[kEach];
+  __syncthreads();  // the merge's use of the shared memory
+#pragma unroll
+  for (uint32_t u = 0; u < kEach; ++u) {
+    const uint32_t q = u * kResidentThreads + tid;
+    if (q >= run) break;  // (whole warps)
+    key[u] = i0 + q < i1 ? a.keyB[i0 + q] : kNoIndex;
+    uint32_t before = 0;
+    for (uint32_t l = 0; l < 32; ++l) {
+      const uint32_t k = __shfl_sync(0xffffffffu, key[u], l);
+      before += k < key[u] || (k == key[u] && l < lane);
+    }
+    at[u] = (q & ~31u) + before;
+    so.key[at[u]] = key[u];
+  }
+  __syncthreads();
+  for (uint32_t w = 32; w < run; w <<= 1) {
+#pragma unroll
+    for (uint32_t u = 0; u < kEach; ++u) {
+      if (u * kResidentThreads + tid >= run) break;
+      const uint32_t other = (at[u] & ~(w - 1u)) ^ w;
+      const uint32_t before = keys_before(so.key + other, w, key[u], (at[u] & w) != 0);
+      at[u] = (at[u] & ~(2u * w - 1u)) + (at[u] & (w - 1u)) + before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t u = 0; u < kEach; ++u)
+      if (u * kResidentThreads + tid < run) so.key[at[u]] = key[u];
+    __syncthreads();
+  }
+#pragma unroll
+  for (uint32_t u = 0; u < kEach; ++u)
+    if (u * kResidentThreads + tid < run) so.slot[at[u]] = (uint16_t)(u * kResidentThreads + tid);
   cluster_barrier();
+  for (uint32_t q = tid; q < C * run / 4; q += kResidentThreads)
+    reinterpret_cast<uint4*>(so.all)[q] = ld_block(so.key + (4 * q & (run - 1u)), 4 * q / run);
+  __syncthreads();
+  for (uint32_t q = tid; q < i1 - i0; q += kResidentThreads) {  // in sorted order: a warp's bisections stay close
+    const uint32_t k = so.key[q], i = i0 + so.slot[q];
+    uint32_t rank = q;
+#pragma unroll 4
+    for (uint32_t c = 0; c < C; ++c)
+      if (c != cta) rank += keys_before(so.all + c * run, run, k, c < cta);
+    const float2 v = a.velB[i];
+    a.keyA[rank] = k;
+    a.perm[rank] = i;
+    a.posA[rank] = a.posB[i];
+    a.velpA[rank] = make_float4(v.x, v.y, 0.f, 0.f);
+    if (a.track_ids) a.idsA[rank] = a.idsB[i];
+  }
+  cluster_barrier();  // (and no block's keys are read any more)
   uint32_t* r = reinterpret_cast<uint32_t*>(a.ranges);
   for (uint32_t i = i0 + tid; i < i1; i += kResidentThreads) {
     const uint32_t k = a.keyA[i];
@@ -1356,7 +1416,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     }
     if (!merge) {
       if (cta == 0 && tid == 0) *m.epoch = epoch;
-      resident_sort<PREC>(a, sh, i0, i1, epoch);
+      resident_sort<PREC>(a, sh, per, i0, i1, epoch);
     }
     // the header of the iteration before: by the block with the least of the merge
     if (headers && it > 0 && cta == C - 1 && tid >= kResidentThreads - kDiagThreads)
