@@ -1374,7 +1374,7 @@ static sphg_status export_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_
   }
   if (!s->exp_offs) {
     if (cudaMalloc((void**)&s->exp_offs, (size_t)(n + 1) * sizeof(int64_t)) != cudaSuccess ||
-        (!s->htotal && cudaMallocHost((void**)&s->htotal, sizeof(int64_t)) != cudaSuccess)) {
+        (!s->htotal && cudaMallocHost((void**)&s->htotal, 2 * sizeof(int64_t)) != cudaSuccess)) {
       cudaGetLastError();
       return fail(SPHG_OOM, "neighbour-list buffers");
     }
@@ -1394,6 +1394,8 @@ static sphg_status export_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_
   sphg::ListArgs l = list_args(s);
   l.offs = s->exp_offs;
   l.total = s->htotal;
+  l.err = reinterpret_cast<uint32_t*>(s->htotal + 1);  // the export's own: the state is not touched
+  *(volatile uint32_t*)l.err = 0u;
   int64_t tot = 0;
   for (int round = 0; round < 2; ++round) {
     l.idx = idx ? s->exp_idx : nullptr;
@@ -1401,6 +1403,8 @@ static sphg_status export_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_
     SPHG_CUDA(sphg::launch_lists(s->args(), s->opt.precision, form, l, st));
     if (round == 0 && offs) SPHG_TRY(copy_out(s, offs, s->exp_offs, (size_t)(n + 1) * sizeof(int64_t), st));
     SPHG_CUDA(cudaStreamSynchronize(st));
+    if (*(volatile uint32_t*)l.err)
+      return fail(SPHG_TIMEOUT, "a look-back wait of the neighbour lists gave up; the lists are not valid");
     tot = *(volatile int64_t*)s->htotal;
     if (!idx || tot <= l.cap) break;
     SPHG_TRY(grow(tot));

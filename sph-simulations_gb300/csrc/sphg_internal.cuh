@@ -95,7 +95,7 @@ struct sphg_sim {
   // pinned words the device reports in: [0, kErrorWords) error words, then the
   // upload's "a value is not finite"
   uint32_t* hwords = nullptr;
-  int64_t* htotal = nullptr;  // pinned: entries of the exported lists
+  int64_t* htotal = nullptr;  // pinned: entries of the exported lists, and whether their look-back gave up
   double* hcfl = nullptr;  // pinned: max |v|^2, max |a|^2 of each instance
   // pinned host staging of upload/download (grows on demand)
   char* hstage = nullptr;

@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kListThreads) lists_assemble(StepArgs a, ListA
       t -= r;
       if (r == 0) {
         if (++spins > kListSpinLimit) {  // give up: flag the error
-          if (lane == 0) atomicExch(o.err, 1u);
+          if (lane == 0) *(volatile uint32_t*)o.err = 1u;
           break;
         }
         __nanosleep(32);

@@ -93,8 +93,8 @@ cudaError_t launch_force(const StepArgs& a, int precision, int mode, cudaStream_
 // offs: n + 1 entries; idx: entries of the lists in `form`, at most cap (null:
 // offsets and total only); *overflow set when they would be more; total
 // (device-accessible) or null.  words: lists_blocks(n), ctl: 4 words, both zero
-// before the first launch and not shared between launches that overlap; *err set
-// when a look-back wait gave up.
+// before the first launch and not shared between launches that overlap; *err
+// (device-accessible) set when a look-back wait gave up.
 enum ListForm { kListIndices = 0, kListPacked = 1, kListCoded = 2 };  // j; j << 5 | tag; ascending, delta-coded
 struct ListArgs {
   int64_t* offs;

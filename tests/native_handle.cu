@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "../include/sphg.h"
+#include "../sph-simulations_gb300/csrc/sphg_internal.cuh"
 
 // A kernel's attributes belong to the device that was current when they were set.
 // With one device at hand the program plays two: it keeps, by the device it plays,
@@ -93,11 +94,59 @@ int devices() {
   return 0;
 }
 
+struct Lists {
+  std::vector<int64_t> offs;
+  std::vector<int32_t> idx;
+  int64_t total = 0;
+  sphg_status count(sphg_sim* s) { return sphg_neighbor_lists(s, nullptr, nullptr, &total, nullptr); }
+  sphg_status get(sphg_sim* s, int64_t n) {
+    sphg_status st = count(s);
+    if (st != SPHG_OK) return st;
+    offs.assign(n + 1, -1);
+    idx.assign(total, -1);
+    return sphg_neighbor_lists(s, offs.data(), idx.data(), &total, nullptr);
+  }
+};
+// A computed state of n = 200 particles: two blocks of the list assembly.
+constexpr int64_t kListN = 200;
+sphg_sim* list_handle() {
+  const State st = lattice(20, 10);
+  const sphg_params p = box(0.12);
+  sphg_sim* s = nullptr;
+  if (sphg_create(&p, nullptr, kListN, &s) != SPHG_OK ||
+      sphg_upload(s, st.x.data(), st.y.data(), st.vx.data(), st.vy.data(), nullptr) != SPHG_OK ||
+      sphg_preloop(s, nullptr) != SPHG_OK)
+    std::exit(failed("handle"));
+  return s;
+}
+
+// The assembly's blocks take the numbers 1 and 2 instead of 0 and 1 (its words are
+// padded to 256 bytes), so their look-back waits for a block that never comes and
+// gives up: the export says so, the state and the next export are as they were.
+int lookback() {
+  sphg_sim* s = list_handle();
+  Lists a, b, c;
+  if (a.get(s, kListN) != SPHG_OK) return failed("export");
+  const uint32_t one = 1;
+  if (cudaMemcpy(s->list_ctl, &one, sizeof(one), cudaMemcpyHostToDevice) != cudaSuccess) return failed("copy");
+  b.offs.assign(kListN + 1, -1);
+  b.idx.assign(a.total, -1);
+  if (sphg_neighbor_lists(s, b.offs.data(), b.idx.data(), &b.total, nullptr) != SPHG_TIMEOUT)
+    return failed("a wait that gave up is not reported");
+  if (c.get(s, kListN) != SPHG_OK) return failed("the next export");
+  if (c.offs != a.offs || c.idx != a.idx) return failed("the next export is another");
+  std::vector<double> x(kListN);
+  if (sphg_download(s, x.data(), nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr) != SPHG_OK)
+    return failed("the state after it");
+  return sphg_destroy(s);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "devices") return devices();
+  if (check == "lookback") return lookback();
   std::printf("unknown check\n");
   return 2;
 }

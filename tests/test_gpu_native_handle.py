@@ -33,3 +33,9 @@ def test_small_handles_on_a_second_device(program):
     handle made on another one (played by the program's wrapped calls) runs too,
     with the same bits."""
     _check(program, "devices")
+
+
+def test_an_export_reports_its_own_timeout(program):
+    """A look-back wait of the neighbour lists that gives up (bounded, a few seconds)
+    is the export's error, not the state's."""
+    _check(program, "lookback")
