@@ -1372,12 +1372,10 @@ static sphg_status export_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_
     if (offs) offs[0] = 0;
     return SPHG_OK;
   }
-  if (!s->exp_offs) {
-    if (cudaMalloc((void**)&s->exp_offs, (size_t)(n + 1) * sizeof(int64_t)) != cudaSuccess ||
-        (!s->htotal && cudaMallocHost((void**)&s->htotal, 2 * sizeof(int64_t)) != cudaSuccess)) {
-      cudaGetLastError();
-      return fail(SPHG_OOM, "neighbour-list buffers");
-    }
+  if ((!s->exp_offs && cudaMalloc((void**)&s->exp_offs, (size_t)(n + 1) * sizeof(int64_t)) != cudaSuccess) ||
+      (!s->htotal && cudaMallocHost((void**)&s->htotal, 2 * sizeof(int64_t)) != cudaSuccess)) {
+    cudaGetLastError();
+    return fail(SPHG_OOM, "neighbour-list buffers");
   }
   auto grow = [&](int64_t entries) -> sphg_status {
     if (entries <= s->exp_cap) return SPHG_OK;

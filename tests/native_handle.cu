@@ -17,7 +17,7 @@
 // A kernel's attributes belong to the device that was current when they were set.
 // With one device at hand the program plays two: it keeps, by the device it plays,
 // which kernels may use more than 48 KB of shared memory, and refuses the launches
-// that the device would refuse (linked with --wrap of the two calls).
+// that the device would refuse (the program is linked with --wrap of the calls it replaces).
 static int fake_device = 0;
 static std::set<std::pair<int, const void*>> large_memory;
 extern "C" cudaError_t __real_cudaFuncSetAttribute(const void* f, cudaFuncAttribute attr, int value);
@@ -29,6 +29,12 @@ extern "C" cudaError_t __real_cudaLaunchKernelExC(const cudaLaunchConfig_t* c, c
 extern "C" cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
   if (c->dynamicSmemBytes > (48u << 10) && !large_memory.count({fake_device, f})) return cudaErrorInvalidValue;
   return __real_cudaLaunchKernelExC(c, f, args);
+}
+// Allocations that fail on request: the next `refuse_pinned` pinned ones.
+static int refuse_pinned = 0;
+extern "C" cudaError_t __real_cudaMallocHost(void** p, size_t bytes);
+extern "C" cudaError_t __wrap_cudaMallocHost(void** p, size_t bytes) {
+  return refuse_pinned-- > 0 ? cudaErrorMemoryAllocation : __real_cudaMallocHost(p, bytes);
 }
 
 namespace {
@@ -141,12 +147,25 @@ int lookback() {
   return sphg_destroy(s);
 }
 
+// The first export gets its device buffer but not its pinned one; the second both.
+int pinned() {
+  sphg_sim* s = list_handle();
+  Lists a;
+  refuse_pinned = 1;
+  if (a.count(s) != SPHG_OOM) return failed("an allocation that failed is not reported");
+  refuse_pinned = 0;
+  if (a.get(s, kListN) != SPHG_OK) return failed("the export after it");
+  if (a.total < kListN || a.offs[kListN] != a.total) return failed("its lists");
+  return sphg_destroy(s);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "devices") return devices();
   if (check == "lookback") return lookback();
+  if (check == "pinned") return pinned();
   std::printf("unknown check\n");
   return 2;
 }

@@ -17,7 +17,8 @@ def program(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("native") / "native_handle")
     objs = sorted(glob.glob(os.path.join(B.BUILD, "*.cu.o")))
     assert objs, "the library's objects are not built"
-    wrap = ["-Xlinker", "--wrap=cudaFuncSetAttribute,--wrap=cudaLaunchKernelExC"]
+    wrap = ["-Xlinker", ",".join("--wrap=" + f for f in ("cudaFuncSetAttribute", "cudaLaunchKernelExC",
+                                                         "cudaMallocHost"))]
     subprocess.check_call([B.nvcc()] + B.NVCC_FLAGS + [os.path.join(HERE, "native_handle.cu")] + objs + wrap +
                           ["-o", exe])
     return exe
@@ -39,3 +40,8 @@ def test_an_export_reports_its_own_timeout(program):
     """A look-back wait of the neighbour lists that gives up (bounded, a few seconds)
     is the export's error, not the state's."""
     _check(program, "lookback")
+
+
+def test_an_export_after_a_failed_allocation(program):
+    """The export's two buffers are had one by one: the next call gets the missing one."""
+    _check(program, "pinned")
