@@ -1377,17 +1377,17 @@ static sphg_status export_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_
     cudaGetLastError();
     return fail(SPHG_OOM, "neighbour-list buffers");
   }
-  auto grow = [&](int64_t entries) -> sphg_status {
-    if (entries <= s->exp_cap) return SPHG_OK;
-    if (s->exp_idx) SPHG_CUDA(cudaFree(s->exp_idx));
+  auto grow = [&](int64_t entries) {
+    if (entries <= s->exp_cap) return true;
+    if (s->exp_idx) cudaFree(s->exp_idx);
     s->exp_idx = nullptr;
     s->exp_cap = 0;
     if (cudaMalloc((void**)&s->exp_idx, (size_t)entries * sizeof(uint32_t)) != cudaSuccess) {
       cudaGetLastError();
-      return fail(SPHG_OOM, "neighbour-list buffers");
+      return false;
     }
     s->exp_cap = entries;
-    return SPHG_OK;
+    return true;
   };
   sphg::ListArgs l = list_args(s);
   l.offs = s->exp_offs;
@@ -1405,10 +1405,13 @@ static sphg_status export_lists(sphg_sim* s, int64_t* offs, int32_t* idx, int64_
       return fail(SPHG_TIMEOUT, "a look-back wait of the neighbour lists gave up; the lists are not valid");
     tot = *(volatile int64_t*)s->htotal;
     if (!idx || tot <= l.cap) break;
-    SPHG_TRY(grow(tot));
+    if (!grow(tot)) return fail(SPHG_OOM, "neighbour-list buffers");
   }
   if (total) *total = tot;
-  if (!idx) return grow(tot);  // for the call that asks for the entries
+  if (!idx) {
+    grow(tot);  // for the call that asks for the entries, which reports it when there is no room
+    return SPHG_OK;
+  }
   if (tot > 0) {
     SPHG_TRY(copy_out(s, idx, s->exp_idx, (size_t)tot * sizeof(int32_t), st));
     SPHG_CUDA(cudaStreamSynchronize(st));

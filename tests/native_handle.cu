@@ -30,11 +30,17 @@ extern "C" cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t* c, c
   if (c->dynamicSmemBytes > (48u << 10) && !large_memory.count({fake_device, f})) return cudaErrorInvalidValue;
   return __real_cudaLaunchKernelExC(c, f, args);
 }
-// Allocations that fail on request: the next `refuse_pinned` pinned ones.
+// Allocations that fail on request: the next `refuse_pinned` pinned ones, and device
+// ones after the next `allow_device`.
 static int refuse_pinned = 0;
 extern "C" cudaError_t __real_cudaMallocHost(void** p, size_t bytes);
 extern "C" cudaError_t __wrap_cudaMallocHost(void** p, size_t bytes) {
   return refuse_pinned-- > 0 ? cudaErrorMemoryAllocation : __real_cudaMallocHost(p, bytes);
+}
+static int allow_device = 1 << 30;
+extern "C" cudaError_t __real_cudaMalloc(void** p, size_t bytes);
+extern "C" cudaError_t __wrap_cudaMalloc(void** p, size_t bytes) {
+  return allow_device-- <= 0 ? cudaErrorMemoryAllocation : __real_cudaMalloc(p, bytes);
 }
 
 namespace {
@@ -159,6 +165,21 @@ int pinned() {
   return sphg_destroy(s);
 }
 
+// A call for the total needs no room for the entries.
+int count_only() {
+  sphg_sim* s = list_handle();
+  Lists a;
+  allow_device = 1;  // the offsets
+  if (a.count(s) != SPHG_OK || a.total < kListN) return failed("the total");
+  a.idx.assign(a.total, -1);
+  if (sphg_neighbor_lists(s, nullptr, a.idx.data(), &a.total, nullptr) != SPHG_OOM)
+    return failed("an allocation that failed is not reported");
+  allow_device = 1 << 30;
+  if (a.get(s, kListN) != SPHG_OK) return failed("the export after it");
+  if (a.offs[kListN] != a.total || a.idx[a.total - 1] < 0) return failed("its lists");
+  return sphg_destroy(s);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -166,6 +187,7 @@ int main(int argc, char** argv) {
   if (check == "devices") return devices();
   if (check == "lookback") return lookback();
   if (check == "pinned") return pinned();
+  if (check == "count_only") return count_only();
   std::printf("unknown check\n");
   return 2;
 }

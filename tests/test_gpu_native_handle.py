@@ -18,7 +18,7 @@ def program(tmp_path_factory):
     objs = sorted(glob.glob(os.path.join(B.BUILD, "*.cu.o")))
     assert objs, "the library's objects are not built"
     wrap = ["-Xlinker", ",".join("--wrap=" + f for f in ("cudaFuncSetAttribute", "cudaLaunchKernelExC",
-                                                         "cudaMallocHost"))]
+                                                         "cudaMallocHost", "cudaMalloc"))]
     subprocess.check_call([B.nvcc()] + B.NVCC_FLAGS + [os.path.join(HERE, "native_handle.cu")] + objs + wrap +
                           ["-o", exe])
     return exe
@@ -45,3 +45,9 @@ def test_an_export_reports_its_own_timeout(program):
 def test_an_export_after_a_failed_allocation(program):
     """The export's two buffers are had one by one: the next call gets the missing one."""
     _check(program, "pinned")
+
+
+def test_a_total_without_room_for_the_entries(program):
+    """The call for the total succeeds when the entries' buffer cannot be had; the
+    one that asks for the entries reports it."""
+    _check(program, "count_only")
