@@ -931,12 +931,19 @@ sphg_status sphg_create(const sphg_params* p, const sphg_options* o, int64_t n, 
 
 sphg_status sphg_destroy(sphg_sim* s) { return destroy_impl(s); }
 
+// Whether the device may read or write a caller's array in place: at its entries'
+// natural alignment (a packed buffer may hold it at any address, which only host
+// code reaches).
+static bool in_place(const void* p, size_t entry) { return reinterpret_cast<uintptr_t>(p) % entry == 0; }
+
 sphg_status sphg_upload(sphg_sim* s, const double* x, const double* y, const double* vx,
                         const double* vy, void* stream) {
   if (!s || (s->n > 0 && (!x || !y || !vx || !vy))) return fail(SPHG_INVALID_ARG, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t n = s->n;
-  if (n > 0 && s->host_direct) {
+  const bool direct = s->host_direct != 0 && in_place(x, sizeof(double)) && in_place(y, sizeof(double)) &&
+                      in_place(vx, sizeof(double)) && in_place(vy, sizeof(double));
+  if (n > 0 && direct) {
     volatile uint32_t* any_bad = s->hwords + sphg::kErrorWords;
     *any_bad = 0u;
     SPHG_CUDA(sphg::launch_upload_direct(s->args(), s->opt.precision, x, y, vx, vy, s->flags + 6,
@@ -1045,11 +1052,6 @@ static sphg_status device_errors(sphg_sim* s, cudaStream_t st) {
   SPHG_CUDA(cudaStreamSynchronize(st));
   return report(w);
 }
-
-// Whether the device may write a caller's array in place: at its entries' natural
-// alignment (a packed buffer may hold it at any address, which only host code
-// reaches).
-static bool in_place(const void* p, size_t entry) { return reinterpret_cast<uintptr_t>(p) % entry == 0; }
 
 // Makes the pages of the caller's result arrays resident, so that the device's
 // writes that follow find them mapped: a device write into a page the host has
@@ -1225,6 +1227,7 @@ sphg_status sphg_set_dt(sphg_sim* s, int32_t inst, double dt) {
 // host memory (mapped under unified addressing), or -- when host access is on
 // and the device reads and writes pageable memory -- the array itself.
 static double* device_view(sphg_sim* s, double* out) {
+  if (!in_place(out, sizeof(double))) return nullptr;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, out) != cudaSuccess) {
     cudaGetLastError();

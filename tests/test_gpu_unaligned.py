@@ -64,3 +64,43 @@ def test_neighbour_lists(by):
                                         i.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), ctypes.byref(total), None))
     assert total.value == len(idx) and np.array_equal(o, offs) and np.array_equal(i, idx)
     sim.close()
+
+
+@pytest.mark.parametrize("prec", ["plain", "split"])
+@pytest.mark.parametrize("by", [1, 4])
+def test_upload(by, prec):
+    import sphg as S
+    n = 1001
+    sim, state = _sim(S, n, prec)
+    sim.set_host_access(0)
+    sim.upload(*state)
+    sim.preloop()
+    want = sim.download()
+    sim.set_host_access(1)
+    for odd in range(4):
+        arrays = list(state)
+        arrays[odd] = _unaligned(n, np.float64, by)
+        arrays[odd][:] = state[odd]
+        sim.upload(*arrays)
+        sim.preloop()
+        got = sim.download()
+        for k in want:
+            assert np.array_equal(got[k], want[k]), (odd, k)
+    sim.close()
+
+
+@pytest.mark.parametrize("by", [1, 4])
+def test_headers(by):
+    import sphg as S
+    n = 1001
+    sim, state = _sim(S, n, "split")
+    want = sim.step_headers(5)
+    sim.upload(*state)
+    sim.preloop()
+    got = _unaligned(5 * 6, np.float64, by)
+    sim.step_headers(5, out=got)
+    one = _unaligned(6, np.float64, by)
+    sim.diagnostics_async(one.ctypes.data)
+    sim.diagnostics()  # waits
+    assert np.array_equal(got, want.ravel()) and np.array_equal(one, want.ravel()[-6:])
+    sim.close()
