@@ -150,8 +150,8 @@ sphg_status sphg_device_attributes(int32_t device, int32_t* out);
  *      pages (the default when the device can access pageable host memory);
  *   2: the same without touching the pages (writes into pages the host never
  *      touched fault them in one by one).
- * The results are the same.  A download that returns an error leaves the arrays'
- * contents undefined. */
+ * The results are the same.  A download that reports a state that is not valid
+ * leaves the FP64 arrays as they were (and the indices, in modes 1 and 2). */
 sphg_status sphg_set_host_access(sphg_sim* s, int32_t mode);
 
 /* One instance of n particles. */

@@ -30,10 +30,17 @@ __device__ __forceinline__ double floor_div(double t, double cs, double inv_cs) 
   return floor(__ddiv_rn(t, cs));
 }
 
-// The error words of the device state into the handle's pinned block (one
-// thread; the host reads them after the synchronisation that ends the call).
-__device__ __forceinline__ void report_errors(const HostErrors& e) {
-  for (int k = 0; k < kErrorWords; ++k) e.out[k] = *e.word[k];
+// Whether the state is valid by its error words, which go into the handle's pinned
+// block (the host reads them after the synchronisation that ends the call).
+__device__ __forceinline__ bool state_valid(const HostErrors& e, bool report) {
+  bool valid = true;
+#pragma unroll
+  for (int k = 0; k < kErrorWords; ++k) {
+    const uint32_t w = *e.word[k];
+    valid = valid && w == 0u;
+    if (report) e.out[k] = w;
+  }
+  return valid;
 }
 
 // An FP64 position as its cell (clamped to [0, cmax]) and FP32 offset in it.
@@ -171,7 +178,7 @@ __global__ void download_direct_kernel(StepArgs a, int precision, double* __rest
                                        double* __restrict__ rho, double* __restrict__ fx,
                                        double* __restrict__ fy, int32_t* __restrict__ ids, HostErrors errors) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t == 0) report_errors(errors);
+  if (!state_valid(errors, t == 0)) return;  // the call fails: the arrays stay as they are
   auto write = [&](auto* out, auto&& value) {
     if (!out) return;
     const int64_t i = line_entry(out, t);
