@@ -1294,49 +1294,42 @@ __device__ __forceinline__ uint32_t keys_before(const uint32_t* keys, uint32_t r
 // of the blocks before come first, of those after last.  `per` slots a block.
 // Over an iteration that merges it costs nothing at 1,023 particles and 12 us at
 // 16,384.  An iteration of 9,000 / 12,000 / 16,384 particles that nearly all move:
-// 36 / 38 / 44 us (as a graph with the radix sort about 60 at any of them; comparing
-// every key with every other 433 / 572 / 758).
+// 35 / 38 / 43 us (as a graph with the radix sort about 60 at any of them; comparing
+// every key with every other 433 / 572 / 758).  The keys stay in shared memory
+// between the steps: held in registers they made the merging iterations, which never
+// come here, up to 2 % slower (spills around this code).
 template <int PREC>
 __device__ __forceinline__ void resident_sort(const StepArgs& a, ResidentShared<PREC>& sh, uint32_t per, uint32_t i0,
                                               uint32_t i1, uint32_t epoch) {
   const uint32_t n = (uint32_t)a.n, C = gridDim.x, cta = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-  constexpr uint32_t kEach = kResidentSortKeys / kResidentThreads;  // keys a thread at most
   auto& so = sh.sort;
   uint32_t run = 32;  // of a block; missing keys are kNoIndex, which no key reaches
-  while (run < per) run <<= 1;
-  uint32_t key[kEach], at[kEach];
+  bool there = true;  // the runs lie in so.key and so.slot (the last ones), or beside them
+  for (; run < per; run <<= 1) there = !there;
+  uint32_t* const other_key = so.all;  // not in use before the copies
+  uint16_t* const other_slot = reinterpret_cast<uint16_t*>(so.all + kResidentSortKeys);
   __syncthreads();  // the merge's use of the shared memory
-#pragma unroll
-  for (uint32_t u = 0; u < kEach; ++u) {
-    const uint32_t q = u * kResidentThreads + tid;
-    if (q >= run) break;  // (whole warps)
-    key[u] = i0 + q < i1 ? a.keyB[i0 + q] : kNoIndex;
-    uint32_t before = 0;
+  for (uint32_t q = tid; q < run; q += kResidentThreads) {  // (whole warps)
+    const uint32_t k = i0 + q < i1 ? a.keyB[i0 + q] : kNoIndex;
+    uint32_t at = q & ~31u;
     for (uint32_t l = 0; l < 32; ++l) {
-      const uint32_t k = __shfl_sync(0xffffffffu, key[u], l);
-      before += k < key[u] || (k == key[u] && l < lane);
+      const uint32_t v = __shfl_sync(0xffffffffu, k, l);
+      at += v < k || (v == k && l < lane);
     }
-    at[u] = (q & ~31u) + before;
-    so.key[at[u]] = key[u];
+    (there ? so.key : other_key)[at] = k;
+    (there ? so.slot : other_slot)[at] = (uint16_t)q;
   }
-  __syncthreads();
-  for (uint32_t w = 32; w < run; w <<= 1) {
-#pragma unroll
-    for (uint32_t u = 0; u < kEach; ++u) {
-      if (u * kResidentThreads + tid >= run) break;
-      const uint32_t other = (at[u] & ~(w - 1u)) ^ w;
-      const uint32_t before = keys_before(so.key + other, w, key[u], (at[u] & w) != 0);
-      at[u] = (at[u] & ~(2u * w - 1u)) + (at[u] & (w - 1u)) + before;
+  for (uint32_t w = 32; w < run; w <<= 1, there = !there) {
+    __syncthreads();
+    const uint32_t* from = there ? so.key : other_key;
+    for (uint32_t q = tid; q < run; q += kResidentThreads) {
+      const uint32_t k = from[q];
+      const uint32_t at = (q & ~(2u * w - 1u)) + (q & (w - 1u)) +
+                          keys_before(from + ((q & ~(w - 1u)) ^ w), w, k, (q & w) != 0);
+      (there ? other_key : so.key)[at] = k;
+      (there ? other_slot : so.slot)[at] = (there ? so.slot : other_slot)[q];
     }
-    __syncthreads();
-#pragma unroll
-    for (uint32_t u = 0; u < kEach; ++u)
-      if (u * kResidentThreads + tid < run) so.key[at[u]] = key[u];
-    __syncthreads();
   }
-#pragma unroll
-  for (uint32_t u = 0; u < kEach; ++u)
-    if (u * kResidentThreads + tid < run) so.slot[at[u]] = (uint16_t)(u * kResidentThreads + tid);
   cluster_barrier();
   for (uint32_t q = tid; q < C * run / 4; q += kResidentThreads)
     reinterpret_cast<uint4*>(so.all)[q] = ld_block(so.key + (4 * q & (run - 1u)), 4 * q / run);
@@ -1344,7 +1337,7 @@ __device__ __forceinline__ void resident_sort(const StepArgs& a, ResidentShared<
   for (uint32_t q = tid; q < i1 - i0; q += kResidentThreads) {  // in sorted order: a warp's bisections stay close
     const uint32_t k = so.key[q], i = i0 + so.slot[q];
     uint32_t rank = q;
-#pragma unroll 4
+#pragma unroll 1
     for (uint32_t c = 0; c < C; ++c)
       if (c != cta) rank += keys_before(so.all + c * run, run, k, c < cta);
     const float2 v = a.velB[i];
