@@ -98,7 +98,7 @@ __device__ __forceinline__ void record_movers(const StepArgs& a, uint32_t i, uin
         atomicSub(r.sup_net + (bi >> kMergeSupShift), 1);
       }
     }
-    if (before >= (uint32_t)kGroupCap - 1u || in_block >= (uint32_t)kBlockInsertCap - 1u) r.total[1] = 1u;
+    if (before >= (uint32_t)kGroupCap || in_block >= (uint32_t)kBlockInsertCap) r.total[1] = 1u;
   }
 }
 
