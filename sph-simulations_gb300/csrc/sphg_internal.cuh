@@ -85,6 +85,7 @@ struct sphg_sim {
   uint64_t cap_keys = 0;        // arena capacity (cell keys)
   int cap_inst = 0;             // arena capacity (instances)
   int force_batched = 0;        // always use the per-instance-descriptor kernels
+  uint64_t serial = 0;          // number of the handle among those made by sphg_create*
   int resident = 0;             // blocks of the cluster its iterations run in (0: graphs)
   int tile_bits = 0, tile_cap = 0, tile_grid = 0;
   bool uploaded = false, preloop_done = false;
