@@ -313,12 +313,11 @@ def device_record(name, args, opts, stream, steps, warmup, with_e2e=True, world=
     clk = clocks.stop()
     total_ms = max_over_ranks(total_ms)
     value = replica_throughput(n, world, steps, total_ms)
-    full_sort_kernels = int(sim.debug(sphg.DBG_RESORT, stream=sptr)[2])
-    per_step = sim.launches_per_step()
+    saved = int(sim.debug(sphg.DBG_RESORT, stream=sptr)[2])
     rs = resort_summary(log)
+    launches = steps * sim.launches_per_step() - (rs["steps"] - rs["full_sorts"]) * saved
     if opts.compute == sphg.LISTS:
-        per_step -= 4  # the lists are assembled in one kernel of the five the library counts for them
-    launches = int(round(steps * per_step - (rs["steps"] * rs["merged_fraction"]) * full_sort_kernels))
+        launches -= 3 * rs["full_sorts"]  # two list kernels where the library counts five
     # per-phase profile (CUDA events between the kernels of one iteration)
     phases = np.array([sim.profile_step(stream=sptr) for _ in range(10)])
     names = ["keys", "sort", "reorder", "density", "force_integrate"]

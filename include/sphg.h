@@ -230,7 +230,7 @@ enum {
   SPHG_DBG_VEL_NEXT = 4,    /* double[2n] integrated velocities awaiting the next sort */
   SPHG_DBG_RESORT = 5       /* int32[3]  last iteration: 1 if the incremental re-sort ran
                                (0: the full radix sort), particles that changed cell,
-                               kernels of a full sort (histogram + radix passes) */
+                               kernel launches that an iteration that merges saves */
 };
 sphg_status sphg_get_debug(sphg_sim* s, int32_t which, void* host, void* stream);
 
@@ -330,9 +330,11 @@ sphg_status sphg_autotune(int32_t ninst, const sphg_params* p, const int64_t* co
  * phases; ms[0..4] = keys, sort, reorder (+cell ranges), density, force+integrate
  * (milliseconds, summed over the instances of the handle). */
 sphg_status sphg_profile_step(sphg_sim* s, float* ms, void* stream);
-/* Kernel launches of a main-loop iteration that runs the full sort (an upper
- * bound in the lists mode and for small single instances, which launch fewer);
- * in a graph, an iteration that merges launches SPHG_DBG_RESORT[2] fewer. */
+/* Kernel launches of a main-loop iteration that runs the full sort; one that merges
+ * launches SPHG_DBG_RESORT[2] fewer.  In the lists mode five are counted for its list
+ * kernel, three or four more than an iteration that sorts fully launches; a small
+ * single instance (see use_graph) needs one launch for up to 128 iterations, however
+ * they sort. */
 int32_t sphg_launches_per_step(const sphg_sim* s);
 
 /* Stand-alone kernels on caller-owned DEVICE buffers. */

@@ -1330,6 +1330,36 @@ sphg_status sphg_step_headers(sphg_sim* s, int64_t nsteps, double* out, void* st
   return SPHG_OK;
 }
 
+// Kernels launched for an iteration that sorts fully, and for one that merges.
+struct LaunchCounts {
+  int full, merged;
+};
+static LaunchCounts launch_counts(const sphg_sim* s) {
+  const int radix = 1 + (s->key_bits + 7) / 8;  // histogram, passes
+  const bool branch = s->movers_on && s->opt.use_graph && s->cond_graph;
+  LaunchCounts c;
+  if (fused_on(const_cast<sphg_sim*>(s))) {
+    // the launch (which only decides when it does not merge), the sort, the launch's post part
+    c.full = 1 + radix + 1;
+    c.merged = branch ? 1 : c.full;
+    return c;
+  }
+  // the merge, density and forces; the sort and the reorder, with density and forces
+  // of their own where a graph keeps them in a branch (those of its chain return at
+  // once), else before the same ones
+  const int merge = s->movers_on ? 1 : 0, work = 2;
+  c.full = merge + radix + 1 + work + (branch ? work : 0);
+  c.merged = branch ? merge + work : c.full;
+  // the list kernel (five are counted for the one or two of an iteration that sorts
+  // fully, as callers have been told)
+  if (s->opt.compute == SPHG_COMPUTE_LISTS) {
+    c.full += 5;
+    c.merged = branch ? c.merged + 1 : c.full;
+  }
+  if (s->resident > 0 && s->n <= sphg::kResidentSingleMaxN) c.merged = 1;  // all of it, up to 128 times
+  return c;
+}
+
 sphg_status sphg_get_debug(sphg_sim* s, int32_t which, void* host, void* stream) {
   if (!s || !host) return fail(SPHG_INVALID_ARG, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
@@ -1353,8 +1383,8 @@ sphg_status sphg_get_debug(sphg_sim* s, int32_t which, void* host, void* stream)
         SPHG_CUDA(cudaMemcpyAsync(c, s->flags + 3, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         SPHG_CUDA(cudaStreamSynchronize(st));
       }
-      // histogram + radix passes of a full sort + the reorder (single-launch iteration: its post part)
-      c[2] = (uint32_t)((s->key_bits + 7) / 8 + 2);
+      const LaunchCounts k = launch_counts(s);
+      c[2] = (uint32_t)(k.full - k.merged);
       std::memcpy(host, c, sizeof(c));
       return SPHG_OK;
     }
@@ -1590,18 +1620,7 @@ sphg_status sphg_profile_step(sphg_sim* s, float* ms, void* stream) {
 
 int32_t sphg_launches_per_step(const sphg_sim* s) {
   if (!s || s->n == 0) return 0;
-  const int passes = (s->key_bits + 7) / 8;
-  // an iteration that runs the full sort: its histogram kernel + radix passes +
-  // reorder + density + force (+ the incremental re-sort's merge kernel).  An
-  // iteration that merges launches (key_bits + 7) / 8 + 2 kernels fewer in a
-  // graph.  An upper bound: the lists mode assembles its lists in one kernel of
-  // the five counted for count, scan and fill, and a small single instance runs
-  // many iterations in one launch.
-  // With the single-launch iteration: the launch (which only decides), the
-  // histogram + radix passes and the launch's post part; an iteration that
-  // merges is the one launch.
-  if (fused_on(const_cast<sphg_sim*>(s))) return passes + 3;
-  return passes + 4 + (s->movers_on ? 1 : 0) + (s->opt.compute == SPHG_COMPUTE_LISTS ? 5 : 0);
+  return launch_counts(s).full;
 }
 
 sphg_status sphg_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,

@@ -19,6 +19,7 @@
 // which kernels may use more than 48 KB of shared memory, and refuses the launches
 // that the device would refuse (the program is linked with --wrap of the calls it replaces).
 static int fake_device = 0;
+static int launched = 0;  // kernels of iterations, captured ones included
 static std::set<std::pair<int, const void*>> large_memory;
 extern "C" cudaError_t __real_cudaFuncSetAttribute(const void* f, cudaFuncAttribute attr, int value);
 extern "C" cudaError_t __wrap_cudaFuncSetAttribute(const void* f, cudaFuncAttribute attr, int value) {
@@ -27,6 +28,7 @@ extern "C" cudaError_t __wrap_cudaFuncSetAttribute(const void* f, cudaFuncAttrib
 }
 extern "C" cudaError_t __real_cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args);
 extern "C" cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
+  ++launched;
   if (c->dynamicSmemBytes > (48u << 10) && !large_memory.count({fake_device, f})) return cudaErrorInvalidValue;
   return __real_cudaLaunchKernelExC(c, f, args);
 }
@@ -180,6 +182,43 @@ int count_only() {
   return sphg_destroy(s);
 }
 
+// The library's counts of launches against those made: graphs hold what their
+// iterations launch when they sort fully.
+int launches() {
+  for (int n1 : {130, 30})  // graphs; one cluster
+    for (int graph : {1, 0})
+      for (int resort : {1, 0}) {
+        const State st = lattice(n1, n1);
+        const sphg_params p = box(1.3 / n1);
+        sphg_options o;
+        sphg_default_options(&o);
+        o.use_graph = graph;
+        o.resort = resort;
+        sphg_sim* s = nullptr;
+        launched = 0;
+        if (sphg_create(&p, &o, (int64_t)n1 * n1, &s) != SPHG_OK) return failed("create");
+        const int made = launched;
+        if (sphg_upload(s, st.x.data(), st.y.data(), st.vx.data(), st.vy.data(), nullptr) != SPHG_OK ||
+            sphg_preloop(s, nullptr) != SPHG_OK)
+          return failed("run");
+        launched = 0;
+        int32_t rs[3];
+        if (sphg_step(s, 1, nullptr) != SPHG_OK || sphg_get_debug(s, SPHG_DBG_RESORT, rs, nullptr) != SPHG_OK)
+          return failed("step");
+        const int full = sphg_launches_per_step(s), merged = full - rs[2];
+        std::printf("%d %d %d: made %d step %d full %d merged %d\n", n1, graph, resort, made, launched, full, merged);
+        if (!graph) {
+          if (launched != full || merged != full) return failed("launches without a graph");
+        } else if (n1 == 130) {  // two graphs, the second with its header (in the branch too)
+          if (made != 2 * full + (resort ? 2 : 1) || merged != (resort ? 3 : full)) return failed("launches of a graph");
+        } else if (resort && (launched != 1 || merged != 1)) {
+          return failed("launches of a cluster");
+        }
+        sphg_destroy(s);
+      }
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -188,6 +227,7 @@ int main(int argc, char** argv) {
   if (check == "lookback") return lookback();
   if (check == "pinned") return pinned();
   if (check == "count_only") return count_only();
+  if (check == "launches") return launches();
   std::printf("unknown check\n");
   return 2;
 }

@@ -51,3 +51,8 @@ def test_a_total_without_room_for_the_entries(program):
     """The call for the total succeeds when the entries' buffer cannot be had; the
     one that asks for the entries reports it."""
     _check(program, "count_only")
+
+
+def test_launch_counts(program):
+    """sphg_launches_per_step and SPHG_DBG_RESORT[2] against the launches made."""
+    _check(program, "launches")
