@@ -1091,12 +1091,13 @@ static sphg_status device_errors(sphg_sim* s, cudaStream_t st) {
 // download that fails leaves them as they were.  (Populated for writing: a page that
 // an instruction reads first, an atomic one included, is mapped to the page of
 // zeros and then copied, small page by small page: a fresh batch's result 97 ms
-// against 12.)
+// against 12.)  Pinned, managed and device memory needs none of it.  False: an array
+// is not mapped at all, nothing was done.
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
 constexpr size_t kTouchBytes = 8u << 20;  // a thread's share at least
-static void touch_pages(void* const (&arrays)[8], const size_t (&bytes)[8]) {
+static bool touch_pages(void* const (&arrays)[8], const size_t (&bytes)[8]) {
   static const size_t page = [] {
     const long p = sysconf(_SC_PAGESIZE);
     return p > 0 ? (size_t)p : (size_t)4096;
@@ -1110,8 +1111,12 @@ static void touch_pages(void* const (&arrays)[8], const size_t (&bytes)[8]) {
     start[k] = reinterpret_cast<char*>(reinterpret_cast<uintptr_t>(arrays[k]) / page * page);
     const size_t len = (size_t)(static_cast<char*>(arrays[k]) + bytes[k] - start[k]);
     map.assign((len + page - 1) / page, 0);
-    const bool known = mincore(start[k], len, map.data()) == 0;
-    if (known && std::all_of(map.begin(), map.end(), [](unsigned char m) { return m & 1; })) continue;
+    const bool mapped = mincore(start[k], len, map.data()) == 0;
+    if (mapped && std::all_of(map.begin(), map.end(), [](unsigned char m) { return m & 1; })) continue;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, arrays[k]) != cudaSuccess) cudaGetLastError();
+    else if (at.type != cudaMemoryTypeUnregistered) continue;
+    if (!mapped) return false;
     first[k + 1] += (int64_t)map.size();
   }
   parallel_for(
@@ -1129,6 +1134,7 @@ static void touch_pages(void* const (&arrays)[8], const size_t (&bytes)[8]) {
         }
       },
       std::max<int64_t>(1, (int64_t)(kTouchBytes / page)));
+  return true;
 }
 
 sphg_status sphg_download(sphg_sim* s, double* x, double* y, double* vx, double* vy, double* rho,
@@ -1140,14 +1146,14 @@ sphg_status sphg_download(sphg_sim* s, double* x, double* y, double* vx, double*
   const bool forces = fx || fy;
   bool direct = s->host_direct != 0 && in_place(ids, sizeof(int32_t));
   for (const double* p : {x, y, vx, vy, rho, fx, fy}) direct = direct && in_place(p, sizeof(double));
+  if (direct && forces) SPHG_CUDA(sphg::launch_force(s->args(), s->opt.precision, sphg::kForceOnly, st));
+  if (direct && s->host_direct == 1) {  // while the device is still at the work enqueued so far
+    void* const arrays[8] = {x, y, vx, vy, rho, fx, fy, ids};
+    size_t bytes[8];
+    for (int k = 0; k < 8; ++k) bytes[k] = (size_t)n * (k < 7 ? sizeof(double) : sizeof(int32_t));
+    direct = touch_pages(arrays, bytes);
+  }
   if (direct) {
-    if (forces) SPHG_CUDA(sphg::launch_force(s->args(), s->opt.precision, sphg::kForceOnly, st));
-    if (s->host_direct == 1) {  // while the device is still at the work enqueued so far
-      void* const arrays[8] = {x, y, vx, vy, rho, fx, fy, ids};
-      size_t bytes[8];
-      for (int k = 0; k < 8; ++k) bytes[k] = (size_t)n * (k < 7 ? sizeof(double) : sizeof(int32_t));
-      touch_pages(arrays, bytes);
-    }
     SPHG_CUDA(sphg::launch_download_direct(s->args(), s->opt.precision, x, y, vx, vy, rho, fx, fy, ids,
                                            host_errors(s), st));
     SPHG_CUDA(cudaStreamSynchronize(st));
@@ -1433,10 +1439,9 @@ sphg_status sphg_get_debug(sphg_sim* s, int32_t which, void* host, void* stream)
 // Device memory into a host array of the caller's, in stream order: written by
 // the device where it reaches the array (its pages touched first), else copied.
 static sphg_status copy_out(sphg_sim* s, void* host, const void* dev, size_t bytes, cudaStream_t st) {
-  if (s->host_direct && in_place(host, sizeof(uint32_t))) {
-    void* const arrays[8] = {host};
-    const size_t sizes[8] = {bytes};
-    touch_pages(arrays, sizes);
+  void* const arrays[8] = {host};
+  const size_t sizes[8] = {bytes};
+  if (s->host_direct && in_place(host, sizeof(uint32_t)) && touch_pages(arrays, sizes)) {
     SPHG_CUDA(sphg::launch_host_copy(static_cast<uint32_t*>(host), static_cast<const uint32_t*>(dev),
                                      (int64_t)(bytes / sizeof(uint32_t)), st));
   } else {
