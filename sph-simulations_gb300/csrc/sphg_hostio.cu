@@ -178,11 +178,13 @@ __global__ void download_direct_kernel(StepArgs a, int precision, double* __rest
                                        double* __restrict__ rho, double* __restrict__ fx,
                                        double* __restrict__ fy, int32_t* __restrict__ ids, HostErrors errors) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (!state_valid(errors, t == 0)) return;  // the call fails: the arrays stay as they are
+  const bool valid = state_valid(errors, t == 0);  // else the call fails: the arrays stay as they are
   auto write = [&](auto* out, auto&& value) {
     if (!out) return;
     const int64_t i = line_entry(out, t);
-    if (i >= 0 && i < a.n) out[i] = value(i);
+    if (i < 0 || i >= a.n) return;
+    const auto v = value(i);  // loaded beside the words
+    if (valid) out[i] = v;
   };
   write(x, [&](int64_t i) { return download_position(a, precision, i, 0); });
   write(y, [&](int64_t i) { return download_position(a, precision, i, 1); });
