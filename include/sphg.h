@@ -332,9 +332,9 @@ sphg_status sphg_autotune(int32_t ninst, const sphg_params* p, const int64_t* co
 sphg_status sphg_profile_step(sphg_sim* s, float* ms, void* stream);
 /* Kernel launches of a main-loop iteration that runs the full sort; one that merges
  * launches SPHG_DBG_RESORT[2] fewer.  In the lists mode five are counted for its list
- * kernel, three or four more than an iteration that sorts fully launches; a small
- * single instance (see use_graph) needs one launch for up to 128 iterations, however
- * they sort. */
+ * kernel, three or four more than an iteration that sorts fully launches.  A small
+ * single instance (see use_graph) is counted as its graph, but needs one launch for up
+ * to 128 iterations, however they sort. */
 int32_t sphg_launches_per_step(const sphg_sim* s);
 
 /* Stand-alone kernels on caller-owned DEVICE buffers. */

@@ -1336,7 +1336,8 @@ sphg_status sphg_step_headers(sphg_sim* s, int64_t nsteps, double* out, void* st
   return SPHG_OK;
 }
 
-// Kernels launched for an iteration that sorts fully, and for one that merges.
+// Kernels launched for an iteration that sorts fully, and for one that merges (of a
+// small instance: if they ran as its graph would).
 struct LaunchCounts {
   int full, merged;
 };
@@ -1362,7 +1363,6 @@ static LaunchCounts launch_counts(const sphg_sim* s) {
     c.full += 5;
     c.merged = branch ? c.merged + 1 : c.full;
   }
-  if (s->resident > 0 && s->n <= sphg::kResidentSingleMaxN) c.merged = 1;  // all of it, up to 128 times
   return c;
 }
 
