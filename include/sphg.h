@@ -338,7 +338,8 @@ sphg_status sphg_profile_step(sphg_sim* s, float* ms, void* stream);
 int32_t sphg_launches_per_step(const sphg_sim* s);
 
 /* Stand-alone kernels on caller-owned DEVICE buffers. */
-/* Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the keys.
+/* Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the keys, in
+ * whole digits of eight (bits = 20 sorts on the low 24).
  * keys_out/vals_out must not alias the inputs; vals_in == NULL sorts the
  * identity 0..n-1.  Buffers need only 4-byte alignment.  n <= 2^30 - 1
  * (SPHG_CAPACITY otherwise).  Scratch is allocated by this call.  Every wait of

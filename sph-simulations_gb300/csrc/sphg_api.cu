@@ -673,8 +673,10 @@ sphg_status alloc_arena(sphg_sim* s, size_t N, uint64_t keys, int ninst, int dia
   // particle with more neighbours walks the stencil again in the force pass, with
   // its warp.  32 slots up to 2^18 particles (slots not needed are never touched:
   // the 6,084-particle example, whose particles gather 15 to 30 neighbours, 41.8 ->
-  // 29.5 us an iteration, others the same); 12 beyond, where 32 measured 0.6 %
-  // slower on the 1M dam break, and in a server's arena, sized for 12.
+  // 29.5 us an iteration, others the same); 12 beyond, for the memory, and in a
+  // server's arena, sized for 12.  12 / 32 slots, plain dam breaks of h = 1.3 dx:
+  // 131,044 particles 26.4 / 26.4, 263,169 35.2 / 35.5, 532,900 55.4 / 55.7, 1,000,000
+  // 92.2 / 92.5 us; of h = 2.2 dx: 50.4 / 39.5, 70.2 / 59.3, 112.8 / 101.3, 189.4 / 173.6.
   s->nbr_slots = (N < ((size_t)1 << 27) && s->opt.compute == SPHG_COMPUTE_SORTED)
                      ? (N <= ((size_t)1 << 18) && !s->force_batched ? 32 : 12) : 0;
   auto layout = [&](Arena& A) {

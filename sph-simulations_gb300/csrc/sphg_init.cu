@@ -143,7 +143,6 @@ extern "C" sphg_status sphg_upload_lattice(sphg_sim* s, const sphg_lattice* spec
     }
     cudaFreeAsync(dspec, st);
     if (e != cudaSuccess) return fail(SPHG_CUDA_ERROR, std::string("lattice generation: ") + cudaGetErrorString(e));
-    // digit histograms of the next sort restart with the generated state
     SPHG_CUDA(cudaStreamSynchronize(st));
   }
   s->uploaded = true;

@@ -67,7 +67,10 @@ __host__ __device__ inline MoverCounts mover_counts(const MoverRecord& r, uint32
 // Movers up to which an iteration merges, its record being there: small states a
 // quarter (at least 8,192), larger ones any number -- us an iteration of random
 // free particles, merge / full sort after the record: 423,000 particles 94 / 144
-// with 28 % moving, 124 / 168 with 64 %; 2,000,000 382 / 494 and 533 / 631.
+// with 28 % moving, 124 / 168 with 64 %; 2,000,000 382 / 494 and 533 / 631.  Either
+// side of the line, with 23 % moving, merge / full sort without a record: 40,000
+// 34.6 / 42.0, 60,000 38.3 / 47.8, 70,000 39.7 / 48.2, 131,072 45.9 / 60.5, 262,144
+// 58.3 / 73.9; a full sort after the record takes 58 to 62 at 40,000 to 70,000.
 inline int64_t mover_limit(int64_t n) {
   if (n > 65536) return n;
   return n / 4 > 8192 ? n / 4 : 8192;

@@ -1234,12 +1234,11 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocks) step_diag(StepArgs 
 // plain loads.  An iteration the merge does not take (merge_wanted) is sorted in
 // the cluster too (resident_sort).
 // Measured, us an iteration, cluster against graph (split precision, 64
-// iterations a call): 1,023 particles 12.9 / 23.4, 6,400 14.8 / 25.1, 14,375
-// 18.4 / 25.3, 16,200 18.8 / 25.9, 20,300 25.5 / 25.8 (a second round of the
-// cluster's 16,384 threads), 32,400 30.2 / 27.0; one iteration a call 17.1 / 23.4
-// at 1,023, 22.9 / 26.0 at 16,200.  (Later: 1,023 11.5 / 17.6, 6,400 13.1 / 18.8,
-// 16,129 17.7 / 19.6; one a call 15.3 / 17.6, 17.2 / 18.7 and 21.6 / 19.6, so calls
-// of one iteration above kResidentSingleMaxN use the graph.)
+// iterations a call): 1,023 particles 10.7 / 16.8, 6,400 11.9 / 17.5, 12,800
+// 14.5 / 18.5, 16,384 17.3 / 18.7 (more would need a second round of the cluster's
+// 16,384 threads); one iteration a call 14.4 / 17.0, 16.2 / 18.7, 18.6 / 18.8 and
+// 19.1 / 19.0, so calls of one iteration above kResidentSingleMaxN use the graph.
+// Iterations that are not merged: 34.6 / 53.6 at 9,000, 43.9 / 53.5 at 16,384.
 constexpr int kResidentThreads = 1024;
 constexpr int kResidentGroups = kResidentThreads / kResidentMergeThreads;   // merge blocks at a time
 constexpr int kResidentChunks = kResidentThreads / kDiagThreads;    // diagnostics chunks at a time
@@ -1294,8 +1293,8 @@ __device__ __forceinline__ uint32_t keys_before(const uint32_t* keys, uint32_t r
 // of the blocks before come first, of those after last.  `per` slots a block.
 // Over an iteration that merges it costs nothing at 1,023 particles and 12 us at
 // 16,384.  An iteration of 9,000 / 12,000 / 16,384 particles that nearly all move:
-// 35 / 38 / 43 us (as a graph with the radix sort about 60 at any of them; comparing
-// every key with every other 433 / 572 / 758).  The keys stay in shared memory
+// 35 / 38 / 44 us (as a graph with the radix sort 52 to 54 at any of them; comparing
+// every key with every other 441 / 583 / 775).  The keys stay in shared memory
 // between the steps: held in registers they made the merging iterations, which never
 // come here, up to 2 % slower (spills around this code).
 template <int PREC>

@@ -269,8 +269,7 @@ class Sim:
     def download(self, forces=True, stream=None, out=None):
         """Current state as FP64 arrays in slot order.  out: optional dict of the
         caller's arrays to fill (x, y, vx, vy, rho, ids, and fx, fy with forces),
-        each C-contiguous with n entries of the right type; reused buffers whose
-        pages are resident let host-access mode 2 write them from the device."""
+        each C-contiguous with n entries of the right type."""
         n = self.n
         names = ("x", "y", "vx", "vy", "rho") + (("fx", "fy") if forces else ())
         if out is None:
