@@ -16,7 +16,9 @@ namespace sphg {
 
 // Threads of a merge block: four slots each in the kernel of its own, whose many
 // blocks hide each other's latency (eight warps of two slots: 1M dam break 81.8 ->
-// 83.3 us an iteration, batch of 256 411 -> 420); one each in the resident
+// 83.3 us an iteration, batch of 256 411 -> 420, 524,176 particles 48.5 -> 49.1,
+// 262,144 32.6 -> 32.6, 512 x 512 vortex 37.1 -> 36.6, 131,044 25.3 -> 25.0, 93,636
+// 25.0 -> 24.8, 40,000 21.0 -> 20.8); one each in the resident
 // kernel, where a block has an SM's schedulers to itself and takes as long as its
 // instructions (1,023 particles 11.7 -> 10.95 us, 6,084 28.1 -> 25.5, 12,800 16.6
 // -> 16.2).
