@@ -62,7 +62,9 @@ __device__ __forceinline__ void record_movers(const StepArgs& a, uint32_t i, uin
     return;
   }
   // insertion point: the new cell's range when it holds particles now (the slot
-  // itself is not among them), else a warp-wide 32-way search of the keys
+  // itself is not among them), else a warp-wide 32-way search of the keys, once for
+  // every cell of the warp's movers (32 of 30,000 particles into one empty cell:
+  // 29.3 us an iteration, searched for one by one 43.3)
   uint32_t p = 0;
   bool search = false;
   if (mine) {
@@ -70,9 +72,8 @@ __device__ __forceinline__ void record_movers(const StepArgs& a, uint32_t i, uin
     search = cr.z != epoch || cr.x >= cr.y;
     p = i < cr.x ? cr.x : cr.y;
   }
-  for (unsigned todo = __ballot_sync(0xffffffffu, search); todo; todo &= todo - 1) {
-    const int l = __ffs(todo) - 1;
-    const uint32_t k = __shfl_sync(0xffffffffu, key, l);
+  for (unsigned todo = __ballot_sync(0xffffffffu, search); todo;) {
+    const uint32_t k = __shfl_sync(0xffffffffu, key, __ffs(todo) - 1);
     int64_t lo = 0, hi = a.n;
     while (hi > lo) {
       const int64_t step = (hi - lo + 31) / 32;
@@ -83,7 +84,9 @@ __device__ __forceinline__ void record_movers(const StepArgs& a, uint32_t i, uin
       if (nhi < hi) hi = nhi;
       if (lo > hi) lo = hi;
     }
-    if (lane == l) p = (uint32_t)lo;
+    const bool found = search && key == k;
+    if (found) p = (uint32_t)lo;
+    todo &= ~__ballot_sync(0xffffffffu, found);
   }
   if (mine && p <= (uint64_t)a.n) {
     const int sh = 8 * (int)(p & 3u);
